@@ -36,7 +36,7 @@
 #include <memory>
 #include <mutex>
 
-#include "rr_internal.h"
+#include "pmleaf.h"
 
 namespace rr {
 
@@ -640,8 +640,10 @@ size_t base_smem_bytes(int m, int n, int K, bool m_smem) {
   return bytes;
 }
 
-// ---------------------------------------------------------------- leaves + block basis (main path)
-// The main path splits a block of K leaves in two kernels:
+// ---------------------------------------------------------------- leaves + block basis on the CUDA cores
+// The form a context selects with rr_ctx_set_pm_tensor_cores(ctx, 0); the
+// default is the cluster kernel of pmleaf.cu.  A block of K leaves is split in
+// two kernels:
 //
 //   pm_leaves_kernel (one CTA) runs the K order-1 leaves in sequence and, for
 //   each, records the stored transform T_k (transposed, Tt[k][s][i]) and its
@@ -651,13 +653,9 @@ size_t base_smem_bytes(int m, int n, int K, bool m_smem) {
 //   factors m_{K-1} ... m_0 (m_k = D1 T_k + x Dx T_k) in parallel and writes the
 //   block's basis, normalised by the row scales.
 //
-// Elimination.  For m <= 32 rows and n + m <= 48 columns (b <= 16) one warp
-// eliminates with one row per lane, held in registers: the pivot row is
-// broadcast by shuffles, the pivot column is the unpivoted column of least
-// list position (one redux.sync), and no CTA barrier is needed.  Larger
-// blocks keep the matrix in shared memory and give each warp the rows
-// i == warp (mod 16), with one CTA barrier per pivot step.  Either way the
-// loop stops once all n columns have pivots: no later row can get one.
+// Elimination.  The matrix is kept in shared memory; each warp takes the rows
+// i == warp (mod 16), with one CTA barrier per pivot step.  The loop stops once
+// all n columns have pivots: no later row can get one.
 //
 // Residual update.  The rows are regrouped so that pivot rows ("x" rows,
 // shifted by one coefficient) come first, each group padded to a multiple of
@@ -952,490 +950,6 @@ __global__ void __launch_bounds__(kLeafThreads) pm_leaves_kernel(LeafParams P) {
   }
 }
 
-// ---------------------------------------------------------------- leaves, tensor-core path (b <= 16)
-// For m <= 32 rows and n <= 16 columns the residual update runs on the int8
-// tensor cores, exactly: residues are < 2^31, so with byte limbs
-//   (T R)[i][c] = sum over a, b of 256^(a+b) (T_a R_b)[i][c],
-// and per shift class s = a + b the limb products summed over the 32-long
-// inner dimension stay below 4 * 32 * 255^2 < 2^23, exact in int32
-// (mma.sync m16n8k32 u8).  Classes 0..3 are recombined exactly in 64 bits
-// (< 2^48), classes 4..6 are added with weights 2^(8s) mod p, and one
-// Montgomery reduction gives (T R) R^{-1} -- the value the CUDA-core path
-// produces.  The residual lives in shared memory only as byte planes,
-// plane[t][limb][c][i] (one 32-byte row per column c, K index i), so each B
-// fragment is two 32-bit loads; the transform T is staged the same way for
-// the A fragments.  Row r of a plane keeps word w at w ^ 4 (r >> 2 & 1), so the
-// fragment loads of rows r and r + 4 fall in different banks.
-//
-// The elimination runs in kElimWarps warps, one row per lane, each warp
-// holding kElimColsPerWarp of the 48 columns in registers; every column is
-// updated unconditionally (padding columns are zero and stay zero), so the
-// updates of a step are independent.  Two warps per SM sub-partition hide
-// each other's dependency latencies (the elimination is the serial part of a
-// leaf).
-constexpr int kMmaRows = 32;
-constexpr int kMmaCols = 16;
-constexpr int kElimWarps = 8;
-constexpr int kRpartStride = kMmaCols + 1;            // row stride of the published columns
-constexpr int kRpartSize = kMmaRows * kRpartStride;
-constexpr int kElimColsPerWarp = 6;  // 8 x 6 = 48 >= n + m
-static_assert(kElimWarps * kElimColsPerWarp >= kMmaRows + kMmaCols, "elimination columns");
-static_assert(kElimWarps <= kLeafWarps, "elimination warps");
-
-// Named barriers of the elimination warps and of the update warps.
-__device__ __forceinline__ void elim_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kElimWarps * 32) : "memory"); }
-__device__ __forceinline__ void upd_bar() {
-  asm volatile("bar.sync 2, %0;" ::"n"((kLeafWarps - kElimWarps) * 32) : "memory");
-}
-constexpr uint64_t kLeafWaitNs = 2000000000ull;  // 2 s of %globaltimer per hand-off wait
-__device__ __forceinline__ uint64_t leaf_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void leaf_mma_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__host__ __device__ constexpr int plane_word(int r, int w) { return r * 8 + (w ^ (((r >> 2) & 1) << 2)); }
-
-// Words of one residual coefficient in plane form: 4 limbs x (n padded to 8) rows x 8 words.
-__host__ __device__ constexpr int leaf_plane_words(int n) { return 32 * 8 * ((n + 7) / 8); }
-
-// Shared-memory bytes of pm_leaves_mma_kernel.
-size_t leaves_mma_smem_bytes(int m, int n, int K) {
-  size_t words = (size_t)2 * K * leaf_plane_words(n) + 2048 + (size_t)m * (m + 1) + (size_t)m * n + 2 * (size_t)m;
-  size_t bytes = (words * 4 + 15) & ~(size_t)15;
-  bytes += 2 * (size_t)m * 8 + (size_t)m * 4 + 64;
-  return bytes;
-}
-
-__device__ __forceinline__ void plane_store(uint32_t* coeff, int NPc, int col, int row, uint32_t v) {
-  unsigned char* b = reinterpret_cast<unsigned char*>(coeff);
-  const int wo = plane_word(col, row >> 2), bo = row & 3;
-#pragma unroll
-  for (int l = 0; l < 4; ++l) b[4 * (l * NPc * 8 + wo) + bo] = (unsigned char)(v >> (8 * l));
-}
-
-__global__ void __launch_bounds__(kLeafThreads) pm_leaves_mma_kernel(LeafParams P) {
-  leaf_select(P);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int m = P.m, n = P.n, K = P.K;
-  const int W = n + m;
-  const int NT = (n + 7) / 8, MT = (m + 15) / 16, NPc = 8 * NT;
-  const int PW = leaf_plane_words(n);
-  const int TQS = m + 1;
-  const ModP M = P.M;
-  const uint32_t p = M.p;
-  uint32_t* Rc = reinterpret_cast<uint32_t*>(smem_raw);  // [K][PW] residual byte planes
-  uint32_t* Rn = Rc + K * PW;
-  uint32_t* Tp = Rn + K * PW;                             // 2 x [4][32 rows][8 words] byte planes of T
-  uint32_t* Tq = Tp + 2048;                               // [m][TQS]: Tq[s][i] = T[i][s]
-  uint32_t* R0 = Tq + m * TQS;                            // [m][n]: coefficient 0 of the residual
-  uint32_t* sigma = R0 + m * n;                           // m
-  uint32_t* sig_tmp = sigma + m;                          // m
-  const size_t w32 = (size_t)2 * K * PW + 2048 + (size_t)m * TQS + (size_t)m * n + 2 * (size_t)m;
-  int64_t* sdelta = reinterpret_cast<int64_t*>(smem_raw + ((w32 * 4 + 15) & ~(size_t)15));
-  int64_t* sdelta_tmp = sdelta + m;
-  int* perm = reinterpret_cast<int*>(sdelta_tmp + m);
-  __shared__ unsigned long long s_mx2[2];     // pivot-row masks of the last two leaves
-  __shared__ volatile int s_tready, s_c1, s_abort;
-  __shared__ int s_ok_e, s_ok_u;
-  __shared__ uint32_t rpart[2 * kRpartSize];  // first n columns of A, all rows, double buffered
-
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
-  const uint32_t Wt[3] = {M.c32, (uint32_t)((uint64_t)M.c32 * 256 % p), (uint32_t)((uint64_t)M.c32 * 65536 % p)};
-
-  // padding bytes (rows i >= m of every column, columns c >= n) stay zero for good
-  for (int e = tid; e < 2 * K * PW + 2048; e += nt) Rc[e] = 0;
-  __syncthreads();
-  for (int e = tid; e < K * m * n; e += nt) {
-    const int t = e / (m * n), i = (e / n) % m, c = e % n;
-    const uint32_t v = P.G[(int64_t)i * P.g_rs + (int64_t)c * P.g_cs + t];
-    plane_store(Rc + t * PW, NPc, c, i, v);
-    if (t == 0) R0[i * n + c] = v;
-  }
-  for (int i = tid; i < m; i += nt) {
-    sdelta[i] = P.delta[i];
-    sigma[i] = 1;
-  }
-  __syncthreads();
-
-  // Two warp groups overlap consecutive leaves: the elimination warps (E,
-  // warps 0 .. kElimWarps-1) run leaf k+1 while the update warps (U, the
-  // others) still apply T_k to the remaining coefficients of the residual.
-  // Leaf k+1 needs only coefficient 0 of the new residual, which E computes
-  // itself (from coefficients 0 and 1 of the old one); U computes the others,
-  // coefficient 1 first.  Residual buffer j & 1 holds the residual before leaf
-  // j; E writes only coefficient 0 of a buffer and U only coefficients >= 1,
-  // and T_k's byte planes and mask are double buffered by k & 1.  Hand-offs are
-  // counters in shared memory: s_tready = k + 1 once T_k, its mask and the new
-  // coefficient 0 are written (U may start on leaf k), s_c1 = k + 1 once U has
-  // written coefficient 1 of the residual after leaf k (E may take T_{k+1} and
-  // reuse T_{k-1}'s planes).  A wait gives up after kLeafWaitNs, raises
-  // s_abort and sets *P.status = 3; both groups then leave their loops.
-  if (tid == 0) {
-    s_tready = 0;
-    s_c1 = 0;
-    s_abort = 0;
-  }
-  __syncthreads();
-  const int tiles = MT * NT;  // 1, 2 or 4: a divisor of the group's warp count
-  auto wait_count = [&](volatile int* cnt, int target) -> bool {
-    const uint64_t t0 = leaf_ns();
-    while (*cnt < target) {
-      if (s_abort) return false;
-      if (leaf_ns() - t0 > kLeafWaitNs) {
-        s_abort = 1;
-        atomicExch(P.status, 3);
-        return false;
-      }
-      __nanosleep(32);
-    }
-    __threadfence_block();
-    return true;
-  };
-  // outputs t in [tmin, tmax] (and < rem) of Rn[t][i] = T_i . Rc[t + 1 - mask_i],
-  // from the products T Rc[tq] for the tq of this warp's share
-  auto residual = [&](int gw, int gwarps, int tq_first, int tq_last, int tmin, int tmax, const uint32_t* Tpl,
-                      const uint32_t* Rcl, uint32_t* Rnl, unsigned long long mx, int rem) {
-    const int tile = gw % tiles, tq0 = tq_first + gw / tiles, tqs = gwarps / tiles;
-    const int mt = tile / NT, ntl = tile % NT;
-    const int r0 = mt * 16 + g, r1 = r0 + 8, col = ntl * 8 + g;
-    if (tq0 > tq_last) return;
-    uint32_t A[4][4];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      A[l][0] = Tpl[l * 256 + plane_word(r0, t4)];
-      A[l][1] = Tpl[l * 256 + plane_word(r1, t4)];
-      A[l][2] = Tpl[l * 256 + plane_word(r0, t4 + 4)];
-      A[l][3] = Tpl[l * 256 + plane_word(r1, t4 + 4)];
-    }
-    for (int tq = tq0; tq <= tq_last; tq += tqs) {
-      uint32_t Bf[4][2];
-      const uint32_t* rc = Rcl + tq * PW;
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        Bf[l][0] = rc[l * NPc * 8 + plane_word(col, t4)];
-        Bf[l][1] = rc[l * NPc * 8 + plane_word(col, t4 + 4)];
-      }
-      int C[7][4];
-#pragma unroll
-      for (int s = 0; s < 7; ++s)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) C[s][v] = 0;
-#pragma unroll
-      for (int l = 0; l < 4; ++l)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) leaf_mma_u8(C[l + r], A[l], Bf[r][0], Bf[r][1]);
-      // classes 0..3 exactly in 64 bits (< 2^48), classes 4..6 with their weights
-      uint32_t lo[4], hi[4];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const uint64_t x = (uint64_t)(uint32_t)C[0][v] + ((uint64_t)(uint32_t)C[1][v] << 8) +
-                           ((uint64_t)(uint32_t)C[2][v] << 16) + ((uint64_t)(uint32_t)C[3][v] << 24);
-        lo[v] = (uint32_t)x;
-        hi[v] = (uint32_t)(x >> 32);
-        mac_cc((uint32_t)C[4][v], Wt[0], lo[v], hi[v]);
-        mac_cc((uint32_t)C[5][v], Wt[1], lo[v], hi[v]);
-        mac_cc((uint32_t)C[6][v], Wt[2], lo[v], hi[v]);
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int row = (v < 2) ? r0 : r1;
-        const int c = ntl * 8 + 2 * t4 + (v & 1);
-        if (row < m && c < n) {
-          const int t = tq - 1 + (int)((mx >> row) & 1ull);
-          if (t >= tmin && t <= tmax && t < rem) {
-            const uint32_t val = redc_cc(lo[v], hi[v], M);
-            plane_store(Rnl + t * PW, NPc, c, row, val);
-            if (t == 0) R0[row * n + c] = val;
-          }
-        }
-      }
-    }
-  };
-  uint32_t* const Rbuf[2] = {Rc, Rn};
-
-  if (warp < kElimWarps) {
-    for (int leaf = 0; leaf < K; ++leaf) {
-      // stable sort of delta, descending (src/sigma_basis.rs:357-359): lane q
-      // takes the row of sorted position q
-      if (warp == 0 && lane < m) {
-        const int64_t di = sdelta[lane];
-        int pos = 0;
-        for (int j = 0; j < m; ++j) {
-          const int64_t dj = sdelta[j];
-          pos += (dj > di) || (dj == di && j < lane);
-        }
-        perm[pos] = lane;
-      }
-      elim_bar();
-      const int myrow = lane < m ? perm[lane] : 0;
-      // this warp's columns of row `lane` of A = [pi r | pi] (src/sigma_basis.rs:369-380)
-      const int c0 = kElimColsPerWarp * warp;
-      uint32_t a[kElimColsPerWarp];
-#pragma unroll
-      for (int cl = 0; cl < kElimColsPerWarp; ++cl) {
-        const int c = c0 + cl;
-        uint32_t v = 0;
-        if (lane < m && c < W) v = c < n ? R0[myrow * n + c] : ((c - n) == myrow ? 1u : 0u);
-        a[cl] = v;
-      }
-      // LSP elimination (src/modular_linalg.rs:188-239), fraction-free:
-      // row_i <- (piv row_i - a_i,cs row_k) R^{-1}.  Every warp keeps the list
-      // positions of the unpivoted columns (lane c < n; -1 once pivoted) and
-      // picks the non-zero column of least position.  The owners of the first
-      // n columns publish them for all rows after every update (double
-      // buffered), so one barrier per pivot step lets each warp read both row
-      // k and the pivot column.
-      int lpos = lane < n ? lane : -1;
-      int rank = 0, cur = 0;
-      bool piv_row = false;
-      auto publish = [&](uint32_t* dst) {
-        if (lane < m) {
-#pragma unroll
-          for (int cl = 0; cl < kElimColsPerWarp; ++cl)
-            if (c0 + cl < n) dst[lane * kRpartStride + c0 + cl] = a[cl];
-        }
-      };
-      publish(rpart);
-      elim_bar();
-      for (int k = 0; k < m && rank < n; ++k) {
-        const uint32_t* rp = rpart + cur * kRpartSize;
-        const uint32_t mine = lane < n ? rp[k * kRpartStride + lane] : 0u;
-        const int key = (lpos >= 0 && mine != 0) ? ((lpos << 5) | lane) : 0x7fffffff;
-        const int best = __reduce_min_sync(0xffffffffu, key);
-        if (best == 0x7fffffff) continue;  // no pivot in row k (same decision in every warp)
-        const int cs = best & 31, ts = best >> 5;
-        if (lpos >= 0) lpos = (lane == cs) ? -1 : (lpos == 0 ? ts - 1 : lpos - 1);
-        ++rank;
-        piv_row = piv_row || (lane == k);
-        const uint32_t f = lane < m ? rp[lane * kRpartStride + cs] : 0u;
-        const uint32_t piv = rp[k * kRpartStride + cs];
-        const uint32_t nf = p - f;
-        const bool upd = lane > k && lane < m;
-#pragma unroll
-        for (int cl = 0; cl < kElimColsPerWarp; ++cl) {
-          const uint32_t ak = __shfl_sync(0xffffffffu, a[cl], k);
-          const uint32_t nv = redc_2mac(piv, a[cl], nf, ak, M);
-          a[cl] = upd ? nv : a[cl];
-        }
-        if (rank < n) {  // the last pivot's update is final: nobody reads it back
-          cur ^= 1;
-          publish(rpart + cur * kRpartSize);
-          elim_bar();
-        }
-      }
-      // T (transposed) = columns n.. of A; c_i = T[i][perm[i]] (owned by one warp)
-      uint32_t* Tg = P.Tt + (size_t)leaf * m * m;
-#pragma unroll
-      for (int cl = 0; cl < kElimColsPerWarp; ++cl) {
-        const int c = c0 + cl;
-        if (c >= n && c < W && lane < m) {
-          const int s = c - n;
-          Tq[s * TQS + lane] = a[cl];
-          Tg[s * m + lane] = a[cl];
-          if (s == myrow) {
-            if (a[cl] == 0) atomicExch(P.status, 2);
-            sig_tmp[lane] = redc((uint64_t)a[cl] * sigma[myrow], M);
-          }
-        }
-      }
-      if (warp == 0) {
-        const unsigned long long mx = (unsigned long long)__ballot_sync(0xffffffffu, piv_row && lane < m);
-        if (lane < m) sdelta_tmp[lane] = sdelta[myrow] - (piv_row ? 1 : 0);  // src/sigma_basis.rs:408-411
-        if (lane == 0) {
-          P.mask[leaf] = mx;
-          s_mx2[leaf & 1] = mx;
-        }
-      }
-      elim_bar();
-      if (warp == 0 && lane < m) {
-        sigma[lane] = sig_tmp[lane];
-        sdelta[lane] = sdelta_tmp[lane];
-      }
-      const int rem = K - leaf - 1;
-      if (rem == 0) break;
-      // coefficient 1 of this leaf's residual is U's (leaf - 1 > = 0), and
-      // U's work on leaf - 1 no longer reads the planes of T_{leaf - 2}
-      if (leaf > 0) {
-        if (tid == 0) s_ok_e = wait_count(&s_c1, leaf) ? 1 : 0;
-        elim_bar();
-        if (!s_ok_e) break;
-      }
-      uint32_t* const Tpl = Tp + (leaf & 1) * 1024;
-      // byte planes of T: row i, word w holds limb l of T[i][4w .. 4w+3]
-      for (int e = tid; e < m * 8; e += kElimWarps * 32) {
-        const int i = e >> 3, w = e & 7;
-        uint32_t v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = (4 * w + j < m) ? Tq[(4 * w + j) * TQS + i] : 0u;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          const uint32_t lo = __byte_perm(v[0], v[1], 0x40 + 0x11 * l) & 0xffffu;  // byte l of v0, byte l of v1
-          const uint32_t hi = __byte_perm(v[2], v[3], 0x40 + 0x11 * l) & 0xffffu;
-          Tpl[l * 256 + plane_word(i, w)] = lo | (hi << 16);
-        }
-      }
-      elim_bar();
-      // coefficient 0 of the next residual (products with coefficients 0 and 1)
-      residual(warp, kElimWarps, 0, std::min(1, rem), 0, 0, Tpl, Rbuf[leaf & 1], Rbuf[(leaf + 1) & 1],
-               s_mx2[leaf & 1], rem);
-      elim_bar();
-      if (tid == 0) {
-        __threadfence_block();
-        s_tready = leaf + 1;
-      }
-    }
-  } else {
-    const int uw = warp - kElimWarps, uwarps = kLeafWarps - kElimWarps;
-    for (int leaf = 0; leaf + 1 < K; ++leaf) {
-      if (tid == kElimWarps * 32) s_ok_u = wait_count(&s_tready, leaf + 1) ? 1 : 0;
-      upd_bar();
-      if (!s_ok_u) break;
-      const int rem = K - leaf - 1;
-      const uint32_t* Tpl = Tp + (leaf & 1) * 1024;
-      const uint32_t* Rcl = Rbuf[leaf & 1];
-      uint32_t* Rnl = Rbuf[(leaf + 1) & 1];
-      const unsigned long long mx = s_mx2[leaf & 1];
-      // coefficient 1 first (products with coefficients 1 and 2), then the rest
-      residual(uw, uwarps, 1, std::min(2, rem), 1, rem - 1, Tpl, Rcl, Rnl, mx, rem);
-      upd_bar();
-      if (tid == kElimWarps * 32) {
-        __threadfence_block();
-        s_c1 = leaf + 1;
-      }
-      residual(uw, uwarps, 3, rem, 1, rem - 1, Tpl, Rcl, Rnl, mx, rem);
-      upd_bar();
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < m; i += nt) {
-    P.sigma_inv[i] = inv_fermat(sigma[i], M);
-    P.delta[i] = sdelta[i];
-  }
-}
-
-// Block basis on the int8 tensor cores (2b <= 32): CTA (j, z) keeps column j
-// of generator z's block basis as byte planes Vp[limb][t][8 words]
-// (coefficient t = plane row, K index s = byte s) and applies
-//   V_{k+1}[t' + mask_k(i)][i] = (T_k V_k[t'])[i] 2^-32,
-// the same Montgomery convention as the CUDA-core kernel below, with exact
-// u8-limb mma.sync products (T_k staged as byte planes as in the leaves kernel).
-__device__ __forceinline__ uint32_t plane_load(const uint32_t* coeff, int NPc, int col, int row) {
-  const unsigned char* b = reinterpret_cast<const unsigned char*>(coeff);
-  const int wo = plane_word(col, row >> 2), bo = row & 3;
-  uint32_t v = 0;
-#pragma unroll
-  for (int l = 0; l < 4; ++l) v |= (uint32_t)b[4 * (l * NPc * 8 + wo) + bo] << (8 * l);
-  return v;
-}
-
-// Plane rows of the block basis kernel: K + 2 coefficients, multiple of 8.
-__host__ __device__ constexpr int bb_rows(int K) { return (K + 2 + 7) & ~7; }
-
-size_t block_basis_mma_smem_bytes(int K) { return ((size_t)2 * 4 * bb_rows(K) * 8 + 1024) * 4; }
-
-__global__ void __launch_bounds__(256) pm_block_basis_mma_kernel(const uint32_t* __restrict__ Tt,
-                                                                 const unsigned long long* __restrict__ mask,
-                                                                 const uint32_t* __restrict__ sigma_inv, int m, int K,
-                                                                 uint32_t* Mout, int64_t out_rs, int64_t out_cs,
-                                                                 int64_t out_bs, ModP M) {
-  extern __shared__ __align__(16) uint32_t bbm_smem[];
-  Tt += (int64_t)blockIdx.y * K * m * m;
-  mask += (int64_t)blockIdx.y * K;
-  sigma_inv += (int64_t)blockIdx.y * m;
-  Mout += (int64_t)blockIdx.y * out_bs;
-  const int VR = bb_rows(K);
-  uint32_t* Vc = bbm_smem;          // [4][VR][8] byte planes of V_k
-  uint32_t* Vn = Vc + 4 * VR * 8;   // V_{k+1}
-  uint32_t* Tp = Vn + 4 * VR * 8;   // [4][32][8] byte planes of T_k
-  const int j = blockIdx.x;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-  const int g = lane >> 2, t4 = lane & 3;
-  const uint32_t p = M.p;
-  const uint32_t Wt[3] = {M.c32, (uint32_t)((uint64_t)M.c32 * 256 % p), (uint32_t)((uint64_t)M.c32 * 65536 % p)};
-  const int MT = (m + 15) / 16;
-  for (int e = tid; e < 2 * 4 * VR * 8 + 1024; e += nt) bbm_smem[e] = 0;
-  __syncthreads();
-  if (tid == 0) plane_store(Vc, VR, 0, j, 1u);  // V_0 = e_j
-  for (int k = 0; k < K; ++k) {
-    const unsigned long long mk = mask[k];
-    const uint32_t* Tk = Tt + (size_t)k * m * m;  // Tk[s * m + i] = T_k[i][s]
-    for (int e = tid; e < m * 8; e += nt) {
-      const int i = e >> 3, w = e & 7;
-      uint32_t v[4];
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) v[jj] = (4 * w + jj < m) ? Tk[(4 * w + jj) * m + i] : 0u;
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        const uint32_t lo = __byte_perm(v[0], v[1], 0x40 + 0x11 * l) & 0xffffu;
-        const uint32_t hi = __byte_perm(v[2], v[3], 0x40 + 0x11 * l) & 0xffffu;
-        Tp[l * 256 + plane_word(i, w)] = lo | (hi << 16);
-      }
-    }
-    for (int e = tid; e < 4 * (k + 2) * 8; e += nt) {  // rows 0 .. k+1 of V_{k+1}
-      const int l = e / ((k + 2) * 8), r = e - l * (k + 2) * 8;
-      Vn[l * VR * 8 + r] = 0;
-    }
-    __syncthreads();
-    const int NTk = (k + 1 + 7) / 8;
-    for (int job = warp; job < MT * NTk; job += nwarps) {
-      const int mt = job / NTk, ntl = job % NTk;
-      const int r0 = mt * 16 + g, r1 = r0 + 8, col = ntl * 8 + g;
-      uint32_t A[4][4], Bf[4][2];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        A[l][0] = Tp[l * 256 + plane_word(r0, t4)];
-        A[l][1] = Tp[l * 256 + plane_word(r1, t4)];
-        A[l][2] = Tp[l * 256 + plane_word(r0, t4 + 4)];
-        A[l][3] = Tp[l * 256 + plane_word(r1, t4 + 4)];
-        Bf[l][0] = Vc[l * VR * 8 + plane_word(col, t4)];
-        Bf[l][1] = Vc[l * VR * 8 + plane_word(col, t4 + 4)];
-      }
-      int C[7][4];
-#pragma unroll
-      for (int q = 0; q < 7; ++q)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) C[q][v] = 0;
-#pragma unroll
-      for (int l = 0; l < 4; ++l)
-#pragma unroll
-        for (int r = 0; r < 4; ++r) leaf_mma_u8(C[l + r], A[l], Bf[r][0], Bf[r][1]);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int row = (v < 2) ? r0 : r1;
-        const int tp = ntl * 8 + 2 * t4 + (v & 1);
-        if (row < m && tp <= k) {
-          const uint64_t x = (uint64_t)(uint32_t)C[0][v] + ((uint64_t)(uint32_t)C[1][v] << 8) +
-                             ((uint64_t)(uint32_t)C[2][v] << 16) + ((uint64_t)(uint32_t)C[3][v] << 24);
-          uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
-          mac_cc((uint32_t)C[4][v], Wt[0], lo, hi);
-          mac_cc((uint32_t)C[5][v], Wt[1], lo, hi);
-          mac_cc((uint32_t)C[6][v], Wt[2], lo, hi);
-          plane_store(Vn, VR, tp + (int)((mk >> row) & 1ull), row, redc_cc(lo, hi, M));
-        }
-      }
-    }
-    __syncthreads();
-    uint32_t* tv = Vc;
-    Vc = Vn;
-    Vn = tv;
-  }
-  for (int e = tid; e < (K + 1) * m; e += nt) {
-    const int t = e / m, r = e % m;
-    Mout[(int64_t)r * out_rs + (int64_t)j * out_cs + t] = mulmod(plane_load(Vc, VR, t, r), sigma_inv[r], M);
-  }
-}
-
 // Block basis, one CTA per column j: V_0 = e_j, V_{k+1}[t][i] = T_k[i] . V_k[t - mask_k(i)]
 // (t <= k + 1), with the same Montgomery convention as the residual; then
 // Mout[i][j][t] = V_K[t][i] sigma_inv[i].  Rows are taken in the grouped slot
@@ -1600,7 +1114,7 @@ struct Pm {
   DevBuf<int> status;
   int64_t cs = 0;                      // residual coefficient stride of the leaves kernel (words)
   int fold4 = 0;
-  bool mma = false;                    // tensor-core leaves kernel (b <= 16)
+  bool mma = false;                    // leaf blocks on clusters and tensor cores (pmleaf.cu)
   // per recursion depth: MM, GG, MMM ([nb] each)
   std::vector<std::unique_ptr<DevBuf<uint32_t>>> bufs;
 };
@@ -1745,6 +1259,10 @@ int poly_mat_mul(Pm& P, MatView A, int mA, int r, int64_t la, MatView B, int k, 
 }
 
 int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
+  if (P.mma)
+    return leaf_block_launch(LeafBlock{G.p, G.rs, G.cs, G.bs, P.m, P.n, nleaves, P.delta.ptr, Mout.p, Mout.rs, Mout.cs,
+                                       Mout.bs, P.M, P.status.ptr, 0, 0, 0},
+                             P.nb, P.s);
   LeafParams L;
   L.G = G.p;
   L.g_rs = G.rs;
@@ -1761,9 +1279,7 @@ int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
   L.M = P.M;
   L.status = P.status.ptr;
   const unsigned nb = (unsigned)P.nb;
-  if (P.mma) {
-    pm_leaves_mma_kernel<<<nb, kLeafThreads, leaves_mma_smem_bytes(P.m, P.n, nleaves), P.s>>>(L);
-  } else if (P.n % 4 == 0) {
+  if (P.n % 4 == 0) {
     const size_t smem = leaves_smem_bytes(P.m, P.n, nleaves, P.cs);
     if (P.fold4) pm_leaves_kernel<4, 4><<<nb, kLeafThreads, smem, P.s>>>(L);
     else pm_leaves_kernel<4, 2><<<nb, kLeafThreads, smem, P.s>>>(L);
@@ -1776,12 +1292,6 @@ int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
   // the leaves kernel indexes its transforms with the block's own K; the
   // block basis reads them with the same K
   const dim3 grid((unsigned)P.m, nb);
-  if (P.mma) {
-    pm_block_basis_mma_kernel<<<grid, 256, block_basis_mma_smem_bytes(nleaves), P.s>>>(
-        P.Tt.ptr, P.leafmask.ptr, P.sigma_inv.ptr, P.m, nleaves, Mout.p, Mout.rs, Mout.cs, Mout.bs, P.M);
-    RR_CUDA(cudaGetLastError());
-    return RR_OK;
-  }
   const size_t bsm = block_basis_smem_bytes(P.m, nleaves);
   if (P.fold4)
     pm_block_basis_kernel<4><<<grid, 256, bsm, P.s>>>(P.Tt.ptr, P.leafmask.ptr, P.sigma_inv.ptr, P.m, nleaves, Mout.p,
@@ -1797,15 +1307,15 @@ int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
 // words plus 4, so that neighbouring coefficients start in different banks.
 int64_t leaf_coeff_stride(int m, int n) { return (((int64_t)m * n + 3) & ~(int64_t)3) + 4; }
 
-// Largest block of leaves (a power of two <= 64 for m <= 16, <= 32 otherwise,
-// and <= d) whose double-buffered residual fits in shared memory.
-int pick_block_leaves(int m, int n, int64_t d, bool mma, size_t* smem) {
+// Largest block of leaves of the CUDA-core kernels (a power of two <= 64 for
+// m <= 16, <= 32 otherwise, and <= d) whose double-buffered residual fits in
+// shared memory.
+int pick_block_leaves(int m, int n, int64_t d, size_t* smem) {
   const int kmax = m <= 16 ? 64 : 32;
   int K = (int)std::min<int64_t>(d, kmax);
   const int64_t cs = leaf_coeff_stride(m, n);
-  auto bytes = [&](int k) { return mma ? leaves_mma_smem_bytes(m, n, k) : leaves_smem_bytes(m, n, k, cs); };
-  while (K > 1 && bytes(K) > kBaseSmemBudget) K /= 2;
-  *smem = bytes(K);
+  while (K > 1 && leaves_smem_bytes(m, n, K, cs) > kBaseSmemBudget) K /= 2;
+  *smem = leaves_smem_bytes(m, n, K, cs);
   return K;
 }
 
@@ -1815,10 +1325,8 @@ int set_leaves_smem_limit(size_t bytes, size_t basis_bytes) {
   RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<4, 2>, attr, (int)bytes));
   RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<1, 4>, attr, (int)bytes));
   RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<1, 2>, attr, (int)bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_leaves_mma_kernel, attr, (int)bytes));
   RR_CUDA(cudaFuncSetAttribute(pm_block_basis_kernel<4>, attr, (int)basis_bytes));
   RR_CUDA(cudaFuncSetAttribute(pm_block_basis_kernel<2>, attr, (int)basis_bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_block_basis_mma_kernel, attr, (int)block_basis_mma_smem_bytes(64)));
   return RR_OK;
 }
 
@@ -1875,8 +1383,8 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   P.p = p;
   P.M = make_modp(p);
   size_t leaves_smem = 0;
-  P.mma = ctx->pm_tensor_cores && P.m <= kMmaRows && P.n <= kMmaCols;
-  P.K = pick_block_leaves(P.m, P.n, d, P.mma, &leaves_smem);
+  P.mma = ctx->pm_tensor_cores;
+  P.K = P.mma ? (int)std::min<int64_t>(d, leaf_block_max(P.m)) : pick_block_leaves(P.m, P.n, d, &leaves_smem);
   P.cs = leaf_coeff_stride(P.m, P.n);
   P.fold4 = fold4_ok(p, P.M);
   const int m = P.m, n = P.n;
@@ -1955,16 +1463,19 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   }
   RR_TRY(P.delta.alloc_async((size_t)nb * m, P.s));
   RR_TRY(P.status.alloc_async(1, P.s));
-  RR_TRY(P.Tt.alloc_async((size_t)nb * P.K * m * m, P.s));
-  RR_TRY(P.leafmask.alloc_async((size_t)nb * P.K, P.s));
-  RR_TRY(P.sigma_inv.alloc_async((size_t)nb * m, P.s));
+  if (!P.mma) {
+    RR_TRY(P.Tt.alloc_async((size_t)nb * P.K * m * m, P.s));
+    RR_TRY(P.leafmask.alloc_async((size_t)nb * P.K, P.s));
+    RR_TRY(P.sigma_inv.alloc_async((size_t)nb * m, P.s));
+  }
   RR_CUDA(cudaMemsetAsync(P.delta.ptr, 0, (size_t)nb * m * sizeof(int64_t), P.s));
   RR_CUDA(cudaMemsetAsync(P.status.ptr, 0, sizeof(int), P.s));
   // the limits are per kernel, shared by every caller in the process (the
   // batched engine runs generators on several threads): always the budget,
   // never this call's size, so a concurrent smaller call cannot lower them
   if (leaves_smem > kBaseSmemBudget) return fail(RR_EUNSUPPORTED, "leaf block needs %zu bytes of shared memory", leaves_smem);
-  RR_TRY(set_leaves_smem_limit(kBaseSmemBudget, block_basis_smem_bytes(64, 64)));
+  if (P.mma) RR_TRY(leaf_block_prepare(P.n));
+  else RR_TRY(set_leaves_smem_limit(kBaseSmemBudget, block_basis_smem_bytes(64, 64)));
   // G = [S; I], coefficients [0, d], one after the other
   DevBuf<uint32_t> dseq, G;
   const int np = b * (b + 1) / 2;
