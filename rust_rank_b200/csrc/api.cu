@@ -305,6 +305,7 @@ int rr_krylov_create(rr_matrix* mat, int32_t b, const uint32_t* row_precond, con
     RR_CUDA(cudaStreamSynchronize(s));
   }
   RR_TRY(krylov_occupancy(kr.get()));
+  RR_TRY(resident_prepare(kr.get()));
   kr->base = seq_len;
   kr->len = seq_len;
   RR_TRY(ensure_capacity(kr.get(), 64));
@@ -334,6 +335,8 @@ int rr_krylov_destroy(rr_krylov* kr) {
 // started and the graph can be replayed), and the run length that uses it.
 constexpr int64_t kGraphApps = 16;
 constexpr int64_t kGraphMinRun = 2 * kGraphApps;
+// Shortest run worth a resident launch (it reads the CSR into shared memory first).
+constexpr int64_t kResidentMinRun = 4;
 
 // Captures kGraphApps applications (they are recorded, not run: the host
 // state the launches advance is restored afterwards).  The capture runs on a
@@ -376,7 +379,14 @@ static int queue_apps(rr_krylov* kr, int64_t n_apps) {
   if (kr->len == 0) kr->len = 1;  // publish S_0
   RR_TRY(ensure_capacity(kr, kr->len - kr->base + 2 * n_apps + 1));
   int64_t i = 0;
-  if (n_apps >= kGraphMinRun) {
+  if (kr->res_grid > 0 && n_apps >= kResidentMinRun) {
+    for (bool taken = true; taken && i < n_apps;) {
+      const int k = (int)std::min<int64_t>(kResMaxApps, n_apps - i);
+      RR_TRY(resident_run(kr, k, &taken));
+      if (taken) i += k;
+    }
+  }
+  if (n_apps - i >= kGraphMinRun) {
     if (!kr->graph) RR_TRY(capture_graph(kr));
     if (kr->cur != kr->graph_cur) {
       RR_TRY(krylov_launch_application(kr, nullptr));

@@ -603,6 +603,8 @@ int rr_batch_create(rr_ctx* ctx, int32_t nmat, const int64_t* m, const int64_t* 
   RR_CUDA(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi));
   RR_CUDA(cudaStreamCreateWithPriority(&bt->stream, cudaStreamNonBlocking, prio_hi));
   RR_CUDA(cudaStreamSynchronize(st));
+  CoopHold hold;
+  RR_TRY(hold.begin(ctx->device, bt->stream));
   RR_TRY(tune_phases(bt.get(), pblocks));
   RR_TRY(krylov_status(bt.get()));
   RR_CUDA(cudaMemsetAsync(bt->gram_all.ptr, 0, bt->gram_all.bytes(), bt->stream));
@@ -641,6 +643,8 @@ int rr_batch_krylov(rr_batch* bt) {
   if (!bt) return fail(RR_EINVAL, "NULL handle");
   if (bt->done) return fail(RR_ESTATE, "the batch's sequences were already computed");
   RR_CUDA(cudaSetDevice(bt->ctx->device));
+  CoopHold hold;
+  RR_TRY(hold.begin(bt->ctx->device, bt->stream));
   RR_TRY(krylov_run(bt, nullptr, nullptr));
   RR_TRY(krylov_status(bt));
   bt->done = true;
@@ -677,7 +681,9 @@ int rr_batch_ranks(rr_batch* bt, int32_t workers, int64_t* ranks) {
   std::vector<cudaEvent_t> ev(nmat, nullptr);
   Progress prog;
   const bool overlap = !bt->done;
+  CoopHold hold;
   if (overlap) {
+    RR_TRY(hold.begin(bt->ctx->device, bt->stream));
     for (int s = 0; s < nmat; ++s) {
       cudaError_t e = cudaEventCreateWithFlags(&ev[s], cudaEventDisableTiming);
       if (e != cudaSuccess) {

@@ -37,45 +37,13 @@
 #include <numeric>
 #include <type_traits>
 
-#include "krylov_params.h"
+#include "krylov_gram.cuh"
 
 namespace rr {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 static_assert(kWarps == kPassWarps, "host-side run tables assume this many warps per CTA");
-
-// Threads of a warp split into RPW row slots of TPR threads; a thread owns
-// LPT lanes of its row's block, as NV 128-bit words interleaved with the other
-// threads of the slot: word v of thread `sub` is word v * TPR + sub of the row
-// (lanes 4 (v TPR + sub) .. + 3).  So one warp load instruction reads TPR
-// adjacent 16-byte words per row -- whole 32-byte sectors for B >= 8 -- and a
-// gathered row costs the L1 the minimum of B / 8 sector accesses.
-template <int B>
-constexpr int kDefaultLpt = (B >= 16) ? 8 : 4;
-
-template <int B, int L = kDefaultLpt<B>>
-struct Shape {
-  static constexpr int LPT = L;                   // lanes of the block per thread
-  static constexpr int NV = LPT / 4;              // 128-bit words per thread per row
-  static constexpr int TPR = B / LPT;             // threads per row
-  static constexpr int RPW = 32 / TPR;            // rows per warp batch (slots)
-  // block lane of this thread's lane l
-  static __device__ __forceinline__ int lane_of(int sub, int l) { return 4 * ((l >> 2) * TPR + sub) + (l & 3); }
-  // 128-bit word index within a row of this thread's word v
-  static __device__ __forceinline__ int word_of(int sub, int v) { return v * TPR + sub; }
-};
-
-__device__ __forceinline__ void pair_of(int q, int B, int& i, int& j) {
-  // q enumerates (i <= j) row-major: offset(i) = i*B - i*(i-1)/2
-  i = 0;
-  int off = 0;
-  while (q >= off + (B - i)) {
-    off += B - i;
-    ++i;
-  }
-  j = i + (q - off);
-}
 
 // acc[l] += sum over entries k = beg, beg+stride, ... < end of val * X[col][lane l]
 // for this thread's LPT lanes (lane block `sub`).  Four entries per step, all
@@ -229,8 +197,6 @@ __device__ __forceinline__ void gather_sum8(const uint2* __restrict__ cv, uint32
   }
 }
 
-__device__ __forceinline__ int pair_index(int i, int j, int B) { return i * B - i * (i - 1) / 2 + (j - i); }
-
 // Programmatic dependent launch: the single-matrix kernels are launched so
 // that the next kernel of an application may be scheduled while the previous
 // one finishes.  griddep_wait() blocks until the previous kernel has completed
@@ -239,234 +205,6 @@ __device__ __forceinline__ int pair_index(int i, int j, int B) { return i * B - 
 // griddep_launch() tells the scheduler a CTA has no more main-loop work.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// ---------------------------------------------------------------- Gram terms
-// Both accumulators sum G[i][j] = sum over rows of gz[i] * gu[j] (i <= j) for
-// the rows a warp processes, then add their residues into the CTA's red[].
-
-// CUDA cores (B = 4): the batch is staged in shared memory and every lane
-// accumulates a few (i, j) pairs over the staged rows.
-template <int B, int FE, int L = kDefaultLpt<B>>
-struct GramCore {
-  static constexpr int LPT = Shape<B, L>::LPT, RPW = Shape<B, L>::RPW;
-  static constexpr int NP = B * (B + 1) / 2, PPL = (NP + 31) / 32;
-  static constexpr int kWords = 2 * RPW * B;  // shared words per warp
-  uint32_t* zs;  // [RPW][B]
-  uint32_t* us;
-  uint32_t pij[PPL];
-  unsigned long long acc[PPL];
-
-  __device__ __forceinline__ void init(uint32_t* w, int lane) {
-    zs = w;
-    us = w + RPW * B;
-#pragma unroll
-    for (int t = 0; t < PPL; ++t) {
-      const int q = lane + 32 * t;
-      int i = 0, j = 0;
-      if (q < NP) pair_of(q, B, i, j);
-      pij[t] = ((uint32_t)i << 8) | (uint32_t)j;
-      acc[t] = 0;
-    }
-  }
-  __device__ __forceinline__ void add(const uint32_t (&gz)[LPT], const uint32_t (&gu)[LPT], int slot, int sub,
-                                      int lane, const ModP& M, const uint32_t (&)[3]) {
-#pragma unroll
-    for (int l = 0; l < LPT; ++l) {
-      zs[slot * B + Shape<B, L>::lane_of(sub, l)] = gz[l];
-      us[slot * B + Shape<B, L>::lane_of(sub, l)] = gu[l];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < PPL; ++t) {
-      if (lane + 32 * t < NP) {
-        const int i = pij[t] >> 8, j = pij[t] & 0xff;
-        unsigned long long a = acc[t];
-#pragma unroll
-        for (int rr = 0; rr < RPW; ++rr) {
-          a = mad_wide(zs[rr * B + i], us[rr * B + j], a);
-          if ((rr % FE) == FE - 1) a = fold(a, M);
-        }
-        acc[t] = a;
-      }
-    }
-    __syncwarp();
-  }
-  __device__ __forceinline__ void finish(int, int, int, const ModP&, const uint32_t (&)[3]) {}
-  __device__ __forceinline__ void reset() {
-#pragma unroll
-    for (int t = 0; t < PPL; ++t) acc[t] = 0;
-  }
-  __device__ __forceinline__ void emit(unsigned long long* red, int lane, const ModP& M) {
-#pragma unroll
-    for (int t = 0; t < PPL; ++t) {
-      const int q = lane + 32 * t;
-      if (q < NP) atomicAdd(&red[q], (unsigned long long)reduce(acc[t], M));
-    }
-  }
-};
-
-// D += A * B with A 16x32 u8 (row-major fragments), B 32x8 u8, D 16x8 s32.
-__device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// Tensor cores (B >= 8): exact integer Gram by byte limbs.  Residues are
-// < 2^31, so z = sum_a z_a 256^a with bytes z_a, and
-//   Z^T U = sum_{a,c} 256^{a+c} Z_a^T U_c.
-// A warp stages 32 rows (one K tile) as byte planes P[limb][lane][row] in
-// shared memory -- each row's four limbs are spread over four rows' words with
-// a 4x4 byte transpose across lanes (two shuffles and two byte permutes) --
-// then issues 16 m16n8k32 u8 MMAs per 16x8 output tile.  Per K tile a limb
-// pair's product is < 32 * 255^2 < 2^21, so the shift classes s = a + c stay
-// exact in int32; classes 0..3 are recombined exactly in 64 bits (< 2^48) and
-// classes 4..6 are added with their weights 2^{8s} mod p.
-template <int B, int FE, int L = kDefaultLpt<B>>
-struct GramMma {
-  static constexpr int LPT = Shape<B, L>::LPT, TPR = Shape<B, L>::TPR, RPW = Shape<B, L>::RPW;
-  static constexpr int TB = 32 / RPW;           // batches per K tile
-  static constexpr int BM = B < 16 ? 16 : B;    // rows of the M dimension (zero padded)
-  static constexpr int MT = BM / 16, NT = B / 8;
-  static constexpr int RS = 9;                  // words per (limb, lane) plane row: 32 bytes + 4 pad
-  static constexpr int kPlane = 4 * BM * RS;    // words per plane set
-  static constexpr int kWords = 2 * kPlane;     // shared words per warp
-  uint32_t* pz;
-  uint32_t* pu;
-  unsigned long long acc[MT][NT][4];
-  int bt;
-
-  __device__ __forceinline__ void init(uint32_t* w, int lane) {
-    pz = w;
-    pu = w + kPlane;
-    for (int q = lane; q < kWords; q += 32) w[q] = 0;  // zero padding rows stay zero
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[mt][nt][v] = 0;
-    bt = 0;
-    __syncwarp();
-  }
-
-  // 4x4 byte transpose among the lanes holding rows 4q..4q+3 (lane distance
-  // TPR): afterwards byte k of the word of the lane with row 4q+rho is limb
-  // rho of the value of row 4q+k.
-  __device__ __forceinline__ static uint32_t transpose4(uint32_t w, int rho) {
-    uint32_t p = __shfl_xor_sync(0xffffffffu, w, TPR);
-    w = (rho & 1) ? __byte_perm(p, w, 0x7351) : __byte_perm(w, p, 0x6240);
-    p = __shfl_xor_sync(0xffffffffu, w, 2 * TPR);
-    return (rho & 2) ? __byte_perm(p, w, 0x7632) : __byte_perm(w, p, 0x5410);
-  }
-
-  __device__ __forceinline__ void stage(const uint32_t (&gz)[LPT], const uint32_t (&gu)[LPT], int slot, int sub) {
-    const int rho = slot & 3;
-    const int word = (bt * RPW + (slot & ~3)) >> 2;  // 4-row group inside the K tile
-#pragma unroll
-    for (int l = 0; l < LPT; ++l) {
-      const int i = Shape<B, L>::lane_of(sub, l);
-      pz[(rho * BM + i) * RS + word] = transpose4(gz[l], rho);
-      pu[(rho * BM + i) * RS + word] = transpose4(gu[l], rho);
-    }
-  }
-
-  __device__ __forceinline__ void flush(int lane, const ModP& M, const uint32_t (&W)[3]) {
-    __syncwarp();
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      uint32_t A[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const uint32_t* r0 = pz + (a * BM + mt * 16 + g) * RS;
-        const uint32_t* r1 = r0 + 8 * RS;
-        A[a][0] = r0[t];
-        A[a][1] = r1[t];
-        A[a][2] = r0[t + 4];
-        A[a][3] = r1[t + 4];
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        if (mt * 16 > nt * 8 + 7) continue;  // tile entirely below the diagonal
-        uint32_t Bf[4][2];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint32_t* r = pu + (c * BM + nt * 8 + g) * RS;
-          Bf[c][0] = r[t];
-          Bf[c][1] = r[t + 4];
-        }
-        uint64_t lo[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-          int C[4] = {0, 0, 0, 0};
-#pragma unroll
-          for (int a = 0; a <= s; ++a) mma_u8(C, A[a], Bf[s - a][0], Bf[s - a][1]);
-#pragma unroll
-          for (int v = 0; v < 4; ++v) lo[v] += (uint64_t)(uint32_t)C[v] << (8 * s);
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[mt][nt][v] = fold(acc[mt][nt][v] + lo[v], M);
-#pragma unroll
-        for (int s = 4; s < 7; ++s) {
-          int C[4] = {0, 0, 0, 0};
-#pragma unroll
-          for (int a = s - 3; a < 4; ++a) mma_u8(C, A[a], Bf[s - a][0], Bf[s - a][1]);
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[mt][nt][v] = mad_wide((uint32_t)C[v], W[s - 4], acc[mt][nt][v]);
-        }
-      }
-    }
-    __syncwarp();
-  }
-
-  __device__ __forceinline__ void add(const uint32_t (&gz)[LPT], const uint32_t (&gu)[LPT], int slot, int sub,
-                                      int lane, const ModP& M, const uint32_t (&W)[3]) {
-    stage(gz, gu, slot, sub);
-    if (++bt == TB) {
-      flush(lane, M, W);
-      bt = 0;
-    }
-  }
-
-  __device__ __forceinline__ void reset() {
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[mt][nt][v] = 0;
-    bt = 0;
-  }
-
-  __device__ __forceinline__ void finish(int slot, int sub, int lane, const ModP& M, const uint32_t (&W)[3]) {
-    if (bt == 0) return;
-    uint32_t z[LPT];
-#pragma unroll
-    for (int l = 0; l < LPT; ++l) z[l] = 0;
-    while (bt < TB) {  // zero the rows of the batches the tile did not get
-      stage(z, z, slot, sub);
-      ++bt;
-    }
-    flush(lane, M, W);
-    bt = 0;
-  }
-
-  __device__ __forceinline__ void emit(unsigned long long* red, int lane, const ModP& M) {
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int i = mt * 16 + g + (v >= 2 ? 8 : 0);
-          const int j = nt * 8 + 2 * t + (v & 1);
-          if (i <= j && j < B) atomicAdd(&red[pair_index(i, j, B)], (unsigned long long)reduce(acc[mt][nt][v], M));
-        }
-  }
-};
 
 // Batched mode: where the Gram partials of segment sg go (its own slot for
 // this launch's term, or the segment's shared accumulator); NP = padded pairs.

@@ -588,6 +588,7 @@ __device__ void leaf_eliminate(const LeafBlock& P, uint32_t* sm, const volatile 
             if (c < n) X.rowbuf[rowpar * 32 + c] = sk[cl] == 0 ? of_row<RL>(a[0][cl], a[RL - 1][cl], kr) : 0u;
           }
         }
+        __syncwarp();  // a warp must arrive at a named barrier as one
         elim_bar<EW>();
         const uint32_t v = lane >= rank && lane < n ? X.rowbuf[rowpar * 32 + lst] : 0u;
         rowpar ^= 1;
@@ -611,6 +612,7 @@ __device__ void leaf_eliminate(const LeafBlock& P, uint32_t* sm, const volatile 
 #pragma unroll
           for (int r = 0; r < RL; ++r) X.fb[par * MP + lane + 32 * r] = pick<CPW>(a[r], cs % CPW);
         }
+        __syncwarp();
         elim_bar<EW>();
 #pragma unroll
         for (int r = 0; r < RL; ++r) f[r] = X.fb[par * MP + lane + 32 * r];

@@ -1,0 +1,522 @@
+// resident.cu -- runs of applications of B on matrices that fit the chip: one
+// launch per run, the CSR of A and of A^T in shared memory.
+//
+// Algebra and block layout as in krylov.cu; the run replaces its pass kernels
+// where those are bound by latency: a pass over a 20,000-row matrix moves 2 MB
+// and took 10 us, in launch, dependent loads (offsets, entries, gathers) and
+// the finish of the Gram term, which the next pass waited for.  Here
+//
+//   * every CTA keeps the entries of its rows in shared memory for the whole
+//     run (row batches of equal degree, padded to the longest row, so that an
+//     entry is one conflict-free read);
+//   * a pass is the gathers (from L2: the blocks are rewritten by other SMs),
+//     the row epilogue and one grid barrier;
+//   * a CTA's Gram warps read the rows it has just written and add their Gram
+//     term while the other warps run the next pass; terms go to a slot each and
+//     are reduced mod p once, after the run.
+//
+// Measured (us per application, B200; before: the pass kernels in a CUDA
+// graph): 1500 x 1200, b = 4: 5.7 against 14.1; 20,000^2, b = 8: 7.2 against
+// 21; 30,011 x 23,017, b = 5: 8.1 against 22; 194,003 x 151,007, b = 16:
+// 45 against 63.  The small ones are bound by the barrier and one gather's
+// latency; the last by the rate at which L2 serves random 64-byte rows
+// (8500 gathers per SM and pass, 4.2 TB/s in all).
+//
+// The grid barrier gives up after 2 s of %globaltimer and sets *status.
+#include <algorithm>
+#include <mutex>
+
+#include "krylov_gram.cuh"
+
+namespace rr {
+
+namespace {
+
+constexpr int kGatherWarps = 16;
+// Gram warps: at width 16 four of them take longer than a pass of the largest
+// matrices that fit.
+template <int B>
+constexpr int kGramWarps = B >= 16 ? 8 : 4;
+template <int B>
+constexpr int kResThreads = 32 * (kGatherWarps + kGramWarps<B>);
+constexpr int kMaxBatches = 512;  // row batches of one CTA, per matrix
+constexpr int64_t kResMaxDegree = 64;
+constexpr uint64_t kBarrierNs = 2000000000ull;
+constexpr size_t kResSmem = 227 * 1024 - 2048;
+
+struct ResCsr {
+  const uint32_t* rowptr;
+  const uint2* cv;
+  int64_t rows;
+};
+
+struct ResParams {
+  ResCsr A, At;
+  uint4* X[2];
+  uint4* U;
+  int cur0;
+  int apps;
+  const uint32_t *dr_m, *dc_m, *dc_r, *drinv_r, *dcinv_r;
+  unsigned long long* gram;  // [2 apps][NP], zero at launch
+  unsigned int* bar;         // arrivals, zero at launch
+  int* status;
+  ModP M;
+  uint32_t w4, w5, w6;
+};
+
+__device__ __forceinline__ uint64_t res_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void gather_bar() { __barrier_sync_count(1, 32 * kGatherWarps); }
+template <int B>
+__device__ __forceinline__ void gram_bar() {
+  __barrier_sync_count(2, 32 * kGramWarps<B>);
+}
+
+__device__ __forceinline__ uint32_t redc_c(uint64_t T, const ModP& M) {  // T < p 2^32
+  const uint32_t q = (uint32_t)T * M.pinv;
+  const uint32_t t = (uint32_t)(((uint64_t)q * M.p + T) >> 32);
+  return min(t, t - M.p);
+}
+
+// The entries of a CTA's row batches (batch j of the CTA = batch blockIdx.x +
+// j gridDim.x of the matrix), batch after batch, [step][slot] with zero entries
+// past a row's end.  first[j] = the batch's first entry, first[count] = the end.
+template <int B>
+__device__ int load_entries(const ResCsr& C, uint2* ell, int* first) {
+  constexpr int RPW = 128 / B;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t nbatch = (C.rows + RPW - 1) / RPW;
+  const int count = blockIdx.x < nbatch ? (int)((nbatch - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
+  // rows are in decreasing degree order: the first row of a batch is its longest
+  for (int j = tid; j < count; j += kResThreads<B>) {
+    const int64_t r = ((int64_t)blockIdx.x + (int64_t)j * gridDim.x) * RPW;
+    first[j + 1] = (int)(C.rowptr[r + 1] - C.rowptr[r]) * RPW;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int base = 0;
+    for (int j0 = 0; j0 < count; j0 += 32) {
+      int v = j0 + lane < count ? first[j0 + lane + 1] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (j0 + lane < count) first[j0 + lane + 1] = base + v;
+      base += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) first[0] = 0;
+  }
+  __syncthreads();
+  for (int j = warp; j < count; j += kResThreads<B> / 32) {
+    const int64_t r0 = ((int64_t)blockIdx.x + (int64_t)j * gridDim.x) * RPW;
+    const int b0 = first[j], len = first[j + 1] - b0;
+    for (int e = lane; e < len; e += 32) {
+      const int64_t r = r0 + e % RPW;
+      uint2 v = make_uint2(0u, 0u);
+      if (r < C.rows) {
+        const uint32_t k = C.rowptr[r] + (uint32_t)(e / RPW);
+        if (k < C.rowptr[r + 1]) v = C.cv[k];
+      }
+      ell[b0 + e] = v;
+    }
+  }
+  return count;
+}
+
+// acc += val * g for the four lanes of each of the first `n` loaded entries
+template <int N>
+__device__ __forceinline__ void mac_entries(const uint2 (&e)[N], const uint4 (&g)[N], const ModP& M, uint64_t (&acc)[4]) {
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    acc[0] += (uint64_t)e[u].y * g[u].x;
+    acc[1] += (uint64_t)e[u].y * g[u].y;
+    acc[2] += (uint64_t)e[u].y * g[u].z;
+    acc[3] += (uint64_t)e[u].y * g[u].w;
+    if ((u & 3) == 3) {  // four products fit between folds for every p < 2^31
+#pragma unroll
+      for (int l = 0; l < 4; ++l) acc[l] = fold(acc[l], M);
+    }
+  }
+}
+
+// One pass of the gather warps over the CTA's row batches: Y = scaled rows of C X.
+template <int B, bool EVEN>
+__device__ __forceinline__ void res_pass(const ResCsr& C, const uint2* ell, const int* first, int count, const uint4* X,
+                                         uint4* Y, const uint32_t* __restrict__ scale,
+                                         const uint32_t* __restrict__ scale2, const ModP& M) {
+  constexpr int TPR = B / 4, RPW = 32 / TPR;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % TPR, slot = lane / TPR;
+  const uint4* Xs = X + sub;
+  for (int j = warp; j < count; j += kGatherWarps) {
+    const int64_t r = ((int64_t)blockIdx.x + (int64_t)j * gridDim.x) * RPW + slot;
+    const bool on = r < C.rows;
+    const uint32_t s1 = on ? __ldg(scale + r) : 0u;
+    const uint32_t s2 = EVEN && on ? __ldg(scale2 + r) : 0u;
+    const uint2* ep = ell + first[j] + slot;
+    int left = (first[j + 1] - first[j]) / RPW;
+    uint64_t acc[4] = {0, 0, 0, 0};
+    for (; left >= 8; left -= 8, ep += 8 * RPW) {
+      uint2 e[8];
+      uint4 g[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) e[u] = ep[u * RPW];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) g[u] = __ldcg(Xs + (size_t)e[u].x * TPR);
+      mac_entries<8>(e, g, M, acc);
+    }
+    if (left > 0) {  // the same count in every lane
+      uint2 e[7];
+      uint4 g[7];
+#pragma unroll
+      for (int u = 0; u < 7; ++u) e[u] = u < left ? ep[u * RPW] : make_uint2(0u, 0u);
+#pragma unroll
+      for (int u = 0; u < 7; ++u) {
+        g[u] = make_uint4(0, 0, 0, 0);
+        if (u < left) g[u] = __ldcg(Xs + (size_t)e[u].x * TPR);
+      }
+      mac_entries<7>(e, g, M, acc);
+    }
+    if (on) {
+      uint32_t o[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        o[l] = redc_c((uint64_t)redc_c(fold(acc[l], M), M) * s1, M);  // d_r z, or w'
+        if (EVEN) o[l] = redc_c((uint64_t)o[l] * s2, M);              // d_c w'
+      }
+      __stcg(Y + r * TPR + sub, make_uint4(o[0], o[1], o[2], o[3]));
+    }
+  }
+}
+
+// The Gram term of the CTA's rows of Y: odd z (x) Y with z = Y d_r^{-1}, even
+// w (x) w with w = Y d_c^{-1}.  Four batches are loaded before the first is used.
+template <int B, bool EVEN, class Gram>
+__device__ __forceinline__ void res_gram(Gram& gram, int64_t rows, int count, const uint4* Y,
+                                         const uint32_t* __restrict__ inv, const ModP& M, const uint32_t (&W)[3],
+                                         uint32_t* part, unsigned long long* out) {
+  constexpr int TPR = B / 4, RPW = 32 / TPR;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) - kGatherWarps, sub = lane % TPR, slot = lane / TPR;
+  for (int j0 = warp; j0 < count; j0 += 4 * kGramWarps<B>) {
+    uint4 y[4];
+    uint32_t s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = j0 + u * kGramWarps<B>;
+      const int64_t r = ((int64_t)blockIdx.x + (int64_t)j * gridDim.x) * RPW + slot;
+      const bool on = j < count && r < rows;
+      y[u] = on ? __ldcg(Y + r * TPR + sub) : make_uint4(0, 0, 0, 0);
+      s[u] = on ? __ldg(inv + r) : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (j0 + u * kGramWarps<B> >= count) break;
+      const uint32_t v[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
+      uint32_t z[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) z[l] = redc_c((uint64_t)v[l] * s[u], M);
+      if (EVEN) gram.add_sym(z, slot, sub, lane, M, W);
+      else gram.add(z, v, slot, sub, lane, M, W);
+    }
+  }
+  if (EVEN) gram.finish_sym(slot, sub, lane, M, W);
+  else gram.finish(slot, sub, lane, M, W);
+  gram.store(part + warp * B * B, lane, M);
+  gram.reset();
+  gram_bar<B>();
+  for (int e = threadIdx.x - 32 * kGatherWarps; e < B * B; e += 32 * kGramWarps<B>) {
+    const int i = e / B, c = e % B;
+    if (i <= c) {
+      unsigned long long v = 0;
+#pragma unroll
+      for (int w = 0; w < kGramWarps<B>; ++w) v += part[w * B * B + e];
+      if (v) atomicAdd(out + pair_index(i, c, B), v);
+    }
+  }
+  gram_bar<B>();
+}
+
+template <int B>
+using ResGram = typename std::conditional<(B >= 8), GramMma<B, 4, 4>, GramCore<B, 4, 4>>::type;
+
+template <int B>
+constexpr size_t res_fixed_smem() {  // Gram staging, the Gram warps' sums, batch offsets
+  return (size_t)4 * kGramWarps<B> * (ResGram<B>::kWords + B * B) + 4 * 2 * (kMaxBatches + 2);
+}
+
+template <int B>
+__global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P, int entriesA) {
+  constexpr int NP = B * (B + 1) / 2;
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  __shared__ int s_stop;
+  uint2* const ellA = reinterpret_cast<uint2*>(res_smem + res_fixed_smem<B>());
+  uint2* const ellAt = ellA + entriesA;
+  uint32_t* const staging = reinterpret_cast<uint32_t*>(res_smem);
+  uint32_t* const part = staging + (size_t)kGramWarps<B> * ResGram<B>::kWords;
+  int* const firstA = reinterpret_cast<int*>(part + kGramWarps<B> * B * B);
+  int* const firstAt = firstA + kMaxBatches + 2;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const ModP M = P.M;
+  if (tid == 0) s_stop = 0;
+  const int nA = load_entries<B>(P.A, ellA, firstA);
+  const int nAt = load_entries<B>(P.At, ellAt, firstAt);
+  __syncthreads();
+  if (warp < kGatherWarps) {
+    int cur = P.cur0;
+    unsigned int target = 0;
+    for (int p = 0; p < 2 * P.apps; ++p) {
+      if ((p & 1) == 0) {
+        res_pass<B, false>(P.A, ellA, firstA, nA, P.X[cur], P.U, P.dr_m, nullptr, M);
+      } else {
+        res_pass<B, true>(P.At, ellAt, firstAt, nAt, P.U, P.X[cur ^ 1], P.dc_m, P.dc_r, M);
+        cur ^= 1;
+      }
+      __syncthreads();  // the rows are written, and the Gram warps are done with the previous pass
+      if (p + 1 == 2 * P.apps) break;
+      target += gridDim.x;
+      if (tid == 0) {
+        // one arrival per CTA; all CTAs wait on the same word (a release word of
+        // its own, written by the last to arrive, was 2 us slower per application)
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.bar) : "memory");
+        uint64_t t0 = 0;
+        for (int spins = 0;; ++spins) {
+          unsigned int seen;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(P.bar) : "memory");
+          if (seen >= target) break;
+          if ((spins & 255) == 255) {
+            const uint64_t t = res_ns();
+            if (t0 == 0) t0 = t;
+            if (*(volatile int*)P.status || t - t0 > kBarrierNs) {
+              atomicExch(P.status, 1);
+              s_stop = 1;
+              break;
+            }
+          }
+        }
+      }
+      gather_bar();
+      if (*(volatile int*)&s_stop) {
+        __syncthreads();  // the Gram warps leave here too
+        break;
+      }
+    }
+  } else {
+    ResGram<B> gram;
+    gram.init(staging + (size_t)(warp - kGatherWarps) * ResGram<B>::kWords, lane);
+    const uint32_t W[3] = {P.w4, P.w5, P.w6};
+    int cur = P.cur0;
+    for (int p = 0; p < 2 * P.apps; ++p) {
+      __syncthreads();
+      if (*(volatile int*)&s_stop) break;
+      unsigned long long* out = P.gram + (size_t)p * NP;
+      if ((p & 1) == 0) {
+        res_gram<B, false>(gram, P.A.rows, nA, P.U, P.drinv_r, M, W, part, out);
+      } else {
+        res_gram<B, true>(gram, P.At.rows, nAt, P.X[cur ^ 1], P.dcinv_r, M, W, part, out);
+        cur ^= 1;
+      }
+    }
+  }
+}
+
+// Cooperative grids of one device.  Grids that together need more SMs than
+// there are must not be in flight together: each could hold some SMs and wait
+// for the rest.  Runs of the whole device follow one another through an event;
+// runs of a share of it (the lanes of a rank service, 1 / kCoopShares of the
+// SMs at most) follow the runs of the same share and of the whole device.  None
+// is queued while a batch holds the device.
+struct CoopChain {
+  std::mutex m;
+  cudaEvent_t done[kCoopShares + 1] = {};  // the last run of each share, and of the whole device
+  int holds = 0;                           // batches with persistent launches in flight
+  // stream s waits for the last run of share q (an event never recorded does not wait)
+  int wait(cudaStream_t s, int q) {
+    if (done[q]) RR_CUDA(cudaStreamWaitEvent(s, done[q], 0));
+    return RR_OK;
+  }
+};
+constexpr int kMaxDevices = 64;
+CoopChain g_coop[kMaxDevices];
+
+class CoopTurn {
+ public:
+  // share < 0: the whole device
+  int begin(int device, cudaStream_t s, int share, bool* taken) {
+    *taken = false;
+    if (device < 0 || device >= kMaxDevices) return RR_OK;
+    chain_ = &g_coop[device];
+    chain_->m.lock();
+    if (chain_->holds > 0) return RR_OK;
+    share_ = share < 0 ? kCoopShares : share;
+    if (!chain_->done[share_]) RR_CUDA(cudaEventCreateWithFlags(&chain_->done[share_], cudaEventDisableTiming));
+    for (int q = 0; q <= kCoopShares; ++q)
+      if (share < 0 || q == share_ || q == kCoopShares) RR_TRY(chain_->wait(s, q));
+    stream_ = s;
+    *taken = true;
+    return RR_OK;
+  }
+  int end() {
+    RR_CUDA(cudaEventRecord(chain_->done[share_], stream_));
+    return RR_OK;
+  }
+  ~CoopTurn() {
+    if (chain_) chain_->m.unlock();
+  }
+
+ private:
+  CoopChain* chain_ = nullptr;
+  cudaStream_t stream_ = nullptr;
+  int share_ = 0;
+};
+
+// Gram sums of `terms` terms -> sequence terms (real pairs); the sums, the
+// barrier and the device term counter are made ready for the next launch.
+__global__ void resident_finish_kernel(unsigned long long* gram, int terms, int b, int B, uint32_t* S,
+                                       unsigned int* term_ctr, unsigned int* bar, ModP M) {
+  const int NP = B * (B + 1) / 2, npr = b * (b + 1) / 2;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < terms * NP; e += gridDim.x * blockDim.x) {
+    const int t = e / NP;
+    int i, j;
+    pair_of(e - t * NP, B, i, j);
+    if (j < b) S[(size_t)t * npr + pair_index(i, j, b)] = reduce(gram[e], M);
+    gram[e] = 0;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *term_ctr += (unsigned)terms;
+    *bar = 0;
+  }
+}
+
+// Entries of a CTA for one matrix, at most: the row batches of a CTA are every
+// grid-th one of a list of non-increasing lengths, so all but its first are
+// bounded by the mean of the lengths before them.
+int64_t entry_bound(int64_t nnz, int64_t max_degree, int rpw, int grid) {
+  return rpw * max_degree + (nnz + rpw * max_degree) / grid + 1;
+}
+
+template <int B>
+int prepare(rr_krylov* kr) {
+  constexpr int RPW = 128 / B;
+  const rr_matrix* mat = kr->mat;
+  const int64_t degA = mat->max_row_nnz, degAt = mat->max_col_nnz;
+  kr->res_grid = 0;
+  if (degA > kResMaxDegree || degAt > kResMaxDegree) return RR_OK;
+  const int64_t batches = (std::max(mat->m, mat->n) + RPW - 1) / RPW;
+  // a share of the device where the context has one and the matrix fits it
+  const int sms = mat->ctx->num_sms, share = mat->ctx->coop_share;
+  for (int cap : {share < 0 ? sms : sms / kCoopShares, sms}) {
+    const int grid = (int)std::min<int64_t>(batches, cap);
+    if ((batches + grid - 1) / grid > kMaxBatches) continue;
+    const int64_t ea = entry_bound(mat->nnz, degA, RPW, grid), et = entry_bound(mat->nnz, degAt, RPW, grid);
+    const size_t smem = res_fixed_smem<B>() + 8 * (size_t)(ea + et);
+    if (smem > kResSmem) continue;
+    kr->res_grid = grid;
+    kr->res_entriesA = (int)ea;
+    kr->res_smem = smem;
+    kr->res_share = cap < sms ? share : -1;
+    break;
+  }
+  if (kr->res_grid == 0) return RR_OK;
+  // the limit is per kernel, shared by every thread of the process: always the largest
+  RR_CUDA(cudaFuncSetAttribute(resident_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
+  cudaStream_t s = mat->ctx->stream;
+  RR_TRY(kr->res_gram.alloc_async((size_t)2 * kResMaxApps * (B * (B + 1) / 2), s));
+  RR_CUDA(cudaMemsetAsync(kr->res_gram.ptr, 0, kr->res_gram.bytes(), s));
+  RR_TRY(kr->res_bar.alloc_async(1, s));
+  RR_CUDA(cudaMemsetAsync(kr->res_bar.ptr, 0, kr->res_bar.bytes(), s));
+  return RR_OK;
+}
+
+template <int B>
+int run(rr_krylov* kr, int apps, bool* taken) {
+  const rr_matrix* mat = kr->mat;
+  cudaStream_t s = mat->ctx->stream;
+  ResParams P;
+  P.A = ResCsr{mat->A.rowptr.ptr, mat->A.cv.ptr, mat->A.rows};
+  P.At = ResCsr{mat->At.rowptr.ptr, mat->At.cv.ptr, mat->At.rows};
+  P.X[0] = reinterpret_cast<uint4*>(kr->X[0].ptr);
+  P.X[1] = reinterpret_cast<uint4*>(kr->X[1].ptr);
+  P.U = reinterpret_cast<uint4*>(kr->U.ptr);
+  P.cur0 = kr->cur;
+  P.apps = apps;
+  P.dr_m = kr->dr_m.ptr;
+  P.dc_m = kr->dc_m.ptr;
+  P.dc_r = kr->dc_r.ptr;
+  P.drinv_r = kr->drinv_r.ptr;
+  P.dcinv_r = kr->dcinv_r.ptr;
+  P.gram = kr->res_gram.ptr;
+  P.bar = kr->res_bar.ptr;
+  P.status = kr->d_status.ptr;
+  P.M = kr->M;
+  P.w4 = kr->M.c32;
+  P.w5 = (uint32_t)((uint64_t)P.w4 * 256 % kr->M.p);
+  P.w6 = (uint32_t)((uint64_t)P.w5 * 256 % kr->M.p);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)kr->res_grid);
+  cfg.blockDim = dim3(kResThreads<B>);
+  cfg.dynamicSmemBytes = kr->res_smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  {
+    CoopTurn turn;
+    RR_TRY(turn.begin(mat->ctx->device, s, kr->res_share, taken));
+    if (!*taken) return RR_OK;
+    RR_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel<B>, P, kr->res_entriesA));
+    RR_TRY(turn.end());
+  }
+  const int np = kr->b * (kr->b + 1) / 2, NP = B * (B + 1) / 2;
+  resident_finish_kernel<<<std::min((2 * apps * NP + 255) / 256, 296), 256, 0, s>>>(
+      kr->res_gram.ptr, 2 * apps, kr->b, B, kr->S.ptr + (size_t)(kr->len - kr->base) * np, kr->d_term.ptr,
+      kr->res_bar.ptr, kr->M);
+  RR_CUDA(cudaGetLastError());
+  kr->launches += 2;
+  kr->len += 2 * apps;
+  kr->cur ^= apps & 1;
+  return RR_OK;
+}
+
+}  // namespace
+
+int CoopHold::begin(int device, cudaStream_t s) {
+  if (device < 0 || device >= kMaxDevices) return RR_OK;
+  CoopChain& c = g_coop[device];
+  std::lock_guard<std::mutex> lk(c.m);
+  for (int q = 0; q <= kCoopShares; ++q) RR_TRY(c.wait(s, q));
+  device_ = device;
+  ++c.holds;
+  return RR_OK;
+}
+
+CoopHold::~CoopHold() {
+  if (device_ < 0) return;
+  std::lock_guard<std::mutex> lk(g_coop[device_].m);
+  --g_coop[device_].holds;
+}
+
+int resident_prepare(rr_krylov* kr) {
+  switch (kr->B) {
+    case 4: return prepare<4>(kr);
+    case 8: return prepare<8>(kr);
+    case 16: return prepare<16>(kr);
+  }
+  kr->res_grid = 0;
+  return RR_OK;
+}
+
+int resident_run(rr_krylov* kr, int apps, bool* taken) {
+  switch (kr->B) {
+    case 4: return run<4>(kr, apps, taken);
+    case 8: return run<8>(kr, apps, taken);
+    case 16: return run<16>(kr, apps, taken);
+  }
+  return fail(RR_EINVAL, "no resident run at width %d", kr->B);
+}
+
+}  // namespace rr

@@ -132,6 +132,7 @@ struct rr_ctx_s {
   int device = 0;
   cudaStream_t stream = nullptr;
   int num_sms = 0;
+  int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
   int pm_tensor_cores = 1;  // PM-basis contractions on the int8 tensor cores (0: CUDA cores)
 };
 
@@ -209,6 +210,12 @@ struct rr_krylov_s {
   cudaStream_t launch_stream = nullptr;  // set while capturing (a private stream), else the context's
   int graph_cur = 0;
   int64_t graph_launches = 0;
+  // runs with the CSR in shared memory (resident.cu): CTAs (0 = the matrix does
+  // not fit), entries of A per CTA, dynamic shared memory, Gram sums, barrier
+  int res_grid = 0, res_entriesA = 0, res_share = -1;
+  size_t res_smem = 0;
+  rr::DevBuf<unsigned long long> res_gram;
+  rr::DevBuf<unsigned int> res_bar;
   ~rr_krylov_s() {
     if (graph) cudaGraphExecDestroy(graph);
   }
@@ -219,6 +226,24 @@ int krylov_launch_init(rr_krylov* kr, const uint32_t* d_w, bool emit_s0);
 int krylov_reserve(rr_krylov* kr, int64_t terms);
 int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev);
 int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out);
+// Runs of applications in one launch with the CSR in shared memory
+// (resident.cu): resident_prepare sets kr->res_grid where the matrix fits, and
+// resident_run then takes 1 <= apps <= kResMaxApps applications at once, or
+// none (*taken = false) while a batch holds the device.
+constexpr int kResMaxApps = 512;
+constexpr int kCoopShares = 4;  // shares of a device for runs side by side (rr_ctx::coop_share)
+int resident_prepare(rr_krylov* kr);
+int resident_run(rr_krylov* kr, int apps, bool* taken);
+// Held while persistent launches of a batch may be in flight on stream s: no
+// resident run is queued meanwhile, and the stream waits for the last one.
+class CoopHold {
+ public:
+  int begin(int device, cudaStream_t s);
+  ~CoopHold();
+
+ private:
+  int device_ = -1;
+};
 int krylov_occupancy(rr_krylov* kr);
 // Sequence length rule of src/main.rs:497-504; padded block width; device
 // bytes a matrix and its Krylov state hold while resident (server.cpp).

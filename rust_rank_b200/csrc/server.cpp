@@ -432,6 +432,7 @@ int rr_server_create(int device, const rr_server_config* cfg, rr_server** out) {
       for (rr_ctx* x : s->lanes) rr_ctx_destroy(x);
       return rc;
     }
+    if (s->cfg.lanes > 1) c->coop_share = l % rr::kCoopShares;  // the lanes' runs side by side
     s->lanes.push_back(c);
     s->lane_load.push_back(0);
   }
