@@ -197,9 +197,9 @@ __device__ __forceinline__ void gather_sum8(const uint2* __restrict__ cv, uint32
   }
 }
 
-// Programmatic dependent launch: the single-matrix kernels are launched so
-// that the next kernel of an application may be scheduled while the previous
-// one finishes.  griddep_wait() blocks until the previous kernel has completed
+// Programmatic dependent launch: the single-matrix kernels may be launched so
+// that the next kernel of an application is scheduled while the previous one
+// finishes (launch_ex).  griddep_wait() blocks until the previous kernel has completed
 // and its writes are visible (it returns at once for a normal launch), so every
 // such kernel calls it before reading what its predecessor wrote;
 // griddep_launch() tells the scheduler a CTA has no more main-loop work.
@@ -1149,6 +1149,9 @@ static int pass_grid_lean(const rr_krylov* kr, int64_t rows) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(kr->grid_lean, need));
 }
 
+// Gathered bytes per pass up to which the kernels of an application overlap.
+constexpr double kOverlapBytes = 32e6;
+
 // Kernel launches of the single-matrix path, through cudaLaunchKernelEx.
 template <class... Args>
 static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 block, size_t smem,
@@ -1158,14 +1161,22 @@ static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 b
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  // the kernel may be scheduled while its predecessor on the stream finishes;
-  // it waits for it (griddep_wait) before reading the predecessor's output
+  // In small applications the kernel may be scheduled while its predecessor on
+  // the stream finishes; it waits for it (griddep_wait) before reading the
+  // predecessor's output.  In large ones that costs more than it hides: an SM
+  // that goes from a Gram pass or a fused pass (200 or 150 KB of shared memory)
+  // straight to a gathering kernel keeps its shared-memory carve-out, and the
+  // gathers lose most of their L1.  Measured (us per application, overlapped /
+  // not): 1M x 750k Zipf, b = 32: 590 / 453 (its chunks 209 / 144); 190k x 150k,
+  // b = 32: 119 / 104; 600k x 500k, b = 16: 155 / 148; 2M Zipf, b = 16: 543 /
+  // 536, b = 5: 373 / 362; but 60k x 50k Zipf, b = 4 (8 MB gathered a pass):
+  // 28.9 / 30.6.
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed =
+      4.0 * (double)kr->mat->nnz * kr->B <= kOverlapBytes ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  (void)kr;
   RR_CUDA(cudaLaunchKernelEx(&cfg, fn, args...));
   return RR_OK;
 }
