@@ -25,18 +25,20 @@
 //   * m_k = D1 T + x Dx T is applied to the residual series and to the block's
 //     accumulated basis.
 //
-// Products above the blocks are exact NTT products modulo p itself (p must
-// admit the transform length), which equal the reference's exact integer
-// products reduced mod p.  NTTs are decimation-in-frequency forward (natural
-// in, bit-reversed out) and decimation-in-time inverse (bit-reversed in,
-// natural out), so no bit-reversal pass is needed; twiddles use Shoup's
-// precomputed quotients.
+// Products above the blocks are formed directly on the tensor cores while they
+// are short (pmproduct.cu), then by exact NTT products modulo p itself where p
+// admits the transform length, else modulo two or three NTT primes joined by
+// CRT; all equal the reference's exact integer products reduced mod p.  NTTs are
+// decimation-in-frequency forward (natural in, bit-reversed out) and
+// decimation-in-time inverse (bit-reversed in, natural out), so no bit-reversal
+// pass is needed; twiddles use Shoup's precomputed quotients.
 #include <algorithm>
 #include <cstring>
 #include <memory>
 #include <mutex>
 
 #include "pmleaf.h"
+#include "pmproduct.h"
 
 namespace rr {
 
@@ -270,12 +272,12 @@ __global__ void crt_kernel(const uint32_t* __restrict__ R0, const uint32_t* __re
 // Pointwise stage: C[i][j][f] = sum_r A[i][r][f] * B[r][j][f]  (all N-length),
 // for nb matrices stored one after the other.  A thread computes a 4 x 4 tile
 // of (i, j) at one frequency (consecutive threads take consecutive
-// frequencies, so every load is coalesced), 16 carry-chain accumulators,
-// folded every 4 steps (every 2 for primes where 4 products do not fit).  m and k are multiples of 4 here (m = 2b, k in {b, 2b}
-// with b a multiple of 4); pointwise1_kernel covers the rest.
+// frequencies, so every load is coalesced) in 16 64-bit accumulators.  m, r and
+// k are multiples of 4 here (m = r = 2b, k in {b, 2b} with b a multiple of 4);
+// pointwise1_kernel covers the rest.
 __global__ void __launch_bounds__(256) pointwise_kernel(const uint32_t* __restrict__ A, const uint32_t* __restrict__ Bm,
                                                         uint32_t* __restrict__ C, int m, int r, int k, int64_t N, int nb,
-                                                        int fold_mask, ModP M) {
+                                                        ModP M) {
   const int ti = m / 4, tj = k / 4;
   const int64_t per = (int64_t)ti * tj * N;
   const int64_t total = per * nb;
@@ -286,38 +288,34 @@ __global__ void __launch_bounds__(256) pointwise_kernel(const uint32_t* __restri
     const int i0 = 4 * (int)(tile / tj), j0 = 4 * (int)(tile % tj);
     const uint32_t* a = A + bi * (int64_t)m * r * N + (int64_t)i0 * r * N + f;
     const uint32_t* b = Bm + bi * (int64_t)r * k * N + (int64_t)j0 * N + f;
-    uint32_t lo[4][4], hi[4][4];
+    uint64_t acc[4][4];
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 4; ++y) lo[x][y] = hi[x][y] = 0;
-    for (int s = 0; s < r; ++s) {
-      uint32_t av[4], bv[4];
+      for (int y = 0; y < 4; ++y) acc[x][y] = 0;
+    for (int s = 0; s < r; s += 4) {  // r is a multiple of 4; four products fit between folds for every prime < 2^31
 #pragma unroll
-      for (int x = 0; x < 4; ++x) av[x] = a[(int64_t)x * r * N + (int64_t)s * N];
+      for (int u = 0; u < 4; ++u) {
+        uint32_t av[4], bv[4];
 #pragma unroll
-      for (int y = 0; y < 4; ++y) bv[y] = b[(int64_t)s * k * N + (int64_t)y * N];
+        for (int x = 0; x < 4; ++x) av[x] = a[(int64_t)x * r * N + (int64_t)(s + u) * N];
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) mac_cc(av[x], bv[y], lo[x][y], hi[x][y]);
-      if ((s & fold_mask) == fold_mask) {  // fold (hi:lo) -> hi * (2^32 mod p) + lo every 4 (or 2) products
+        for (int y = 0; y < 4; ++y) bv[y] = b[(int64_t)(s + u) * k * N + (int64_t)y * N];
 #pragma unroll
         for (int x = 0; x < 4; ++x)
 #pragma unroll
-          for (int y = 0; y < 4; ++y) {
-            const uint32_t h = hi[x][y];
-            hi[x][y] = 0;
-            mac_cc(h, M.c32, lo[x][y], hi[x][y]);
-          }
+          for (int y = 0; y < 4; ++y) acc[x][y] += (uint64_t)av[x] * bv[y];
       }
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) acc[x][y] = fold(acc[x][y], M);
     }
     uint32_t* c = C + bi * (int64_t)m * k * N + (int64_t)i0 * k * N + (int64_t)j0 * N + f;
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int y = 0; y < 4; ++y)
-        c[(int64_t)x * k * N + (int64_t)y * N] = reduce(((uint64_t)hi[x][y] << 32) | lo[x][y], M);
+      for (int y = 0; y < 4; ++y) c[(int64_t)x * k * N + (int64_t)y * N] = reduce(acc[x][y], M);
   }
 }
 
@@ -345,33 +343,46 @@ __global__ void pointwise1_kernel(const uint32_t* __restrict__ A, const uint32_t
   }
 }
 
-// Direct product for moduli without a suitable NTT: dst coefficient lo + t of
-// sum_s A[i][s] * B[s][j], one thread per output coefficient.
-__global__ void schoolbook_kernel(const uint32_t* A, int mA, int r, int64_t la, int64_t a_rs, int64_t a_cs,
-                                  int64_t a_bs, const uint32_t* Bm, int k, int64_t lb, int64_t b_rs, int64_t b_cs,
-                                  int64_t b_bs, uint32_t* dst, int64_t d_rs, int64_t d_cs, int64_t d_bs, int64_t lo,
-                                  int64_t cnt, int nb, ModP M) {
-  const int64_t per = (int64_t)mA * k * cnt;
-  const int64_t total = per * nb;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t bi = t / per, tt = t % per;
-    const int64_t c = lo + tt % cnt;
-    const int64_t ij = tt / cnt;
-    const int i = (int)(ij / k), j = (int)(ij % k);
-    uint64_t acc = 0;
-    int parity = 0;
-    for (int s = 0; s < r; ++s) {
-      const uint32_t* a = A + bi * a_bs + (int64_t)i * a_rs + (int64_t)s * a_cs;
-      const uint32_t* b = Bm + bi * b_bs + (int64_t)s * b_rs + (int64_t)j * b_cs;
-      const int64_t u0 = c - (lb - 1) > 0 ? c - (lb - 1) : 0;
-      const int64_t u1 = c < la - 1 ? c : la - 1;
-      for (int64_t u = u0; u <= u1; ++u) {
-        acc = mad_wide(a[u], b[c - u], acc);
-        if (++parity == 2) { acc = fold(acc, M); parity = 0; }
-      }
-    }
-    dst[bi * d_bs + (int64_t)i * d_rs + (int64_t)j * d_cs + (c - lo)] = reduce(acc, M);
+// A product of two factors of degree h read off a cyclic transform of length
+// 2h: position 0 holds C[0] + C[2h].  C[2h] = A[h] B[h] is formed directly and
+// taken off again.
+__global__ void unwrap_kernel(PolyView A, PolyView Bm, PolyView dst, int m, int r, int k, int64_t h, int64_t npoly,
+                              ModP M) {
+  const int lane = threadIdx.x & 31;  // a warp per entry of C, a lane per term
+  const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= npoly) return;
+  const int64_t z = q / ((int64_t)m * k);
+  const int i = (int)(q / k % m), j = (int)(q % k);
+  uint32_t top = 0;
+  for (int s = lane; s < r; s += 32)
+    top = addmod(top, mulmod(A.at(z * m * r + (int64_t)i * r + s)[h], Bm.at(z * r * k + (int64_t)s * k + j)[h], M), M.p);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) top = addmod(top, __shfl_xor_sync(0xffffffffu, top, o), M.p);
+  if (lane == 0) {
+    uint32_t* d = dst.at(q);
+    d[2 * h] = top;
+    d[0] = submod(d[0], top, M.p);
   }
+}
+
+// Twiddle tables of a transform prime: w^j and w^-j with their Shoup quotients.
+__global__ void twiddle_kernel(uint32_t* tw, uint32_t* tws, uint32_t* twi, uint32_t* twis, int64_t half, uint32_t w,
+                               uint32_t wi, ModP M) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= half) return;
+  uint32_t x = 1, y = 1, bx = w, by = wi;
+  for (int64_t e = j; e; e >>= 1) {
+    if (e & 1) {
+      x = mulmod(x, bx, M);
+      y = mulmod(y, by, M);
+    }
+    bx = mulmod(bx, bx, M);
+    by = mulmod(by, by, M);
+  }
+  tw[j] = x;
+  twi[j] = y;
+  tws[j] = (uint32_t)(((uint64_t)x << 32) / M.p);
+  twis[j] = (uint32_t)(((uint64_t)y << 32) / M.p);
 }
 
 // G[i][j][t] = seq[pair(i,j)][t] for i < b; G[b+i][i][0] = 1 (src/sigma_basis.rs:33-46)
@@ -1071,7 +1082,6 @@ int grid_for(int64_t work, int threads = 256) {
 struct NttPrime {
   uint32_t q = 0;
   ModP M{};
-  int fold4 = 0;
   int64_t nmax = 0;
   DevBuf<uint32_t> tw, tws, twi, twis;
   Twiddles fwd() const { return Twiddles{tw.ptr, tws.ptr, nmax}; }
@@ -1107,6 +1117,7 @@ struct Pm {
   bool crt = false;
   DevBuf<uint32_t> R[3];                // CRT residues [nb][m*m][d+1] per prime
   DevBuf<uint32_t> FA, FB, FC;          // [nb][m*m][nmax]
+  std::vector<std::unique_ptr<DevBuf<uint32_t>>> FM;  // per depth: the transform of MM, [nb][m*m][2h]
   DevBuf<uint32_t> Tt;                  // leaf transforms of one block [nb][K][m][m]
   DevBuf<unsigned long long> leafmask;  // [nb][K]
   DevBuf<uint32_t> sigma_inv;           // [nb][m]
@@ -1196,18 +1207,18 @@ int ntt_inverse(Pm& P, const NttPrime& Q, uint32_t* a, int64_t N, PolyView dst, 
   return RR_OK;
 }
 
-// One NTT product modulo the transform prime Q: coefficients [lo, lo + cnt)
-// of A * B into dst.
-int ntt_product(Pm& P, const NttPrime& Q, MatView A, int mA, int r, int64_t la, MatView B, int k, int64_t lb,
-                int64_t N, PolyView dst, int64_t lo, int64_t cnt) {
-  RR_TRY(ntt_forward(P, Q, P.FA.ptr, N, A.polys(r, mA), la));
-  RR_TRY(ntt_forward(P, Q, P.FB.ptr, N, B.polys(k, r), lb));
+// One product modulo the transform prime Q by cyclic transforms of length N:
+// coefficients [lo, lo + cnt) into dst.  FA: the transform of A, left in place
+// (computed here when `fresh`).
+int ntt_product(Pm& P, const NttPrime& Q, MatView A, int mA, int r, int64_t la, uint32_t* FA, bool fresh, MatView B,
+                int k, int64_t lb, uint32_t* FB, bool fresh_b, int64_t N, PolyView dst, int64_t lo, int64_t cnt) {
+  if (fresh) RR_TRY(ntt_forward(P, Q, FA, N, A.polys(r, mA), la));
+  if (fresh_b) RR_TRY(ntt_forward(P, Q, FB, N, B.polys(k, r), lb));
   if (mA % 4 == 0 && k % 4 == 0)
-    pointwise_kernel<<<grid_for((int64_t)P.nb * (mA / 4) * (k / 4) * N), 256, 0, P.s>>>(
-        P.FA.ptr, P.FB.ptr, P.FC.ptr, mA, r, k, N, P.nb, Q.fold4 ? 3 : 1, Q.M);
+    pointwise_kernel<<<grid_for((int64_t)P.nb * (mA / 4) * (k / 4) * N), 256, 0, P.s>>>(FA, FB, P.FC.ptr, mA, r, k, N,
+                                                                                        P.nb, Q.M);
   else
-    pointwise1_kernel<<<grid_for((int64_t)P.nb * mA * k * N), 256, 0, P.s>>>(P.FA.ptr, P.FB.ptr, P.FC.ptr, mA, r, k, N,
-                                                                              P.nb, Q.M);
+    pointwise1_kernel<<<grid_for((int64_t)P.nb * mA * k * N), 256, 0, P.s>>>(FA, FB, P.FC.ptr, mA, r, k, N, P.nb, Q.M);
   RR_CUDA(cudaGetLastError());
   return ntt_inverse(P, Q, P.FC.ptr, N, dst, lo, cnt);
 }
@@ -1229,32 +1240,61 @@ CrtParams crt_params(const Pm& P) {
   return C;
 }
 
-// dst[i][j][0..cnt) = coefficients [lo, lo+cnt) of A * B for every generator
-// of the batch, where A is mA x r with la coefficients and B is r x k with lb
-// coefficients.
-int poly_mat_mul(Pm& P, MatView A, int mA, int r, int64_t la, MatView B, int k, int64_t lb, MatView dst, int64_t lo,
-                 int64_t cnt) {
-  int64_t N = 1;
-  while (N < la + lb - 1) N <<= 1;
-  if (!P.use_ntt) {
-    schoolbook_kernel<<<grid_for((int64_t)P.nb * mA * k * cnt), 256, 0, P.s>>>(
-        A.p, mA, r, la, A.rs, A.cs, A.bs, B.p, k, lb, B.rs, B.cs, B.bs, dst.p, dst.rs, dst.cs, dst.bs, lo, cnt, P.nb,
-        P.M);
-    RR_CUDA(cudaGetLastError());
-    return RR_OK;
-  }
+// The two products of a level of the recursion, for every generator of the
+// batch.  MM (m x m, degree h) multiplies both times:
+//
+//   GG[t] = (MM G)[h + t], t < h, from the first 2h coefficients of G (n columns;
+//           deeper levels read no more of GG than its first h coefficients);
+//   M = MMM MM, degree 2h.
+//
+// Short ones are formed directly (pmproduct.cu).  The others go through cyclic
+// transforms of length N = 2h, half of what the full products would need: the
+// wrapped part of MM G (at most coefficient 3h - 1) falls below h, and M wraps
+// in one coefficient, which unwrap_kernel sets right.  The transform of MM is
+// kept between the two (`keep`, modulo p itself only; with CRT primes it is
+// computed again).
+int direct_or_fail(Pm& P, MatView A, int64_t la, MatView B, int k, int64_t lb, MatView dst, int64_t lo, int64_t cnt) {
+  DirectProduct D{};
+  D.A = A.p, D.a_rs = A.rs, D.a_cs = A.cs, D.a_bs = A.bs;
+  D.m = P.m, D.r = P.m, D.la = (int)la;
+  D.B = B.p, D.b_rs = B.rs, D.b_cs = B.cs, D.b_bs = B.bs;
+  D.k = k, D.lb = (int)lb;
+  D.C = dst.p, D.c_rs = dst.rs, D.c_cs = dst.cs, D.c_bs = dst.bs;
+  D.lo = (int)lo, D.cnt = (int)cnt;
+  D.M = P.M;
+  return direct_product(D, P.nb, P.s);
+}
+
+int level_product(Pm& P, MatView A, int64_t la, bool a_is_mm, MatView B, int k, int64_t lb, MatView dst, int64_t lo,
+                  int64_t cnt, int64_t h, uint32_t* keep) {
+  const int m = P.m;
+  if (P.mma && h <= direct_product_max(m)) return direct_or_fail(P, A, la, B, k, lb, dst, lo, cnt);
+  const int64_t N = 2 * h;
   if (N > P.nmax) return fail(RR_EINVAL, "internal: NTT length %lld exceeds table %lld", (long long)N, (long long)P.nmax);
-  if (!P.crt) return ntt_product(P, *P.nps[0], A, mA, r, la, B, k, lb, N, dst.polys(k, mA), lo, cnt);
-  // residues per transform prime, dense [nb][mA * k][cnt], then CRT into dst
-  const int64_t per = (int64_t)mA * k * cnt;
-  for (size_t i = 0; i < P.nps.size(); ++i) {
-    const PolyView Rv{P.R[i].ptr, k, mA * k, (int64_t)k * cnt, cnt, per};
-    RR_TRY(ntt_product(P, *P.nps[i], A, mA, r, la, B, k, lb, N, Rv, lo, cnt));
+  const int64_t ncoef = std::min<int64_t>(cnt, N - lo);  // M's last coefficient is not in the transform
+  if (!P.crt) {
+    uint32_t* FA = a_is_mm ? keep : P.FA.ptr;
+    uint32_t* FB = a_is_mm ? P.FB.ptr : keep;
+    RR_TRY(ntt_product(P, *P.nps[0], A, m, m, la, FA, true, B, k, lb, FB, a_is_mm, N, dst.polys(k, m), lo, ncoef));
+  } else {
+    // residues per transform prime, dense [nb][m * k][ncoef], then CRT into dst
+    const int64_t per = (int64_t)m * k * ncoef;
+    for (size_t i = 0; i < P.nps.size(); ++i) {
+      const PolyView Rv{P.R[i].ptr, k, m * k, (int64_t)k * ncoef, ncoef, per};
+      RR_TRY(ntt_product(P, *P.nps[i], A, m, m, la, P.FA.ptr, true, B, k, lb, P.FB.ptr, true, N, Rv, lo, ncoef));
+    }
+    const int64_t npoly = (int64_t)P.nb * m * k;
+    crt_kernel<<<grid_for(npoly * ncoef), 256, 0, P.s>>>(P.R[0].ptr, P.R[1].ptr,
+                                                         P.nps.size() > 2 ? P.R[2].ptr : nullptr, npoly, ncoef,
+                                                         dst.polys(k, m), crt_params(P));
+    RR_CUDA(cudaGetLastError());
   }
-  const int64_t npoly = (int64_t)P.nb * mA * k;
-  crt_kernel<<<grid_for(npoly * cnt), 256, 0, P.s>>>(P.R[0].ptr, P.R[1].ptr, P.nps.size() > 2 ? P.R[2].ptr : nullptr,
-                                                     npoly, cnt, dst.polys(k, mA), crt_params(P));
-  RR_CUDA(cudaGetLastError());
+  if (!a_is_mm) {
+    const int64_t npoly = (int64_t)P.nb * m * k;
+    unwrap_kernel<<<(unsigned)((npoly + 7) / 8), 256, 0, P.s>>>(A.polys(m, m), B.polys(k, m), dst.polys(k, m), m, m,
+                                                                    k, h, npoly, P.M);
+    RR_CUDA(cudaGetLastError());
+  }
   return RR_OK;
 }
 
@@ -1346,12 +1386,13 @@ int pm_rec(Pm& P, MatView G, int64_t d, int depth, MatView Mo) {
   const MatView MM{P.bufs[3 * depth + 0]->ptr, (int64_t)m * hl, hl, (int64_t)m * m * hl};   // m x m x (h+1)
   const MatView GG{P.bufs[3 * depth + 1]->ptr, (int64_t)n * hl, hl, (int64_t)m * n * hl};   // m x n x (h+1)
   const MatView MMM{P.bufs[3 * depth + 2]->ptr, (int64_t)m * hl, hl, (int64_t)m * m * hl};  // m x m x (h+1)
+  uint32_t* keep = P.FM.size() > (size_t)depth ? P.FM[depth]->ptr : nullptr;
   RR_TRY(pm_rec(P, G, h, depth + 1, MM));
-  // GG = (MM * G)[h .. d]   (poly_mat_mul_red_adaptive(MM, G, p, 0, d+1) + shift_trunc_in(h, h))
-  RR_TRY(poly_mat_mul(P, MM, m, m, hl, G, n, d + 1, GG, h, hl));
+  // GG = (MM * G)[h .. d - 1]   (poly_mat_mul_red_adaptive(MM, G, p, 0, d+1) + shift_trunc_in(h, h))
+  RR_TRY(level_product(P, MM, hl, true, G, n, d, GG, h, h, h, keep));
   RR_TRY(pm_rec(P, GG, h, depth + 1, MMM));
   // M = MMM * MM
-  return poly_mat_mul(P, MMM, m, m, hl, MM, m, hl, Mo, 0, d + 1);
+  return level_product(P, MMM, hl, false, MM, m, hl, Mo, 0, d + 1, h, keep);
 }
 
 }  // namespace
@@ -1388,60 +1429,49 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   P.cs = leaf_coeff_stride(P.m, P.n);
   P.fold4 = fold4_ok(p, P.M);
   const int m = P.m, n = P.n;
-  // NTT table for the largest product: length nextpow2(3d/2 + 1) = 2d (d >= 2)
-  int64_t nmax = 1;
-  while (nmax < d + d / 2 + 1) nmax <<= 1;
-  nmax = std::max<int64_t>(nmax, 2);
+  // the largest transform: length 2h = d
+  const int64_t nmax = std::max<int64_t>(d, 2);
   P.nmax = nmax;
   // NTT products: modulo p itself when p - 1 is divisible by the transform
   // length, else exact integer products by CRT over two or three NTT primes
   // (whose product must exceed inner dimension x length x (p-1)^2)
-  P.use_ntt = d > P.K;
+  const int64_t direct = P.mma ? direct_product_max(m) : 0;  // levels up to this half length take direct products
+  P.use_ntt = d > P.K && d / 2 > direct;
+  if (P.mma && d > P.K) RR_TRY(direct_product_prepare());
   if (P.use_ntt) {
     std::vector<uint32_t> qs;
-    if ((uint64_t)(p - 1) % (uint64_t)nmax == 0) {
-      qs.push_back(p);
-    } else {
-      P.crt = true;
+    if ((uint64_t)(p - 1) % (uint64_t)(2 * nmax) != 0) {
       const long double bound = (long double)m * (long double)(d + 1) * (long double)(p - 1) * (long double)(p - 1);
       long double prod = 1;
       for (int i = 0; i < 3 && prod <= bound; ++i) {
-        if ((uint64_t)(kCrtPrimes[i] - 1) % (uint64_t)nmax != 0)
-          return fail(RR_EUNSUPPORTED, "d = %lld: NTT length %lld beyond the CRT primes", (long long)d, (long long)nmax);
+        if ((uint64_t)(kCrtPrimes[i] - 1) % (uint64_t)(2 * nmax) != 0)
+          return fail(RR_EUNSUPPORTED, "d = %lld: NTT length %lld beyond the CRT primes", (long long)d,
+                      (long long)(2 * nmax));
         qs.push_back(kCrtPrimes[i]);
         prod *= kCrtPrimes[i];
       }
       if (prod <= bound) return fail(RR_EUNSUPPORTED, "d = %lld too large for a three-prime CRT at p = %u", (long long)d, p);
       if (qs.size() < 2) qs.push_back(kCrtPrimes[1]);  // Garner needs two residues
+      P.crt = true;
     }
-    std::vector<uint32_t> t(nmax / 2), ts(nmax / 2), ti(nmax / 2), tis(nmax / 2);
+    if ((uint64_t)(p - 1) % (uint64_t)nmax == 0) {
+      P.crt = false;
+      qs.assign(1, p);
+    }
     for (uint32_t q : qs) {
       std::unique_ptr<NttPrime> Q(new NttPrime());
       Q->q = q;
       Q->M = make_modp(q);
-      Q->fold4 = fold4_ok(q, Q->M);
       Q->nmax = nmax;
       const uint32_t g = find_generator(q);
       const uint32_t w = host_powmod(g, (q - 1) / (uint64_t)nmax, q);
-      const uint32_t wi = host_invmod(w, q);
-      uint64_t x = 1, y = 1;
-      for (int64_t j = 0; j < nmax / 2; ++j) {
-        t[j] = (uint32_t)x;
-        ti[j] = (uint32_t)y;
-        ts[j] = (uint32_t)((x << 32) / q);
-        tis[j] = (uint32_t)((y << 32) / q);
-        x = x * w % q;
-        y = y * wi % q;
-      }
       RR_TRY(Q->tw.alloc_async(nmax / 2, P.s));
       RR_TRY(Q->tws.alloc_async(nmax / 2, P.s));
       RR_TRY(Q->twi.alloc_async(nmax / 2, P.s));
       RR_TRY(Q->twis.alloc_async(nmax / 2, P.s));
-      RR_CUDA(cudaMemcpyAsync(Q->tw.ptr, t.data(), t.size() * 4, cudaMemcpyHostToDevice, P.s));
-      RR_CUDA(cudaMemcpyAsync(Q->tws.ptr, ts.data(), ts.size() * 4, cudaMemcpyHostToDevice, P.s));
-      RR_CUDA(cudaMemcpyAsync(Q->twi.ptr, ti.data(), ti.size() * 4, cudaMemcpyHostToDevice, P.s));
-      RR_CUDA(cudaMemcpyAsync(Q->twis.ptr, tis.data(), tis.size() * 4, cudaMemcpyHostToDevice, P.s));
-      RR_CUDA(cudaStreamSynchronize(P.s));  // the host tables are reused for the next prime
+      twiddle_kernel<<<(unsigned)((nmax / 2 + 255) / 256), 256, 0, P.s>>>(
+          Q->tw.ptr, Q->tws.ptr, Q->twi.ptr, Q->twis.ptr, nmax / 2, w, host_invmod(w, q), Q->M);
+      RR_CUDA(cudaGetLastError());
       P.nps.push_back(std::move(Q));
     }
     RR_TRY(P.FA.alloc_async((size_t)nb * m * m * nmax, P.s));
@@ -1449,6 +1479,11 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
     RR_TRY(P.FC.alloc_async((size_t)nb * m * m * nmax, P.s));
     if (P.crt)
       for (size_t i = 0; i < P.nps.size(); ++i) RR_TRY(P.R[i].alloc_async((size_t)nb * m * m * (d + 1), P.s));
+    else
+      for (int64_t dd = d; dd > P.K && dd / 2 > direct; dd /= 2) {
+        P.FM.emplace_back(new DevBuf<uint32_t>());
+        RR_TRY(P.FM.back()->alloc_async((size_t)nb * m * m * dd, P.s));
+      }
   }
   // per-depth buffers
   {

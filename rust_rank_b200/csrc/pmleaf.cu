@@ -63,6 +63,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "pm_mma.cuh"
 #include "pmleaf.h"
 
 namespace rr {
@@ -199,34 +200,6 @@ __device__ __forceinline__ void elim_bar() {
   asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
 }
 
-// D = A B (no accumulator to clear first)
-__device__ __forceinline__ void mma_u8_first(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
-}
-__device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// Montgomery products with the multiply-adds written in C: in this kernel the
-// compiler's wide multiply-adds issue at 3.6 cycles a warp and the whole
-// redc2 returns after 29 cycles, against 5.0 and 43 for the carry-chain forms
-// of rr_modp.cuh (one warp per SM sub-partition; latency is what counts here).
-__device__ __forceinline__ uint32_t redc64(uint64_t T, const ModP& M) {  // T < p 2^32
-  const uint32_t q = (uint32_t)T * M.pinv;
-  const uint32_t t = (uint32_t)(((uint64_t)q * M.p + T) >> 32);
-  return min(t, t - M.p);
-}
-__device__ __forceinline__ uint32_t redc_mul(uint32_t a, uint32_t b, const ModP& M) { return redc64((uint64_t)a * b, M); }
-__device__ __forceinline__ uint32_t redc2(uint32_t a, uint32_t b, uint32_t c, uint32_t d, const ModP& M) {
-  return redc64((uint64_t)c * d + (uint64_t)a * b, M);
-}
-
 // a^{-1} R mod p (p prime): a^(p-2) on Montgomery representatives; the square
 // and the product of a step are independent.
 __device__ uint32_t inverse_r(uint32_t a, const ModP& M) {
@@ -253,12 +226,6 @@ __device__ __forceinline__ void load_words(const uint32_t* p, uint32_t (&v)[CPW]
   }
 }
 
-// Word of (row, word) in a byte plane: the 8 rows x 4 words that a fragment
-// load reads fall in 32 different banks.
-template <int RL>
-__device__ __forceinline__ int plane_word(int r, int w) {
-  return RL == 1 ? r * 8 + (w ^ (((r >> 2) & 1) << 2)) : r * 16 + (w ^ (((r >> 1) & 3) << 2));
-}
 // Byte offset of (column, row) in a limb plane.
 template <int RL>
 __device__ __forceinline__ int plane_byte(int col, int row) {
@@ -279,15 +246,6 @@ __device__ __forceinline__ uint32_t plane_load(const uint32_t* coeff, int byte) 
   return v;
 }
 
-__device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t (&w)[4]) {
-  // w[l] = bytes l of v[0..3]
-  const uint32_t t0 = __byte_perm(v[0], v[1], 0x5140), t1 = __byte_perm(v[2], v[3], 0x5140);
-  const uint32_t t2 = __byte_perm(v[0], v[1], 0x7362), t3 = __byte_perm(v[2], v[3], 0x7362);
-  w[0] = __byte_perm(t0, t1, 0x5410);
-  w[1] = __byte_perm(t0, t1, 0x7632);
-  w[2] = __byte_perm(t2, t3, 0x5410);
-  w[3] = __byte_perm(t2, t3, 0x7632);
-}
 // Four 16 x 8 byte matrices in the accumulator layout (rows g and g + 8,
 // columns 2 t4 and 2 t4 + 1 of a thread), stored transposed: lane 8 l + c gives
 // the address of the 16 bytes of column c of matrix l.
