@@ -293,6 +293,15 @@ def report_progress(length: int, target: int, elapsed: float, rate: float, num_v
           f"(total {rate * num_v:.1f}/s) | Remaining: {remaining:.1f}s", end="", flush=True, file=out or sys.stdout)
 
 
+def _read_curv(stream: KrylovStream, curv) -> None:
+    """The stream's block into the caller's array, without a second copy where its layout allows."""
+    if (isinstance(curv, np.ndarray) and curv.dtype == np.uint32 and curv.shape == (stream.b, stream.n)
+            and curv.flags.c_contiguous and curv.flags.writeable):
+        stream.get_curv(curv)
+    else:
+        curv[:] = stream.get_curv()
+
+
 def main_loop_s_mt2(stream: KrylovStream, row_precond, col_precond, curv, v, seq: np.ndarray, seq_len: int,
                     max_nlen: int, wdm_filename: str | None = None, theprime: int = DEFAULT_PRIME,
                     save_after: float = 200.0, chunk_terms: int = 1 << 14, report_every: float | None = None) -> int:
@@ -317,7 +326,7 @@ def main_loop_s_mt2(stream: KrylovStream, row_precond, col_precond, curv, v, seq
         L = stream.advance(max_nlen, seq, report=report, chunk_terms=chunk_terms)
         done = max_nlen - L < 2
         if wdm_filename:
-            curv[:] = stream.get_curv()
+            _read_curv(stream, curv)
             save_wdm_file_sym(wdm_filename, stream.a.n_rows, stream.n, theprime, row_precond, col_precond, v, curv,
                               seq[:, :L])
             last_save = time.time()
@@ -325,7 +334,7 @@ def main_loop_s_mt2(stream: KrylovStream, row_precond, col_precond, curv, v, seq
             break
     if report_every is not None:
         print(file=sys.stdout)
-    curv[:] = stream.get_curv()
+    _read_curv(stream, curv)
     return L
 
 

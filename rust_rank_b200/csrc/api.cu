@@ -66,6 +66,9 @@ ModP make_modp(uint32_t p) {
 }
 
 int launch_scatter_block(rr_krylov* kr, const uint32_t* d_V, uint32_t* d_out);
+int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out);
+// Terms from which a fetch transposes on the device: below, the host loop is shorter than the launch and the strided copy.
+constexpr int64_t kTransposeTerms = 1024;
 int launch_precond(rr_krylov* kr, const uint32_t* d_rp, const uint32_t* d_cp, const int32_t* d_rowperm);
 
 }  // namespace rr
@@ -419,15 +422,27 @@ int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int6
   const int np = kr->b * (kr->b + 1) / 2;
   const int64_t cnt = to - from;
   if (cnt == 0) return RR_OK;
-  std::vector<uint32_t> tmp((size_t)cnt * np);
+  cudaStream_t st = kr->mat->ctx->stream;
+  const uint32_t* terms = kr->S.ptr + (size_t)(from - kr->base) * np;
   int dstat = 0;
-  RR_CUDA(cudaMemcpyAsync(tmp.data(), kr->S.ptr + (size_t)(from - kr->base) * np, tmp.size() * 4,
-                          cudaMemcpyDeviceToHost, kr->mat->ctx->stream));
-  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, kr->mat->ctx->stream));
-  RR_CUDA(cudaStreamSynchronize(kr->mat->ctx->stream));
-  if (dstat) return fail(RR_ETIMEOUT, "a device-side wait of the Gram pass gave up; the terms are not valid");
-  for (int64_t t = 0; t < cnt; ++t)
-    for (int q = 0; q < np; ++q) seq[(size_t)q * seq_stride + from + t] = tmp[(size_t)t * np + q];
+  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  std::vector<uint32_t> tmp;
+  if (cnt >= kTransposeTerms) {  // pair-major on the device, then one strided copy
+    DevBuf<uint32_t> pairs;
+    RR_TRY(pairs.alloc_async((size_t)cnt * np, st));
+    RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr));
+    RR_CUDA(cudaMemcpy2DAsync(seq + from, (size_t)seq_stride * 4, pairs.ptr, (size_t)cnt * 4, (size_t)cnt * 4, np,
+                              cudaMemcpyDeviceToHost, st));
+    RR_CUDA(cudaStreamSynchronize(st));
+  } else {
+    tmp.resize((size_t)cnt * np);
+    RR_CUDA(cudaMemcpyAsync(tmp.data(), terms, tmp.size() * 4, cudaMemcpyDeviceToHost, st));
+    RR_CUDA(cudaStreamSynchronize(st));
+  }
+  if (dstat) return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the terms are not valid");
+  if (!tmp.empty())
+    for (int64_t t = 0; t < cnt; ++t)
+      for (int q = 0; q < np; ++q) seq[(size_t)q * seq_stride + from + t] = tmp[(size_t)t * np + q];
   return RR_OK;
 }
 
@@ -519,7 +534,7 @@ int rr_krylov_get_curv(rr_krylov* kr, uint32_t* curv) {
   DevBuf<uint32_t> out;
   RR_TRY(out.alloc_async((size_t)kr->b * kr->mat->n, kr->mat->ctx->stream));
   RR_TRY(krylov_launch_get_curv(kr, out.ptr));
-  RR_CUDA(cudaMemcpyAsync(curv, out.ptr, out.bytes(), cudaMemcpyDeviceToHost, kr->mat->ctx->stream));
+  RR_TRY(rr::download_host(kr->mat->ctx, {{curv, out.ptr, out.bytes()}}, kr->mat->ctx->stream));
   RR_CUDA(cudaStreamSynchronize(kr->mat->ctx->stream));
   return RR_OK;
 }

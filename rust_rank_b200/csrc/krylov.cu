@@ -1604,6 +1604,25 @@ int launch_precond(rr_krylov* kr, const uint32_t* d_rp, const uint32_t* d_cp, co
   return RR_OK;
 }
 
+// out[q][t] = terms[t][q] (32 x 32 tiles through shared memory)
+__global__ void pair_major_kernel(const uint32_t* __restrict__ terms, int64_t count, int np, uint32_t* __restrict__ out) {
+  __shared__ uint32_t tile[32][33];
+  const int64_t t0 = (int64_t)blockIdx.x * 32;
+  const int q0 = blockIdx.y * 32;
+  for (int y = threadIdx.y; y < 32; y += 8)
+    if (t0 + y < count && q0 + (int)threadIdx.x < np) tile[y][threadIdx.x] = terms[(t0 + y) * np + q0 + threadIdx.x];
+  __syncthreads();
+  for (int y = threadIdx.y; y < 32; y += 8)
+    if (q0 + y < np && t0 + threadIdx.x < count) out[(int64_t)(q0 + y) * count + t0 + threadIdx.x] = tile[threadIdx.x][y];
+}
+
+int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out) {
+  const dim3 grid((unsigned)((count + 31) / 32), (unsigned)((np + 31) / 32));
+  pair_major_kernel<<<grid, dim3(32, 8), 0, s>>>(terms, count, np, out);
+  RR_CUDA(cudaGetLastError());
+  return RR_OK;
+}
+
 int launch_scatter_block(rr_krylov* kr, const uint32_t* d_V, uint32_t* d_out) {
   const int64_t n = kr->mat->n;
   const int threads = 256;

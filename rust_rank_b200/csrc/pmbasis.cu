@@ -1530,12 +1530,13 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   const MatView Mv{Mo.ptr, (int64_t)m * (d + 1), d + 1, (int64_t)m * m * (d + 1)};
   RR_TRY(pm_rec(P, Gv, d, 0, Mv));
   int status = 0;
+  std::vector<HostSegment> outs;
   for (int z = 0; z < nb; ++z) {
-    RR_CUDA(cudaMemcpyAsync(Mh[z], Mo.ptr + (size_t)z * m * m * (d + 1), (size_t)m * m * (d + 1) * 4,
-                            cudaMemcpyDeviceToHost, P.s));
-    RR_CUDA(cudaMemcpyAsync(deltah[z], P.delta.ptr + (size_t)z * m, m * sizeof(int64_t), cudaMemcpyDeviceToHost, P.s));
+    outs.push_back({Mh[z], Mo.ptr + (size_t)z * m * m * (d + 1), (size_t)m * m * (d + 1) * 4});
+    outs.push_back({deltah[z], P.delta.ptr + (size_t)z * m, m * sizeof(int64_t)});
   }
-  RR_CUDA(cudaMemcpyAsync(&status, P.status.ptr, sizeof(int), cudaMemcpyDeviceToHost, P.s));
+  outs.push_back({&status, P.status.ptr, sizeof(int)});
+  RR_TRY(download_host(ctx, outs, P.s));
   RR_CUDA(cudaStreamSynchronize(P.s));
   if (status == 3) return fail(RR_ETIMEOUT, "PM-basis leaf kernel: a hand-off between its warp groups gave up");
   if (status) return fail(RR_ECUDA, "PM-basis device status %d (zero row scale)", status);

@@ -160,6 +160,10 @@ struct HostSegment {
   size_t bytes;
 };
 int upload_host(rr_ctx* ctx, const std::vector<HostSegment>& segs, cudaStream_t s);
+// Device results to host arrays, after the work queued on s: the same staging
+// the other way round.  Small and pinned ones are only queued: the caller
+// synchronises s before it uses them.
+int download_host(rr_ctx* ctx, const std::vector<HostSegment>& segs, cudaStream_t s);
 void staging_destroy(Staging* st);
 
 constexpr int64_t kHeavyDegree = 32;   // rows longer than this are split
