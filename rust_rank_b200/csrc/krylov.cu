@@ -223,6 +223,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   constexpr int LPT = S::LPT, NV = S::NV, TPR = S::TPR, RPW = S::RPW;
   constexpr int NP = B * (B + 1) / 2;  // pairs in padded space
   constexpr bool kMma = B >= 8;
+  constexpr bool kSym = MODE != kModeOdd;  // both Gram factors are the same rows: one set of byte planes
   using Gram = typename std::conditional<kMma, GramMma<B, FE, L>, GramCore<B, FE, L>>::type;
 
   const int lane = threadIdx.x & 31;
@@ -235,7 +236,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   for (int q = threadIdx.x; q < NP; q += kThreads) red[q] = 0;
   Gram gram;
   const bool emit = GRAM && (P.S_out != nullptr || P.term_ctr != nullptr);
-  if (emit) gram.init(gram_smem + (size_t)warp * Gram::kWords, lane);
+  if (emit) gram.init(gram_smem + (size_t)warp * (kSym ? Gram::kWordsSym : Gram::kWords), lane, kSym);
   __syncthreads();  // red[] zeroed before a warp may emit into it
 
   const int64_t nbatch = (P.rows + RPW - 1) / RPW;
@@ -274,7 +275,8 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
       const int sg = P.batch_seg[batch];
       if (sg != cur_seg) {
         if (cur_seg >= 0) {
-          gram.finish(slot, sub, lane, M, W);
+          if (kSym) gram.finish_sym(slot, sub, lane, M, W);
+          else gram.finish(slot, sub, lane, M, W);
           gram.emit(cur_seg == seg0 ? red : seg_target(P, acc, cur_seg, NP), lane, M);
           gram.reset();
         }
@@ -351,12 +353,16 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
 #pragma unroll
       for (int l = 0; l < LPT; ++l) { gz[l] = 0; gu[l] = 0; }
     }
-    if (emit) gram.add(gz, gu, slot, sub, lane, M, W);
+    if (emit) {
+      if (kSym) gram.add_sym(gz, slot, sub, lane, M, W);
+      else gram.add(gz, gu, slot, sub, lane, M, W);
+    }
   }
   if (!segmented) griddep_launch();
 
   if (!emit) return;
-  gram.finish(slot, sub, lane, M, W);
+  if (kSym) gram.finish_sym(slot, sub, lane, M, W);
+  else gram.finish(slot, sub, lane, M, W);
   __syncthreads();  // red[] is zeroed before any warp emits into it
   if (segmented) {
     if (cur_seg >= 0) gram.emit(cur_seg == seg0 ? red : seg_target(P, acc, cur_seg, NP), lane, M);
@@ -598,10 +604,8 @@ __device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t
 // mod p (its limb products are exact for any 32-bit operand and its sums are
 // reduced mod p), so the comparison and subtraction are left out.
 __device__ __forceinline__ uint32_t redc_lazy(uint32_t y, uint32_t s, const ModP& M) {
-  uint32_t lo = 0, hi = 0;
-  mac_cc(y, s, lo, hi);
-  mac_cc(lo * M.pinv, M.p, lo, hi);  // lo becomes 0; y s + q p < 2 p 2^32
-  return hi;
+  const uint64_t T = (uint64_t)y * s;
+  return (uint32_t)(((uint64_t)((uint32_t)T * M.pinv) * M.p + T) >> 32);  // y s + q p < 2 p 2^32
 }
 
 // A bounded wait that also ends when another role of the CTA gave up.
@@ -1125,10 +1129,13 @@ int launch_batch_finalize(cudaStream_t s, const unsigned long long* gram_all, co
 }
 
 // ---------------------------------------------------------------- launchers
-// dynamic shared memory of the pass kernel: the per-warp Gram staging area
-template <int B>
+// dynamic shared memory of the pass kernel: the per-warp Gram staging area.
+// The even and initial passes stage one factor only: what they leave of the SM's
+// memory is L1 for their gathers.
+template <int B, bool SYM = false>
 constexpr size_t pass_smem_bytes() {
-  return (size_t)kWarps * 4 * (B >= 8 ? GramMma<B, 4>::kWords : GramCore<B, 4>::kWords);
+  if (B >= 8) return (size_t)kWarps * 4 * (SYM ? GramMma<B, 4>::kWordsSym : GramMma<B, 4>::kWords);
+  return (size_t)kWarps * 4 * GramCore<B, 4>::kWords;
 }
 
 // CTAs for a pass over `rows` rows: the resident maximum, but no more CTAs
@@ -1189,14 +1196,14 @@ static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 b
 template <int B, int FE>
 static int launch_pass_BF(rr_krylov* kr, const PassParams& P, int mode, dim3 grid, cudaStream_t s) {
   const dim3 block(kThreads);
-  const size_t sm = pass_smem_bytes<B>();
+  const size_t sm = pass_smem_bytes<B>(), sm1 = pass_smem_bytes<B, true>();
   switch (mode) {
-    case kModeInit: return launch_ex(kr, pass_kernel<B, kModeInit, FE, true>, grid, block, sm, s, P);
+    case kModeInit: return launch_ex(kr, pass_kernel<B, kModeInit, FE, true>, grid, block, sm1, s, P);
     case kModeOdd:
       if constexpr (kFusedOdd<B>) return launch_ex(kr, pass_kernel<B, kModeOdd, FE, true>, grid, block, sm, s, P);
       else return launch_ex(kr, pass_kernel<B, kModeOdd, FE, false, kLeanLpt<B>>, grid, block, 0, s, P);
     case kModeEven:
-      if constexpr (kFusedEven<B>) return launch_ex(kr, pass_kernel<B, kModeEven, FE, true>, grid, block, sm, s, P);
+      if constexpr (kFusedEven<B>) return launch_ex(kr, pass_kernel<B, kModeEven, FE, true>, grid, block, sm1, s, P);
       else return launch_ex(kr, pass_kernel<B, kModeEven, FE, false, kLeanLpt<B>>, grid, block, 0, s, P);
   }
   return fail(RR_EINVAL, "pass mode %d has no pass kernel at width %d", mode, B);

@@ -49,13 +49,13 @@ template <int B, int FE, int L = kDefaultLpt<B>>
 struct GramCore {
   static constexpr int LPT = Shape<B, L>::LPT, RPW = Shape<B, L>::RPW;
   static constexpr int NP = B * (B + 1) / 2, PPL = (NP + 31) / 32;
-  static constexpr int kWords = 2 * RPW * B;  // shared words per warp
+  static constexpr int kWords = 2 * RPW * B, kWordsSym = kWords;  // shared words per warp
   uint32_t* zs;  // [RPW][B]
   uint32_t* us;
   uint32_t pij[PPL];
   unsigned long long acc[PPL];
 
-  __device__ __forceinline__ void init(uint32_t* w, int lane) {
+  __device__ __forceinline__ void init(uint32_t* w, int lane, bool = false) {
     zs = w;
     us = w + RPW * B;
 #pragma unroll
@@ -144,15 +144,16 @@ struct GramMma {
   static constexpr int RS = 9;                  // words per (limb, lane) plane row: 32 bytes + 4 pad
   static constexpr int kPlane = 4 * BM * RS;    // words per plane set
   static constexpr int kWords = 2 * kPlane;     // shared words per warp
+  static constexpr int kWordsSym = kPlane;      // with add_sym only
   uint32_t* pz;
   uint32_t* pu;
   unsigned long long acc[MT][NT][4];
   int bt;
 
-  __device__ __forceinline__ void init(uint32_t* w, int lane) {
+  __device__ __forceinline__ void init(uint32_t* w, int lane, bool sym = false) {
     pz = w;
     pu = w + kPlane;
-    for (int q = lane; q < kWords; q += 32) w[q] = 0;  // zero padding rows stay zero
+    for (int q = lane; q < (sym ? kWordsSym : kWords); q += 32) w[q] = 0;  // zero padding rows stay zero
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll

@@ -22,8 +22,8 @@ __device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint
 
 // Montgomery products with the multiply-adds written in C: in the
 // PM-basis kernels the compiler's wide multiply-adds issue at 3.6 cycles a warp and the whole
-// redc2 returns after 29 cycles, against 5.0 and 43 for the carry-chain forms
-// of rr_modp.cuh (one warp per SM sub-partition; latency is what counts here).
+// redc2 returns after 29 cycles, against 5.0 and 43 with mad.lo.cc / madc.hi
+// chains (one warp per SM sub-partition; latency is what counts here).
 __device__ __forceinline__ uint32_t redc64(uint64_t T, const ModP& M) {  // T < p 2^32
   const uint32_t q = (uint32_t)T * M.pinv;
   const uint32_t t = (uint32_t)(((uint64_t)q * M.p + T) >> 32);

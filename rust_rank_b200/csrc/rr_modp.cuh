@@ -19,18 +19,21 @@ struct ModP {
 };
 
 #ifdef __CUDACC__
-// a * b + c exactly (mod 2^64), as a carry chain of 32-bit multiply-adds
-// (mad.lo.cc / madc.hi): on sm_100 this issues at about 1.6x the rate of the
-// 64-bit wide multiply-add the compiler emits for (uint64_t)a * b + c.
-__device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) {
-  uint32_t lo = (uint32_t)c, hi = (uint32_t)(c >> 32);
-  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
-  return ((uint64_t)hi << 32) | lo;
-}
+// a * b + c exactly (mod 2^64).  Written in C: ptxas makes one wide multiply-add
+// of it, which issues every 3.6 cycles per warp and SM sub-partition; the
+// mad.lo.cc / madc.hi pair takes 5.0 (CUDA 12.9, B200).
+__device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)a * b + c; }
 
 // Fold a 64-bit accumulator: result == x (mod p) and result < 2^32 * c32 + 2^32.
+// Here the carry chain wins (mad_wide and fold of one accumulator 10.2 cycles
+// against 11.8): the addend is half an accumulator, which the wide form has to
+// be copied into a register pair for.
 __device__ __forceinline__ uint64_t fold(uint64_t x, const ModP& M) {
-  return mad_wide((uint32_t)(x >> 32), M.c32, (uint32_t)x);
+  uint32_t lo = (uint32_t)x, hi = 0;
+  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
+      : "+r"(lo), "+r"(hi)
+      : "r"((uint32_t)(x >> 32)), "r"(M.c32));
+  return ((uint64_t)hi << 32) | lo;
 }
 
 // Exact x mod p for any 64-bit x.  q = floor(x*mu / 2^64) is at most 2 below
@@ -51,7 +54,7 @@ __device__ __forceinline__ uint32_t redc(uint64_t T, const ModP& M) {
   const uint32_t m = (uint32_t)T * M.pinv;
   const uint64_t s = (uint64_t)m * M.p + T;
   const uint32_t t = (uint32_t)(s >> 32);
-  return t >= M.p ? t - M.p : t;
+  return min(t, t - M.p);  // t < 2p
 }
 
 __device__ __forceinline__ uint32_t mulmod(uint32_t a, uint32_t b, const ModP& M) {
@@ -65,27 +68,6 @@ __device__ __forceinline__ uint32_t addmod(uint32_t a, uint32_t b, uint32_t p) {
 
 __device__ __forceinline__ uint32_t submod(uint32_t a, uint32_t b, uint32_t p) {
   return a >= b ? a - b : a + p - b;
-}
-
-// (hi:lo) += a * b with a carry chain of 32-bit multiply-adds; on sm_100 this
-// runs at about 1.6x the rate of the 64-bit wide multiply-add above.
-__device__ __forceinline__ void mac_cc(uint32_t a, uint32_t b, uint32_t& lo, uint32_t& hi) {
-  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
-}
-
-// Montgomery reduction of T = (hi:lo) < p * 2^32: T * 2^-32 mod p, in [0, p).
-__device__ __forceinline__ uint32_t redc_cc(uint32_t lo, uint32_t hi, const ModP& M) {
-  const uint32_t q = lo * M.pinv;
-  mac_cc(q, M.p, lo, hi);  // lo becomes 0; T + q p < 2 p 2^32 <= 2^64
-  return hi >= M.p ? hi - M.p : hi;
-}
-
-// (a b + c d) * 2^-32 mod p for residues a, b, c, d < p < 2^31.
-__device__ __forceinline__ uint32_t redc_2mac(uint32_t a, uint32_t b, uint32_t c, uint32_t d, const ModP& M) {
-  uint32_t lo = 0, hi = 0;
-  mac_cc(a, b, lo, hi);
-  mac_cc(c, d, lo, hi);
-  return redc_cc(lo, hi, M);
 }
 #endif  // __CUDACC__
 
