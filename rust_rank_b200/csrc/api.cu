@@ -338,8 +338,11 @@ int rr_krylov_destroy(rr_krylov* kr) {
 // started and the graph can be replayed), and the run length that uses it.
 constexpr int64_t kGraphApps = 16;
 constexpr int64_t kGraphMinRun = 2 * kGraphApps;
-// Shortest run worth a resident launch (it reads the CSR into shared memory first).
-constexpr int64_t kResidentMinRun = 4;
+// Shortest run worth a resident launch, which reads the CSR into shared memory
+// first.  One application at width 16 is three other launches (2000 x 1500: 42 us
+// against 26 resident); narrower ones are two, which overlap (5003 x 4001, b = 3:
+// 25 us against 30).
+static int64_t resident_min_run(const rr_krylov* kr) { return kr->B >= 16 ? 1 : 4; }
 
 // Captures kGraphApps applications (they are recorded, not run: the host
 // state the launches advance is restored afterwards).  The capture runs on a
@@ -382,7 +385,7 @@ static int queue_apps(rr_krylov* kr, int64_t n_apps) {
   if (kr->len == 0) kr->len = 1;  // publish S_0
   RR_TRY(ensure_capacity(kr, kr->len - kr->base + 2 * n_apps + 1));
   int64_t i = 0;
-  if (kr->res_grid > 0 && n_apps >= kResidentMinRun) {
+  if (kr->res_grid > 0 && n_apps >= resident_min_run(kr)) {
     for (bool taken = true; taken && i < n_apps;) {
       const int k = (int)std::min<int64_t>(kResMaxApps, n_apps - i);
       RR_TRY(resident_run(kr, k, &taken));
