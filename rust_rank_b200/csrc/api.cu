@@ -291,7 +291,7 @@ int rr_krylov_create(rr_matrix* mat, int32_t b, const uint32_t* row_precond, con
   const int64_t heavy = std::max<int64_t>(std::max(mat->A.heavy_rows, mat->At.heavy_rows), 1);
   RR_TRY(kr->heavy_acc.alloc_async((size_t)heavy * B, s));
   RR_CUDA(cudaMemsetAsync(kr->heavy_acc.ptr, 0, kr->heavy_acc.bytes(), s));
-  RR_TRY(kr->gram_acc.alloc_async((size_t)kGramReplicas * (B * (B + 1) / 2), s));
+  RR_TRY(kr->gram_acc.alloc_async((size_t)kGramReplicas * (B * (B + 1)), s));
   RR_CUDA(cudaMemsetAsync(kr->gram_acc.ptr, 0, kr->gram_acc.bytes(), s));
   RR_TRY(kr->d_status.alloc_async(1, s));
   RR_CUDA(cudaMemsetAsync(kr->d_status.ptr, 0, sizeof(int), s));

@@ -225,18 +225,32 @@ __device__ __forceinline__ unsigned long long* seg_target(const PassParams& P, u
   return acc + (size_t)sg * NP;
 }
 
+// Gram terms a pass forms itself: none; that of its mode; or (even pass) both
+// terms of the application.
+enum GramForm { kGramNone = 0, kGramOwn = 1, kGramBoth = 2 };
+
+template <int B, int FE, int L, int GRAM>
+struct GramOf {
+  using type = typename std::conditional<(B >= 8), GramMma<B, FE, L>, GramCore<B, FE, L>>::type;
+};
+template <int B, int FE, int L>
+struct GramOf<B, FE, L, kGramBoth> {
+  using type = GramDual<B, FE, L>;
+};
+
 // One pass over the rows of A (MODE odd), of A^T (even) or the initial
 // scaling (init), by the whole CTA: gram_smem is the per-warp Gram staging,
-// red[NP] the CTA's Gram reduction, is_last a shared flag.
-template <int B, int MODE, int FE, bool COH, bool GRAM = true, int L = kDefaultLpt<B>>
+// red[NP] (2 NP with kGramBoth) the CTA's Gram reduction, is_last a shared flag.
+template <int B, int MODE, int FE, bool COH, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
 __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_smem, unsigned long long* red,
                                           bool& is_last) {
   using S = Shape<B, L>;
   constexpr int LPT = S::LPT, NV = S::NV, TPR = S::TPR, RPW = S::RPW;
   constexpr int NP = B * (B + 1) / 2;  // pairs in padded space
-  constexpr bool kMma = B >= 8;
-  constexpr bool kSym = MODE != kModeOdd;  // both Gram factors are the same rows: one set of byte planes
-  using Gram = typename std::conditional<kMma, GramMma<B, FE, L>, GramCore<B, FE, L>>::type;
+  constexpr bool kBoth = GRAM == kGramBoth;
+  constexpr bool kSym = MODE != kModeOdd && !kBoth;  // both Gram factors are the same rows: one set of byte planes
+  constexpr int kSums = kBoth ? 2 * NP : NP;
+  using Gram = typename GramOf<B, FE, L, GRAM>::type;
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -245,10 +259,13 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   const ModP M = P.M;
   const uint32_t W[3] = {P.w4, P.w5, P.w6};
 
-  for (int q = threadIdx.x; q < NP; q += kThreads) red[q] = 0;
+  for (int q = threadIdx.x; q < kSums; q += kThreads) red[q] = 0;
   Gram gram;
-  const bool emit = GRAM && (P.S_out != nullptr || P.term_ctr != nullptr);
-  if (emit) gram.init(gram_smem + (size_t)warp * (kSym ? Gram::kWordsSym : Gram::kWords), lane, kSym);
+  const bool emit = GRAM != kGramNone && (P.S_out != nullptr || P.term_ctr != nullptr);
+  if (emit) {
+    if constexpr (kBoth) gram.init(gram_smem + (size_t)warp * Gram::kWords, lane);
+    else gram.init(gram_smem + (size_t)warp * (kSym ? Gram::kWordsSym : Gram::kWords), lane, kSym);
+  }
   __syncthreads();  // red[] zeroed before a warp may emit into it
 
   const int64_t nbatch = (P.rows + RPW - 1) / RPW;
@@ -287,7 +304,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
       const int sg = P.batch_seg[batch];
       if (sg != cur_seg) {
         if (cur_seg >= 0) {
-          if (kSym) gram.finish_sym(slot, sub, lane, M, W);
+          if constexpr (kSym) gram.finish_sym(slot, sub, lane, M, W);
           else gram.finish(slot, sub, lane, M, W);
           gram.emit(cur_seg == seg0 ? red : seg_target(P, acc, cur_seg, NP), lane, M);
           gram.reset();
@@ -341,12 +358,24 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
           o[l] = gu[l];
         }
       } else if (MODE == kModeEven) {
-        // w' = d_c t_true = redc(t * d_c R^2); x' = d_c w' = redc(w' * d_c R)
+        // w' = d_c t_true = redc(t * d_c R^2); x' = d_c w' = redc(w' * d_c R);
+        // for the odd term the row's old w = redc(x * d_c^{-1} R)
         const uint32_t s2 = P.scale2[r];
+        if constexpr (kBoth) {
+          const uint32_t s3 = P.scale3[r];
+#pragma unroll
+          for (int v = 0; v < NV; ++v) {
+            const uint4 x = __ldg(P.X_old + r * (B / 4) + S::word_of(sub, v));
+            gu[4 * v + 0] = redc((uint64_t)x.x * s3, M);
+            gu[4 * v + 1] = redc((uint64_t)x.y * s3, M);
+            gu[4 * v + 2] = redc((uint64_t)x.z * s3, M);
+            gu[4 * v + 3] = redc((uint64_t)x.w * s3, M);
+          }
+        }
 #pragma unroll
         for (int l = 0; l < LPT; ++l) {
           gz[l] = redc((uint64_t)t[l] * s1, M);
-          gu[l] = gz[l];
+          if (!kBoth) gu[l] = gz[l];
           o[l] = redc((uint64_t)gz[l] * s2, M);
         }
       } else {
@@ -366,14 +395,14 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
       for (int l = 0; l < LPT; ++l) { gz[l] = 0; gu[l] = 0; }
     }
     if (emit) {
-      if (kSym) gram.add_sym(gz, slot, sub, lane, M, W);
+      if constexpr (kSym) gram.add_sym(gz, slot, sub, lane, M, W);
       else gram.add(gz, gu, slot, sub, lane, M, W);
     }
   }
   if (!segmented) griddep_launch();
 
   if (!emit) return;
-  if (kSym) gram.finish_sym(slot, sub, lane, M, W);
+  if constexpr (kSym) gram.finish_sym(slot, sub, lane, M, W);
   else gram.finish(slot, sub, lane, M, W);
   __syncthreads();  // red[] is zeroed before any warp emits into it
   if (segmented) {
@@ -387,7 +416,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   } else {
     gram.emit(red, lane, M);
     __syncthreads();
-    for (int q = threadIdx.x; q < NP; q += kThreads) atomicAdd(&acc[q], red[q]);
+    for (int q = threadIdx.x; q < kSums; q += kThreads) atomicAdd(&acc[q], red[q]);
   }
   __threadfence();
   __syncthreads();
@@ -432,16 +461,16 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   } else {
     uint32_t* S_out = P.S_out;
     if (P.term_ctr != nullptr) S_out = *P.S_ptr + (size_t)__ldcg(P.term_ctr) * npr;
-    for (int q = threadIdx.x; q < npr; q += kThreads) {
+    for (int q = threadIdx.x; q < kSums / NP * npr; q += kThreads) {  // kGramBoth: the odd term, then the even one
       int i, j;
-      pair_of(q, b, i, j);
-      const int qb = pair_index(i, j, B);
+      pair_of(q % npr, b, i, j);
+      const int qb = q / npr * NP + pair_index(i, j, B);
       S_out[q] = mulmod(reduce(sum_replicas(P, qb), M), P.gram_mul, M);
     }
     __syncthreads();
-    for (int q = threadIdx.x; q < NP * P.replicas; q += kThreads)
-      __stcg(P.gram_acc + (size_t)(q / NP) * P.gram_stride + q % NP, 0ull);
-    if (P.term_ctr != nullptr && threadIdx.x == 0) *P.term_ctr += 1u;  // read above by thread 0 only after the barrier
+    for (int q = threadIdx.x; q < kSums * P.replicas; q += kThreads)
+      __stcg(P.gram_acc + (size_t)(q / kSums) * P.gram_stride + q % kSums, 0ull);
+    if (P.term_ctr != nullptr && threadIdx.x == 0) *P.term_ctr += kSums / NP;  // read above by thread 0 only after the barrier
   }
   if (threadIdx.x == 0) atomicExch(P.counter, 0u);
 }
@@ -454,13 +483,13 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
 // Resident CTAs per SM the register budget is set for: 5 for the lean pass at
 // width 16 (48 registers; one more CTA of latency hiding measured 1.3 % faster
 // than 4 with 62 registers), 2 for fused passes at width 32, else 4.
-template <int B, bool GRAM>
+template <int B, int GRAM>
 constexpr int kPassMinBlocks = (B >= 32 && GRAM) ? 2 : ((!GRAM && B == 16) ? 5 : 4);
 
-template <int B, int MODE, int FE, bool GRAM = true, int L = kDefaultLpt<B>>
+template <int B, int MODE, int FE, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
 __global__ void __launch_bounds__(kThreads, kPassMinBlocks<B, GRAM>) pass_kernel(PassParams P) {
   extern __shared__ __align__(16) uint32_t gram_smem[];
-  __shared__ unsigned long long red[B * (B + 1) / 2];
+  __shared__ unsigned long long red[(GRAM == kGramBoth ? 2 : 1) * (B * (B + 1) / 2)];
   __shared__ bool is_last;
   griddep_wait();
   pass_body<B, MODE, FE, false, GRAM, L>(P, gram_smem, red, is_last);
@@ -472,28 +501,32 @@ __global__ void __launch_bounds__(kThreads, kPassMinBlocks<B, GRAM>) pass_kernel
 template <int B>
 constexpr int kLeanLpt = (B == 16) ? 4 : kDefaultLpt<B>;
 
-// Which single-matrix passes compute their Gram terms themselves (u8-limb
-// mma.sync on the block rows still in registers) and which run without them,
-// followed by a tcgen05 Gram pass (gram_tc_kernel) that reads the written
-// block once more.  Measured per pass on the 2M x 1.5M Zipf matrix: at width
-// 16 the odd pass is faster split (0.251 ms against 0.269 fused), the even
-// pass fused (0.146 against 0.173); at width 32 both are faster split (0.93
-// ms per application against 1.29 fused).
+// Both Gram terms of an application come from the rows of its even pass: the
+// odd one as S_{2k+1} = w_k^T w_{k+1} = sum over the columns of A of w (x) w'
+// (the form of src/main.rs:138-146; the sum over the rows of A, z (x) U, is equal
+// but needs a second pass over U).  Widths up to 8 form them in the even pass
+// (GramDual), wider ones in a tcgen05 pass over the old and the new block
+// (gram_tc_kernel).  Measured (us per application, odd term from the rows of A /
+// both from the columns): 2M x 1.5M Zipf, b = 16: 533 / 516, b = 5: 362 / 326;
+// 1M x 750k Zipf, b = 32: 460 / 451; 600k x 500k incidence, b = 16: 148 / 129;
+// 190k x 150k incidence, b = 32: 104 / 99; 60k x 50k Zipf, b = 4: 28.9 / 23.6.
 template <int B>
-constexpr bool kFusedOdd = (B <= 8);
-template <int B>
-constexpr bool kFusedEven = (B <= 16);
+constexpr bool kGramInPass = B <= 8;
 
 // ---------------------------------------------------------------- Gram pass on tcgen05
-// The Gram term of a block (kModeGram: gz = x * scale, gu = gram_sym ? gz : x
-// per row) on the 5th-generation tensor cores, for padded widths 16 and 32.
+// Both Gram terms of an application (kModeGram: X the block after it, X_old
+// the one before, scale = d_c^{-1}, so that w' = X scale and w = X_old scale) on
+// the 5th-generation tensor cores, for padded widths 16 and 32.
 //
-// Exact integers by byte limbs: with gz = sum_a 256^a Z_a and gu = sum_c 256^c
-// U_c (bytes), G[i][j] = sum_{a,c} 256^{a+c} (Z_a^T U_c)[i][j].  One UMMA
+// Exact integers by byte limbs: with w' = sum_a 256^a W'_a and w = sum_c 256^c
+// W_c (bytes), (w' (x) w)[i][j] = sum_{a,c} 256^{a+c} (W'_a^T W_c)[i][j].  One UMMA
 // D[M x N] += A[M x K] B[N x K]^T (kind::i8, unsigned bytes, s32 accumulators
-// in TMEM) computes all 16 limb pairs at once: A row (a, i) holds limb a of
-// lane i of the tile's rows (K = rows), B row (c, j) limb c of gu; M = 128
-// (4 B rows, zero-padded to 128 for B = 16), N = 4 B.  A CTA stages 128-row
+// in TMEM) computes all 16 limb pairs of both terms at once: row (c, j) of the
+// B operand holds limb c of lane j of w over the tile's rows (K = rows), rows
+// 4B + (c, j) the same of w', N = 8 B; the A operand is the rows of w' in the
+// same memory (M = 128 = 4 B at B = 32; at B = 16 all N rows, of whose results
+// the upper half is read), so a value is stored once however often it is
+// multiplied.  A CTA stages 128-row
 // tiles into shared memory in the canonical K-major layout without swizzle
 // (8-row x 16-byte core matrices; K-adjacent cores 128 bytes apart, 8-row
 // groups 256 bytes apart); one thread issues the four K = 32 MMAs of a tile.
@@ -569,15 +602,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
 template <int B>
 struct TcShape {
   static constexpr int TILE = 128;                           // rows (K bytes) per tile
-  static constexpr int MR = 4 * B;                           // real A rows (limb, lane)
-  static constexpr int M = 128;                              // UMMA M (zero rows above MR)
-  static constexpr int N = 4 * B;                            // UMMA N
-  static constexpr int A_BYTES = M * TILE;
-  static constexpr int B_BYTES = N * TILE;
-  static constexpr int STAGE = A_BYTES + B_BYTES;            // one operand stage
-  static constexpr int OPS = 4;                              // operand stages
-  static constexpr int RAW_Y = TILE * B * 4;                 // a tile's block rows
-  static constexpr int RAW_BYTES = RAW_Y + TILE * 4;         // plus its row scales
+  static constexpr int H = 4 * B;                            // operand rows (limb, lane) of one block
+  static constexpr int M = 128;                              // UMMA M
+  static constexpr int N = 2 * H;                            // UMMA N: w, then w'
+  static constexpr int A_ROW = N - M;                        // first operand row of A
+  static constexpr int STAGE = N * TILE;                     // one operand stage
+  static constexpr int OPS = B >= 32 ? 2 : 4;                // operand stages
+  static constexpr int RAW_Y = TILE * B * 4;                 // a tile's rows of one block
+  static constexpr int RAW_BYTES = 2 * RAW_Y + TILE * 4;     // of both, and the row scales
   static constexpr int RING = 4;                             // raw tiles in flight
   static constexpr int GROUPS = B / 4;                       // 128-bit words per row
   static constexpr int TASKS = (TILE / 4) * GROUPS;          // 4 rows x 4 lanes each
@@ -586,7 +618,7 @@ struct TcShape {
   static constexpr int XW0 = 6;                              // first transposer warp
   static constexpr int WARPS = XW0 + NG * TW;
   static constexpr int THREADS = 32 * WARPS;
-  static constexpr int COLS = 2 * N <= 128 ? 128 : 256;      // two accumulators
+  static constexpr int COLS = 2 * N;                         // two accumulators
   static constexpr uint32_t IDESC = (2u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
   static_assert(TASKS % 32 == 0 && OPS % NG == 0 && RING % NG == 0, "tile shape");
 };
@@ -596,8 +628,8 @@ constexpr size_t gram_tc_smem_bytes() {
   return (size_t)TcShape<B>::OPS * TcShape<B>::STAGE + (size_t)TcShape<B>::RING * TcShape<B>::RAW_BYTES;
 }
 // dynamic + static (the CTA sums, barriers) within the 227 KB a CTA may hold
-static_assert(gram_tc_smem_bytes<16>() + 16 * 16 * 8 + 1024 <= 232448, "Gram stages too large");
-static_assert(gram_tc_smem_bytes<32>() + 32 * 32 * 8 + 1024 <= 232448, "Gram stages too large");
+static_assert(gram_tc_smem_bytes<16>() + 2 * 16 * 16 * 8 + 1024 <= 232448, "Gram stages too large");
+static_assert(gram_tc_smem_bytes<32>() + 2 * 32 * 32 * 8 + 1024 <= 232448, "Gram stages too large");
 
 __device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t (&w)[4]) {
   // w[a] = bytes a of v[0..3]: limb a of four consecutive rows
@@ -640,8 +672,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Thread 0 of the producer: the raw rows (and scales) of `tile` into ring
-// slot `dst` by two 1-D bulk copies completing on `mbar` (rows past the end
+// Thread 0 of the producer: the rows of `tile` of both blocks and their scales
+// into ring slot `dst` by three 1-D bulk copies completing on `mbar` (rows past the end
 // are not copied; the scale copy is rounded up to 16 bytes, which the scale
 // arrays are padded for).
 template <int B>
@@ -652,15 +684,17 @@ __device__ __forceinline__ void tc_fetch(const PassParams& P, int64_t tile, unsi
   const uint32_t ybytes = (uint32_t)rows * B * 4;
   const uint32_t sbytes = (uint32_t)((rows * 4 + 15) & ~15);
   const uint32_t mb = smem_u32(mbar);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(ybytes + sbytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(reinterpret_cast<const uint32_t*>(P.X) + r0 * B), "r"(ybytes), "r"(mb)
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(2 * ybytes + sbytes)
                : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst + T::RAW_Y)),
-               "l"(P.scale + r0), "r"(sbytes), "r"(mb)
-               : "memory");
+  auto copy = [mb](unsigned char* to, const uint32_t* from, uint32_t bytes) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(to)),
+                 "l"(from), "r"(bytes), "r"(mb)
+                 : "memory");
+  };
+  copy(dst, reinterpret_cast<const uint32_t*>(P.X_old) + r0 * B, ybytes);
+  copy(dst + T::RAW_Y, reinterpret_cast<const uint32_t*>(P.X) + r0 * B, ybytes);
+  copy(dst + 2 * T::RAW_Y, P.scale + r0, sbytes);
 }
 
 template <int B>
@@ -672,7 +706,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   __shared__ __align__(8) uint64_t op_full[T::OPS], op_empty[T::OPS];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], fin;
   __shared__ uint32_t tmem_base_s;
-  __shared__ unsigned long long red[B * B];
+  __shared__ unsigned long long red[2 * B * B];  // odd term, even term
   __shared__ bool is_last;
   __shared__ volatile int s_fail;
   __shared__ int64_t s_issued;
@@ -680,10 +714,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ModP M = P.M;
 
-  // zero the operand stages once (the A rows above 4B stay zero), the CTA sums, the barriers
-  for (int e = tid; e < T::OPS * T::STAGE / 16; e += T::THREADS)
-    reinterpret_cast<uint4*>(tc_smem)[e] = make_uint4(0, 0, 0, 0);
-  for (int e = tid; e < B * B; e += T::THREADS) red[e] = 0;
+  for (int e = tid; e < 2 * B * B; e += T::THREADS) red[e] = 0;
   if (tid == 0) {
     s_fail = 0;
     s_issued = 0;
@@ -711,7 +742,6 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the zeroed stages, for the tensor cores
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -724,15 +754,6 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     s_fail = 1;
     atomicExch(status, 1);
   };
-
-  // epilogue state: thread (warp w in 2..5, lane l) owns A row m = 32 (w % 4)
-  // + l = (a, i) and keeps sum_c 256^{a+c} D[m][(c, j)] mod p per lane j
-  uint32_t part[B];
-#pragma unroll
-  for (int j = 0; j < B; ++j) part[j] = 0;
-  const int quad = warp & 3;
-  const int m_row = 32 * quad + lane;
-  const bool reader = warp >= 2 && warp < 6 && m_row < T::MR;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -764,10 +785,10 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a0 = smem_u32(tc_smem + s * T::STAGE), b0 = a0 + T::A_BYTES;
+        const uint32_t b0 = smem_u32(tc_smem + s * T::STAGE), a0 = b0 + (T::A_ROW / 8) * 256;
 #pragma unroll
         for (int kb = 0; kb < T::TILE / 32; ++kb) {
-          const uint64_t da = umma_desc(a0 + kb * (T::M / 8) * 256);
+          const uint64_t da = umma_desc(a0 + kb * (T::N / 8) * 256);
           const uint64_t db = umma_desc(b0 + kb * (T::N / 8) * 256);
           const uint32_t accum = (!first || kb > 0) ? 1u : 0u;
           asm volatile(
@@ -790,10 +811,17 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     }
   } else if (warp < T::XW0) {
     // ------------------------------------------------------------ epilogue
+    // thread (warp w in 2..5, lane l) owns row m = 32 (w % 4) + l of D; the rows
+    // of w' among them, (a, i), add sum_c 256^{a+c} D[m][(c, j)] mod p to the CTA's
+    // sums, per lane j of w (odd term) and of w' (even term)
+    const int quad = warp & 3;
+    const int h_row = 32 * quad + lane - (T::M - T::H);
+    const bool reader = h_row >= 0;
+    const int i = tc_lane<B>(reader ? h_row % B : 0);
     uint32_t wgt[4];  // 2^{8(a + c)} mod p for c = 0..3, a = this row's limb
     {
       uint64_t w = 1;
-      for (int e = 0; e < (reader ? m_row / B : 0); ++e) w = w * 256 % M.p;
+      for (int e = 0; e < (reader ? h_row / B : 0); ++e) w = w * 256 % M.p;
       for (int c = 0; c < 4; ++c) {
         wgt[c] = (uint32_t)w;
         w = w * 256 % M.p;
@@ -807,23 +835,31 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        uint32_t part[B];
 #pragma unroll
-      for (int c0 = 0; c0 < T::N; c0 += 16) {
-        uint32_t v[16];
-        const uint32_t taddr = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(a * T::N + c0);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(taddr)
-            : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (reader) {
+        for (int j = 0; j < B; ++j) part[j] = 0;
+#pragma unroll
+        for (int c0 = 0; c0 < T::H; c0 += 16) {
+          uint32_t v[16];
+          const uint32_t taddr = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(a * T::N + h * T::H + c0);
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+              : "r"(taddr)
+              : "memory");
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int q = 0; q < 16; ++q) {
             const int n = c0 + q, c = n / B, j = tc_lane<B>(n % B);
             part[j] = addmod(part[j], mulmod(v[q], wgt[c], M), M.p);
           }
+        }
+        if (reader) {
+#pragma unroll
+          for (int jj = 0; jj < B; ++jj) atomicAdd(&red[(h * B + i) * B + jj], (unsigned long long)part[jj]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -846,35 +882,33 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
         break;
       }
       const unsigned char* raw = raw0 + slot * T::RAW_BYTES;
-      const uint32_t* scl = reinterpret_cast<const uint32_t*>(raw + T::RAW_Y);
-      unsigned char* const bufA = tc_smem + s * T::STAGE;
-      unsigned char* const bufB = bufA + T::A_BYTES;
+      const uint32_t* scl = reinterpret_cast<const uint32_t*>(raw + 2 * T::RAW_Y);
+      unsigned char* const buf = tc_smem + s * T::STAGE;
       const int64_t r0 = (blockIdx.x + j * gridDim.x) * T::TILE;
-      uint4 y[4];
+      uint4 y[2][4];  // of the old and the new block
       uint32_t sc[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int rr = 4 * qd + q;
         const bool in = r0 + rr < P.rows;
-        y[q] = in ? *reinterpret_cast<const uint4*>(raw + ((size_t)rr * B + 4 * gw) * 4) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          y[h][q] = in ? *reinterpret_cast<const uint4*>(raw + h * T::RAW_Y + ((size_t)rr * B + 4 * gw) * 4)
+                       : make_uint4(0, 0, 0, 0);
         sc[q] = in ? scl[rr] : 0u;
       }
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) {  // lane 4 gw + c4
-        uint32_t z[4], u[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t yv = c4 == 0 ? y[q].x : c4 == 1 ? y[q].y : c4 == 2 ? y[q].z : y[q].w;
-          z[q] = redc_lazy(yv, sc[q], M);
-          u[q] = P.gram_sym ? z[q] : yv;
-        }
-        uint32_t wz[4], wu[4];
-        byte_transpose4(z, wz);
-        byte_transpose4(u, wu);
+        for (int h = 0; h < 2; ++h) {
+          uint32_t z[4], wz[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          *reinterpret_cast<uint32_t*>(bufA + tc_off(T::M, a * B + c4 * T::GROUPS + gw, 4 * qd)) = wz[a];
-          *reinterpret_cast<uint32_t*>(bufB + tc_off(T::N, a * B + c4 * T::GROUPS + gw, 4 * qd)) = wu[a];
+          for (int q = 0; q < 4; ++q)
+            z[q] = redc_lazy(c4 == 0 ? y[h][q].x : c4 == 1 ? y[h][q].y : c4 == 2 ? y[h][q].z : y[h][q].w, sc[q], M);
+          byte_transpose4(z, wz);
+#pragma unroll
+          for (int a = 0; a < 4; ++a)
+            *reinterpret_cast<uint32_t*>(buf + tc_off(T::N, h * T::H + a * B + c4 * T::GROUPS + gw, 4 * qd)) = wz[a];
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // stores visible to the tensor cores
@@ -906,18 +940,11 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::COLS) : "memory");
   }
-  // CTA sums: G[i][j] += part (4 limb rows a per (i, j))
-  if (reader) {
-    const int i = tc_lane<B>(m_row % B);
-#pragma unroll
-    for (int jj = 0; jj < B; ++jj) atomicAdd(&red[i * B + jj], (unsigned long long)part[jj]);
-  }
-  __syncthreads();
   unsigned long long* const acc = P.gram_acc + (size_t)(blockIdx.x % P.replicas) * P.gram_stride;
-  for (int q = tid; q < NP; q += T::THREADS) {
+  for (int q = tid; q < 2 * NP; q += T::THREADS) {
     int i, jj;
-    pair_of(q, B, i, jj);
-    atomicAdd(&acc[q], (unsigned long long)reduce(red[i * B + jj], M));
+    pair_of(q % NP, B, i, jj);
+    atomicAdd(&acc[q], (unsigned long long)reduce(red[(q / NP * B + i) * B + jj], M));
   }
   __threadfence();
   __syncthreads();
@@ -925,21 +952,21 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  // the last CTA: the finished term (real pairs), then reset
+  // the last CTA: the finished terms (real pairs; odd, even), then reset
   const int b = P.b_real;
   const int npr = b * (b + 1) / 2;
   uint32_t* S_out = *P.S_ptr + (size_t)__ldcg(P.term_ctr) * npr;
-  for (int q = tid; q < npr; q += T::THREADS) {
+  for (int q = tid; q < 2 * npr; q += T::THREADS) {
     int i, jj;
-    pair_of(q, b, i, jj);
-    const int qb = pair_index(i, jj, B);
+    pair_of(q % npr, b, i, jj);
+    const int qb = q / npr * NP + pair_index(i, jj, B);
     S_out[q] = mulmod(reduce(sum_replicas(P, qb), M), P.gram_mul, M);
   }
   __syncthreads();
-  for (int q = tid; q < NP * P.replicas; q += T::THREADS)
-    __stcg(P.gram_acc + (size_t)(q / NP) * P.gram_stride + q % NP, 0ull);
+  for (int q = tid; q < 2 * NP * P.replicas; q += T::THREADS)
+    __stcg(P.gram_acc + (size_t)(q / (2 * NP)) * P.gram_stride + q % (2 * NP), 0ull);
   if (tid == 0) {
-    *P.term_ctr += 1u;
+    *P.term_ctr += 2u;
     atomicExch(P.counter, 0u);
   }
 }
@@ -1146,6 +1173,12 @@ constexpr size_t pass_smem_bytes() {
   return (size_t)kWarps * 4 * GramCore<B, 4>::kWords;
 }
 
+// of the even pass that forms both terms
+template <int B>
+constexpr size_t both_smem_bytes() {
+  return (size_t)kWarps * 4 * GramDual<B, 4>::kWords;
+}
+
 // CTAs for a pass over `rows` rows: the resident maximum, but no more CTAs
 // than there are warp batches for (idle CTAs would still add their Gram
 // partials and lengthen the pass on small matrices).
@@ -1196,23 +1229,22 @@ static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 b
   return RR_OK;
 }
 
-// Single-matrix launches: a fused pass (kFusedOdd / kFusedEven) adds its Gram
-// term itself; a lean pass runs without it (no staging, no tensor-core flush,
-// so fewer registers and no shared memory) and is followed by a tcgen05 Gram
-// pass over the block it wrote (kModeGram).  The initial pass computes S_0
-// itself.
+// Single-matrix launches.  The initial pass computes S_0 itself.  The odd pass
+// is lean (no Gram staging, no tensor-core flush, so fewer registers and no
+// shared memory); so is the even pass at widths 16 and 32, whose two terms
+// follow in a Gram pass (kModeGram), while at widths 4 and 8 it adds both.
 template <int B, int FE>
 static int launch_pass_BF(rr_krylov* kr, const PassParams& P, int mode, dim3 grid, cudaStream_t s) {
   const dim3 block(kThreads);
-  const size_t sm = pass_smem_bytes<B>(), sm1 = pass_smem_bytes<B, true>();
   switch (mode) {
-    case kModeInit: return launch_ex(kr, pass_kernel<B, kModeInit, FE, true>, grid, block, sm1, s, P);
+    case kModeInit:
+      return launch_ex(kr, pass_kernel<B, kModeInit, FE>, grid, block, pass_smem_bytes<B, true>(), s, P);
     case kModeOdd:
-      if constexpr (kFusedOdd<B>) return launch_ex(kr, pass_kernel<B, kModeOdd, FE, true>, grid, block, sm, s, P);
-      else return launch_ex(kr, pass_kernel<B, kModeOdd, FE, false, kLeanLpt<B>>, grid, block, 0, s, P);
+      return launch_ex(kr, pass_kernel<B, kModeOdd, FE, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
     case kModeEven:
-      if constexpr (kFusedEven<B>) return launch_ex(kr, pass_kernel<B, kModeEven, FE, true>, grid, block, sm1, s, P);
-      else return launch_ex(kr, pass_kernel<B, kModeEven, FE, false, kLeanLpt<B>>, grid, block, 0, s, P);
+      if constexpr (kGramInPass<B>)
+        return launch_ex(kr, pass_kernel<B, kModeEven, FE, kGramBoth>, grid, block, both_smem_bytes<B>(), s, P);
+      else return launch_ex(kr, pass_kernel<B, kModeEven, FE, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
   }
   return fail(RR_EINVAL, "pass mode %d has no pass kernel at width %d", mode, B);
 }
@@ -1234,7 +1266,7 @@ static int launch_pass_B(rr_krylov* kr, const PassParams& P, int mode) {
       return launch_gram_tc<B>(kr, P, s);
     }
   }
-  const bool lean = (mode == kModeOdd && !kFusedOdd<B>) || (mode == kModeEven && !kFusedEven<B>);
+  const bool lean = mode == kModeOdd || (mode == kModeEven && !kGramInPass<B>);
   const dim3 grid(lean ? pass_grid_lean<B>(kr, P.rows) : pass_grid<B>(kr, P.rows));
   cudaStream_t s = kr->launch_stream ? kr->launch_stream : kr->mat->ctx->stream;
   return kr->fold4 ? launch_pass_BF<B, 4>(kr, P, mode, grid, s) : launch_pass_BF<B, 2>(kr, P, mode, grid, s);
@@ -1287,13 +1319,13 @@ static int occupancy_B(rr_krylov* kr, int* pass_blocks, int* chunk_blocks, int* 
     RR_TRY((set_pass_smem<B, 4>()));
     RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(pass_blocks, pass_kernel<B, kModeOdd, 4>, kThreads, sm));
     RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(chunk_blocks, chunk_kernel<B, 4>, kThreads, 0));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 4, false, kLeanLpt<B>>,
+    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 4, kGramNone, kLeanLpt<B>>,
                                                           kThreads, 0));
   } else {
     RR_TRY((set_pass_smem<B, 2>()));
     RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(pass_blocks, pass_kernel<B, kModeOdd, 2>, kThreads, sm));
     RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(chunk_blocks, chunk_kernel<B, 2>, kThreads, 0));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 2, false, kLeanLpt<B>>,
+    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 2, kGramNone, kLeanLpt<B>>,
                                                           kThreads, 0));
   }
   return RR_OK;
@@ -1448,7 +1480,7 @@ static PassParams base_params(rr_krylov* kr) {
   std::memset(&P, 0, sizeof(P));
   P.heavy_acc = kr->heavy_acc.ptr;
   P.gram_acc = kr->gram_acc.ptr;
-  P.gram_stride = kr->B * (kr->B + 1) / 2;
+  P.gram_stride = kr->B * (kr->B + 1);  // two terms
   P.replicas = kGramReplicas;
   P.counter = kr->counter.ptr;
   P.gram_mul = 1;
@@ -1507,25 +1539,7 @@ int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev) {
   P.X = reinterpret_cast<const uint4*>(x);
   P.Y = reinterpret_cast<uint4*>(kr->U.ptr);
   P.scale = kr->dr_m.ptr;
-  // kFusedOdd / kFusedEven: passes that add their own Gram terms
-  const bool fused_odd = kr->B <= 8, fused_even = kr->B <= 16;
-  if (fused_odd) {
-    P.gram_mul = kr->M.r1;  // the odd pass sums z R^{-1} (x) U
-    P.term_ctr = kr->d_term.ptr;
-    P.S_ptr = kr->d_sptr.ptr;
-  }
   RR_TRY(launch_pass(kr, P, kModeOdd));
-  // odd term: sum over rows of z (x) U with z = U d_r^{-1}
-  if (!fused_odd) {
-    PassParams G = base_params(kr);
-    G.rows = mat->A.live_rows > 0 ? mat->A.live_rows : mat->A.rows;  // zero rows add nothing
-    G.X = reinterpret_cast<const uint4*>(kr->U.ptr);
-    G.scale = kr->drinv_r.ptr;
-    G.gram_sym = 0;
-    G.term_ctr = kr->d_term.ptr;
-    G.S_ptr = kr->d_sptr.ptr;
-    RR_TRY(launch_pass(kr, G, kModeGram));
-  }
   if (ev) RR_CUDA(cudaEventRecord(ev[1], s));
   // pass 2: rows of A^T
   RR_TRY(run_chunks(kr, mat->At, kr->U.ptr));
@@ -1539,19 +1553,20 @@ int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev) {
   P.Y = reinterpret_cast<uint4*>(xn);
   P.scale = kr->dc_m.ptr;
   P.scale2 = kr->dc_r.ptr;
-  P.gram_mul = 1;
-  if (fused_even) {
+  // both terms: w (x) w' and w' (x) w' over the columns, w = x d_c^{-1}
+  if (kr->B <= 8) {  // kGramInPass
+    P.X_old = reinterpret_cast<const uint4*>(x);
+    P.scale3 = kr->dcinv_r.ptr;
     P.term_ctr = kr->d_term.ptr;
     P.S_ptr = kr->d_sptr.ptr;
   }
   RR_TRY(launch_pass(kr, P, kModeEven));
-  // even term: sum over rows of w' (x) w' with w' = x' d_c^{-1}
-  if (!fused_even) {
+  if (kr->B > 8) {
     PassParams G = base_params(kr);
     G.rows = mat->At.live_rows > 0 ? mat->At.live_rows : mat->At.rows;  // zero rows add nothing
+    G.X_old = reinterpret_cast<const uint4*>(x);
     G.X = reinterpret_cast<const uint4*>(xn);
     G.scale = kr->dcinv_r.ptr;
-    G.gram_sym = 1;
     G.term_ctr = kr->d_term.ptr;
     G.S_ptr = kr->d_sptr.ptr;
     RR_TRY(launch_pass(kr, G, kModeGram));

@@ -324,4 +324,151 @@ struct GramMma {
   }
 };
 
+// Both Gram terms of an application from the rows of the even pass: the even
+// term w' (x) w' and the odd term w (x) w' (w the block before the application),
+// which together need one set of operands: no Gram work and no second block of
+// multiply-adds in the odd pass.  Sums: [0, NP) odd, [NP, 2 NP) even.
+template <int B, int FE, int L = kDefaultLpt<B>>
+struct GramDual;
+
+// B = 4: the lanes take the 10 pairs of either term.
+template <int FE>
+struct GramDual<4, FE, 4> {
+  static constexpr int B = 4, RPW = 32, NP = 10;
+  static constexpr int kWords = 2 * RPW * B;
+  uint32_t *zs, *us;  // rows of w' and of w
+  int pi, pj;
+  unsigned long long acc;
+
+  __device__ __forceinline__ void init(uint32_t* w, int lane) {
+    zs = w;
+    us = w + RPW * B;
+    pi = pj = 0;
+    if (lane < 2 * NP) pair_of(lane % NP, B, pi, pj);
+    acc = 0;
+  }
+  __device__ __forceinline__ void add(const uint32_t (&w1)[4], const uint32_t (&w0)[4], int slot, int, int lane,
+                                      const ModP& M, const uint32_t (&)[3]) {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      zs[slot * B + l] = w1[l];
+      us[slot * B + l] = w0[l];
+    }
+    __syncwarp();
+    if (lane < 2 * NP) {
+      const uint32_t* a = lane < NP ? us : zs;
+#pragma unroll
+      for (int rr = 0; rr < RPW; ++rr) {
+        acc = mad_wide(a[rr * B + pi], zs[rr * B + pj], acc);
+        if ((rr % FE) == FE - 1) acc = fold(acc, M);
+      }
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void finish(int, int, int, const ModP&, const uint32_t (&)[3]) {}
+  __device__ __forceinline__ void reset() { acc = 0; }
+  __device__ __forceinline__ void emit(unsigned long long* red, int lane, const ModP& M) {
+    if (lane < 2 * NP) atomicAdd(&red[lane], (unsigned long long)reduce(acc, M));
+  }
+  // the warp's sums as residues, part[pair or NP + pair]
+  __device__ __forceinline__ void store(uint32_t* part, int lane, const ModP& M) {
+    if (lane < 2 * NP) part[lane] = reduce(acc, M);
+  }
+};
+
+// B = 8 on the tensor cores: the 16 rows of an MMA's A operand are the 8 lanes
+// of w' and the 8 of w, so both terms take the products of one.
+template <int FE>
+struct GramDual<8, FE, 4> {
+  static constexpr int B = 8, LPT = 4, TPR = 2, RPW = 16, TB = 2, RS = 9, NP = 36;
+  static constexpr int kWords = 4 * 16 * RS;
+  using Single = GramMma<8, FE, 4>;
+  uint32_t* pl;  // planes [limb][w' lanes 0..7, w lanes 8..15][RS]
+  unsigned long long acc[4];
+  int bt;
+
+  __device__ __forceinline__ void init(uint32_t* w, int) {
+    pl = w;
+    reset();
+  }
+  __device__ __forceinline__ void reset() {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[v] = 0;
+    bt = 0;
+  }
+  __device__ __forceinline__ void stage(const uint32_t (&w1)[LPT], const uint32_t (&w0)[LPT], int slot, int sub) {
+    const int rho = slot & 3, word = (bt * RPW + (slot & ~3)) >> 2;
+#pragma unroll
+    for (int l = 0; l < LPT; ++l) {
+      const int i = Shape<B, 4>::lane_of(sub, l);
+      pl[(rho * 16 + i) * RS + word] = Single::transpose4(w1[l], rho);
+      pl[(rho * 16 + 8 + i) * RS + word] = Single::transpose4(w0[l], rho);
+    }
+  }
+  __device__ __forceinline__ void flush(int lane, const ModP& M, const uint32_t (&W)[3]) {
+    __syncwarp();
+    const int g = lane >> 2, t = lane & 3;
+    uint32_t A[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const uint32_t* r0 = pl + (a * 16 + g) * RS;
+      A[a][0] = r0[t];
+      A[a][1] = r0[8 * RS + t];
+      A[a][2] = r0[t + 4];
+      A[a][3] = r0[8 * RS + t + 4];
+    }
+    // the B operand's column g is lane g of w': the words of A's rows 0..7
+    int C[7][4];
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) C[s][v] = 0;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) mma_u8(C[a + c], A[a], A[c][0], A[c][2]);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      uint64_t x = 0;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) x += (uint64_t)(uint32_t)C[s][v] << (8 * s);
+      uint64_t y = fold(acc[v] + x, M);
+#pragma unroll
+      for (int s = 4; s < 7; ++s) y = mad_wide((uint32_t)C[s][v], W[s - 4], y);
+      acc[v] = y;
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ void add(const uint32_t (&w1)[LPT], const uint32_t (&w0)[LPT], int slot, int sub, int lane,
+                                      const ModP& M, const uint32_t (&W)[3]) {
+    stage(w1, w0, slot, sub);
+    if (++bt == TB) {
+      flush(lane, M, W);
+      bt = 0;
+    }
+  }
+  __device__ __forceinline__ void finish(int slot, int sub, int lane, const ModP& M, const uint32_t (&W)[3]) {
+    if (bt == 0) return;
+    const uint32_t z[LPT] = {0, 0, 0, 0};
+    stage(z, z, slot, sub);  // TB = 2: the one batch the tile did not get
+    flush(lane, M, W);
+    bt = 0;
+  }
+  // entry v of a lane: row g, column 2 t + (v & 1) of the even (v < 2) or odd term
+  __device__ __forceinline__ void emit(unsigned long long* red, int lane, const ModP& M) {
+    const int i = lane >> 2, j0 = 2 * (lane & 3);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int j = j0 + (v & 1);
+      if (i <= j) atomicAdd(&red[(v < 2 ? NP : 0) + pair_index(i, j, B)], (unsigned long long)reduce(acc[v], M));
+    }
+  }
+  // the warp's sums as residues, part[term][i * B + j] for i <= j (others undefined)
+  __device__ __forceinline__ void store(uint32_t* part, int lane, const ModP& M) {
+    const int e = (lane >> 2) * B + 2 * (lane & 3);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) part[(v < 2 ? B * B : 0) + e + (v & 1)] = reduce(acc[v], M);
+  }
+};
+
 }  // namespace rr

@@ -5,9 +5,8 @@
 
 namespace rr {
 
-// kModeGram: no output block; the Gram term of the rows of X with
-// gz = redc(x * scale) and gu = gram_sym ? gz : x (a Gram pass after a pass
-// that did not compute its term).
+// kModeGram: no output block; both Gram terms of an application from the rows
+// of X (the block after it) and X_old (the one before), each scaled by `scale`.
 enum PassMode { kModeInit = 0, kModeOdd = 1, kModeEven = 2, kModeGram = 3 };
 
 struct PassParams {
@@ -22,8 +21,13 @@ struct PassParams {
   uint4* Y;                 // output block   [rows][B/4]
   const uint32_t* scale;    // odd: d_r R^2; even: d_c R^2; init: d_c R   (all mod p)
   const uint32_t* scale2;   // even: d_c R
+  // both Gram terms in one pass: the block before the application, [rows][B/4],
+  // and d_c^{-1} R
+  const uint4* X_old;
+  const uint32_t* scale3;
   unsigned long long* heavy_acc;  // [heavy_rows][B]
-  unsigned long long* gram_acc;   // [replicas][segments][B(B+1)/2]; CTA c adds into replica c % replicas
+  unsigned long long* gram_acc;   // [replicas][gram_stride]; CTA c adds into replica c % replicas.  Per replica:
+                                  // B(B+1)/2 per segment, or the odd and the even term of one matrix
   int64_t gram_stride;            // words per replica (segments * B(B+1)/2)
   int replicas;                   // 1..kGramReplicas
   unsigned int* counter;
@@ -42,7 +46,6 @@ struct PassParams {
   uint32_t gram_mul;        // factor applied to the finished term
   uint32_t w4, w5, w6;      // 2^32, 2^40, 2^48 mod p (limb weights of the tensor-core Gram)
   int b_real;
-  int gram_sym;             // kModeGram: both Gram factors scaled
   ModP M;
   // Batched mode (many matrices stacked block-diagonally, each padded to a
   // multiple of 32 rows): batch_seg[batch] is the matrix of a row batch.  Warps
