@@ -531,8 +531,9 @@ constexpr bool kGramInPass = B <= 8;
 // (8-row x 16-byte core matrices; K-adjacent cores 128 bytes apart, 8-row
 // groups 256 bytes apart); one thread issues the four K = 32 MMAs of a tile.
 // A per-row limb product is < 2^16, so the int32 accumulators are read out
-// every kTcDrain tiles (tcgen05.ld), limb pairs weighted by 2^{8(a+c)} mod p,
-// and the CTA's sums join the same replicated 64-bit accumulators and
+// every kTcDrain tiles (tcgen05.ld): the four limbs c of an entry are joined
+// exactly in 64 bits and kept mod p per limb row (a, i), the four limbs a once
+// at the end; the CTA's sums join the same replicated 64-bit accumulators and
 // last-CTA finish as the pass kernels.  Every wait on an mbarrier gives up
 // after 2 s and sets *status.
 constexpr int kTcDrain = 64;        // tiles between drains of the int32 accumulators
@@ -550,10 +551,10 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
 // Operand rows within a limb: lane i = 4 g + c (g its 128-bit word, c the
 // word's component) sits in row c * B/4 + g, so that the 32 stores of one
 // warp instruction (8 words g x 4 row quads, fixed c) fall in 32 different
-// banks at B = 32.  tc_lane maps a row back to its lane.
+// banks at B = 32.
 template <int B>
-__device__ __forceinline__ constexpr int tc_lane(int r) {
-  return 4 * (r % (B / 4)) + r / (B / 4);
+__device__ __forceinline__ constexpr int tc_row(int lane) {
+  return (lane & 3) * (B / 4) + (lane >> 2);
 }
 
 // Byte offset of (row, k) in a staged operand of R rows x 128 K-bytes.
@@ -567,20 +568,34 @@ __device__ __forceinline__ uint64_t tc_ns() {
   return t;
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}\n"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// Waits read the timer only once a try has failed.
 __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
+  if (mbar_try(addr, parity)) return true;
   const uint64_t t0 = tc_ns();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t}\n"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
+  while (!mbar_try(addr, parity))
     if (tc_ns() - t0 > kTcWaitLimitNs) return false;
-  }
+  return true;
+}
+
+// A bounded wait that also ends when another role of the CTA gave up.
+__device__ __forceinline__ bool mbar_wait_or(uint32_t addr, uint32_t parity, const volatile int* abort) {
+  if (mbar_try(addr, parity)) return true;
+  const uint64_t t0 = tc_ns();
+  while (!mbar_try(addr, parity))
+    if (*abort || tc_ns() - t0 > kTcWaitLimitNs) return false;
+  return true;
 }
 
 // Warp roles of the Gram pass CTA (one CTA per SM):
@@ -595,6 +610,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
 //   warps 6-   transposers, NG groups of TW warps, group g taking tiles
 //              j = g mod NG: scale the rows, split them into byte limbs and
 //              store them in operand stage j mod OPS.
+// The reads of the two blocks are the floor (24 / 30 us at the sizes below); what
+// it takes beyond that is the transposers' multiply-adds and stores, and at
+// either end the fill of the ring and one read-out.  So a raw slot is given back
+// as soon as its rows are in registers, the ring is as deep as shared memory
+// allows at 4 or 2 operand stages, and the read-out reduces 64-bit sums of four
+// limbs (2 B reductions per thread and read-out instead of 8 B, and plain adds
+// to words of its own instead of 64-bit atomics).  Measured, us per launch, without
+// these / with: 750k rows, b = 32: 98.5 / 49.6; 150k rows, b = 32: 49.2 / 21.8;
+// 1.5M rows, b = 16: 92.7 / 48.2; 150k rows, b = 16: 27.6 / 14.3.
+//
 // Hand-offs are mbarriers only (no CTA-wide barrier inside the loop): raw
 // slot full (bulk-copy bytes) / empty (TW arrivals), operand stage full (TW
 // arrivals) / empty (MMA commit), accumulator full (commit) / empty (4
@@ -610,7 +635,7 @@ struct TcShape {
   static constexpr int OPS = B >= 32 ? 2 : 4;                // operand stages
   static constexpr int RAW_Y = TILE * B * 4;                 // a tile's rows of one block
   static constexpr int RAW_BYTES = 2 * RAW_Y + TILE * 4;     // of both, and the row scales
-  static constexpr int RING = 4;                             // raw tiles in flight
+  static constexpr int RING = B >= 32 ? 4 : 8;               // raw tiles in flight
   static constexpr int GROUPS = B / 4;                       // 128-bit words per row
   static constexpr int TASKS = (TILE / 4) * GROUPS;          // 4 rows x 4 lanes each
   static constexpr int TW = TASKS / 32;                      // transposer warps per tile
@@ -620,6 +645,10 @@ struct TcShape {
   static constexpr int THREADS = 32 * WARPS;
   static constexpr int COLS = 2 * N;                         // two accumulators
   static constexpr uint32_t IDESC = (2u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+  static constexpr int SUMS = 2 * B * H;                     // the CTA's sums: [term][lane of w or w'][limb row of w']
+  // a slot's tiles are all one group's: a group that waits for a slot's next
+  // filling has itself taken the one before, so that the parity of its wait is
+  // never two fillings ahead (the copies may complete out of order)
   static_assert(TASKS % 32 == 0 && OPS % NG == 0 && RING % NG == 0, "tile shape");
 };
 
@@ -628,8 +657,8 @@ constexpr size_t gram_tc_smem_bytes() {
   return (size_t)TcShape<B>::OPS * TcShape<B>::STAGE + (size_t)TcShape<B>::RING * TcShape<B>::RAW_BYTES;
 }
 // dynamic + static (the CTA sums, barriers) within the 227 KB a CTA may hold
-static_assert(gram_tc_smem_bytes<16>() + 2 * 16 * 16 * 8 + 1024 <= 232448, "Gram stages too large");
-static_assert(gram_tc_smem_bytes<32>() + 2 * 32 * 32 * 8 + 1024 <= 232448, "Gram stages too large");
+static_assert(gram_tc_smem_bytes<16>() + 4 * TcShape<16>::SUMS + 512 <= 232448, "Gram stages too large");
+static_assert(gram_tc_smem_bytes<32>() + 4 * TcShape<32>::SUMS + 512 <= 232448, "Gram stages too large");
 
 __device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t (&w)[4]) {
   // w[a] = bytes a of v[0..3]: limb a of four consecutive rows
@@ -648,24 +677,6 @@ __device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t
 __device__ __forceinline__ uint32_t redc_lazy(uint32_t y, uint32_t s, const ModP& M) {
   const uint64_t T = (uint64_t)y * s;
   return (uint32_t)(((uint64_t)((uint32_t)T * M.pinv) * M.p + T) >> 32);  // y s + q p < 2 p 2^32
-}
-
-// A bounded wait that also ends when another role of the CTA gave up.
-__device__ __forceinline__ bool mbar_wait_or(uint32_t addr, uint32_t parity, const volatile int* abort) {
-  const uint64_t t0 = tc_ns();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t}\n"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (*abort) return false;
-    if (tc_ns() - t0 > kTcWaitLimitNs) return false;
-  }
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -706,7 +717,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   __shared__ __align__(8) uint64_t op_full[T::OPS], op_empty[T::OPS];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], fin;
   __shared__ uint32_t tmem_base_s;
-  __shared__ unsigned long long red[2 * B * B];  // odd term, even term
+  __shared__ uint32_t sums[T::SUMS];
   __shared__ bool is_last;
   __shared__ volatile int s_fail;
   __shared__ int64_t s_issued;
@@ -714,7 +725,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const ModP M = P.M;
 
-  for (int e = tid; e < 2 * B * B; e += T::THREADS) red[e] = 0;
+  for (int e = tid; e < T::SUMS; e += T::THREADS) sums[e] = 0;
   if (tid == 0) {
     s_fail = 0;
     s_issued = 0;
@@ -812,21 +823,10 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   } else if (warp < T::XW0) {
     // ------------------------------------------------------------ epilogue
     // thread (warp w in 2..5, lane l) owns row m = 32 (w % 4) + l of D; the rows
-    // of w' among them, (a, i), add sum_c 256^{a+c} D[m][(c, j)] mod p to the CTA's
-    // sums, per lane j of w (odd term) and of w' (even term)
+    // of w' among them, (a, i), add sum_c 256^c D[m][(c, j)] mod p to their sums,
+    // per lane j of w (odd term) and of w' (even term)
     const int quad = warp & 3;
     const int h_row = 32 * quad + lane - (T::M - T::H);
-    const bool reader = h_row >= 0;
-    const int i = tc_lane<B>(reader ? h_row % B : 0);
-    uint32_t wgt[4];  // 2^{8(a + c)} mod p for c = 0..3, a = this row's limb
-    {
-      uint64_t w = 1;
-      for (int e = 0; e < (reader ? h_row / B : 0); ++e) w = w * 256 % M.p;
-      for (int c = 0; c < 4; ++c) {
-        wgt[c] = (uint32_t)w;
-        w = w * 256 % M.p;
-      }
-    }
     const int64_t ngrp = (mine + kTcDrain - 1) / kTcDrain;
     for (int64_t G = 0; G < ngrp; ++G) {
       const int a = (int)(G & 1);
@@ -837,29 +837,26 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
-        uint32_t part[B];
+#pragma unroll 1
+        for (int j0 = 0; j0 < B; j0 += 8) {
+          uint32_t v[4][8];
 #pragma unroll
-        for (int j = 0; j < B; ++j) part[j] = 0;
-#pragma unroll
-        for (int c0 = 0; c0 < T::H; c0 += 16) {
-          uint32_t v[16];
-          const uint32_t taddr = tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(a * T::N + h * T::H + c0);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-              : "r"(taddr)
-              : "memory");
+          for (int c = 0; c < 4; ++c)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(v[c][0]), "=r"(v[c][1]), "=r"(v[c][2]), "=r"(v[c][3]), "=r"(v[c][4]), "=r"(v[c][5]),
+                           "=r"(v[c][6]), "=r"(v[c][7])
+                         : "r"(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(a * T::N + h * T::H + c * B + j0))
+                         : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (h_row >= 0) {
+            uint32_t* const sum = sums + (h * B + j0) * T::H + h_row;
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            const int n = c0 + q, c = n / B, j = tc_lane<B>(n % B);
-            part[j] = addmod(part[j], mulmod(v[q], wgt[c], M), M.p);
+            for (int q = 0; q < 8; ++q) {
+              const uint64_t x = (uint64_t)v[0][q] + ((uint64_t)v[1][q] << 8) + ((uint64_t)v[2][q] << 16) +
+                                 ((uint64_t)v[3][q] << 24);
+              sum[q * T::H] = addmod(sum[q * T::H], reduce(x, M), M.p);
+            }
           }
-        }
-        if (reader) {
-#pragma unroll
-          for (int jj = 0; jj < B; ++jj) atomicAdd(&red[(h * B + i) * B + jj], (unsigned long long)part[jj]);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -877,25 +874,24 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
         give_up();
         break;
       }
-      if (j >= T::OPS && !mbar_wait_or(smem_u32(&op_empty[s]), (uint32_t)((j / T::OPS - 1) & 1), &s_fail)) {
-        give_up();
-        break;
-      }
       const unsigned char* raw = raw0 + slot * T::RAW_BYTES;
       const uint32_t* scl = reinterpret_cast<const uint32_t*>(raw + 2 * T::RAW_Y);
       unsigned char* const buf = tc_smem + s * T::STAGE;
       const int64_t r0 = (blockIdx.x + j * gridDim.x) * T::TILE;
       uint4 y[2][4];  // of the old and the new block
-      uint32_t sc[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int rr = 4 * qd + q;
-        const bool in = r0 + rr < P.rows;
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          y[h][q] = in ? *reinterpret_cast<const uint4*>(raw + h * T::RAW_Y + ((size_t)rr * B + 4 * gw) * 4)
-                       : make_uint4(0, 0, 0, 0);
-        sc[q] = in ? scl[rr] : 0u;
+        for (int q = 0; q < 4; ++q)
+          y[h][q] = *reinterpret_cast<const uint4*>(raw + h * T::RAW_Y + ((size_t)(4 * qd + q) * B + 4 * gw) * 4);
+      const uint4 s4 = *reinterpret_cast<const uint4*>(scl + 4 * qd);
+      const int64_t left = P.rows - (r0 + 4 * qd);  // rows past the end: scale 0, so 0 whatever y is
+      const uint32_t sc[4] = {left > 0 ? s4.x : 0u, left > 1 ? s4.y : 0u, left > 2 ? s4.z : 0u, left > 3 ? s4.w : 0u};
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&raw_empty[slot]);  // the rows are in registers: the next copy may come
+      if (j >= T::OPS && !mbar_wait_or(smem_u32(&op_empty[s]), (uint32_t)((j / T::OPS - 1) & 1), &s_fail)) {
+        give_up();
+        break;
       }
 #pragma unroll
       for (int c4 = 0; c4 < 4; ++c4) {  // lane 4 gw + c4
@@ -913,10 +909,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // stores visible to the tensor cores
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&op_full[s]);
-        mbar_arrive(&raw_empty[slot]);
-      }
+      if (lane == 0) mbar_arrive(&op_full[s]);
     }
   }
   griddep_launch();
@@ -944,7 +937,11 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   for (int q = tid; q < 2 * NP; q += T::THREADS) {
     int i, jj;
     pair_of(q % NP, B, i, jj);
-    atomicAdd(&acc[q], (unsigned long long)reduce(red[(q / NP * B + i) * B + jj], M));
+    const uint32_t* sum = sums + (q / NP * B + tc_row<B>(jj)) * T::H + tc_row<B>(i);
+    uint64_t x = 0;  // sum_a 256^a (limb row (a, i))
+#pragma unroll
+    for (int a = 0; a < 4; ++a) x += (uint64_t)sum[a * B] << (8 * a);
+    atomicAdd(&acc[q], (unsigned long long)reduce(x, M));
   }
   __threadfence();
   __syncthreads();
