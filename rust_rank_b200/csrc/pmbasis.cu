@@ -48,17 +48,16 @@ constexpr int kNttBlock = 4096;  // elements transformed per CTA in shared memor
 constexpr int kBaseThreads = 512;
 constexpr size_t kBaseSmemBudget = 220 * 1024;  // dynamic shared memory of one block kernel
 
-struct Twiddles {
-  const uint32_t* w;   // omega^j, j < Nmax/2
-  const uint32_t* ws;  // floor(w * 2^32 / p)
-  int64_t nmax;
-};
-
 __device__ __forceinline__ uint32_t mul_shoup(uint32_t a, uint32_t w, uint32_t ws, uint32_t p) {
   const uint32_t q = __umulhi(a, ws);
   uint32_t r = a * w - q * p;  // in [0, 2p), computed mod 2^32
   return r >= p ? r - p : r;
 }
+
+// Twiddle table of an order-nmax root w: entry h + j, h = 1, 2, 4 .. nmax / 2 and
+// j < h, is (w^(j nmax / 2h), its Shoup quotient): the twiddles of a stage of
+// span 2h are consecutive.
+__device__ __forceinline__ uint32_t mul_tw(uint32_t a, uint2 t, uint32_t p) { return mul_shoup(a, t.x, t.y, p); }
 
 // A batch of strided polynomial matrices seen as a flat list of polynomials:
 // polynomial q is entry (qi / cols, qi % cols) of matrix q / npb (qi = q % npb),
@@ -75,33 +74,31 @@ struct PolyView {
 
 // ---------------------------------------------------------------- NTT kernels
 // Forward DIF stage with butterfly span `len` (len > kNttBlock) in global memory.
-__global__ void ntt_fwd_stage_kernel(uint32_t* a, int64_t N, int64_t npoly, int64_t len, Twiddles tw, uint32_t p) {
+__global__ void ntt_fwd_stage_kernel(uint32_t* a, int64_t N, int64_t npoly, int64_t len, const uint2* tw, uint32_t p) {
   const int64_t half = len / 2;
   const int lh = __ffsll(half) - 1, lp = __ffsll(N / 2) - 1;
   const int64_t total = npoly * (N / 2);
-  const int64_t tstep = tw.nmax / len;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t poly = t >> lp, b = t & (N / 2 - 1);
     const int64_t j = b & (half - 1);
     uint32_t* x = a + poly * N + ((b >> lh) << (lh + 1)) + j;
     const uint32_t u = x[0], v = x[half];
     x[0] = addmod(u, v, p);
-    x[half] = mul_shoup(submod(u, v, p), tw.w[j * tstep], tw.ws[j * tstep], p);
+    x[half] = mul_tw(submod(u, v, p), __ldg(tw + half + j), p);
   }
 }
 
 // Inverse DIT stage with span len (len > kNttBlock) in global memory.
-__global__ void ntt_inv_stage_kernel(uint32_t* a, int64_t N, int64_t npoly, int64_t len, Twiddles tw, uint32_t p) {
+__global__ void ntt_inv_stage_kernel(uint32_t* a, int64_t N, int64_t npoly, int64_t len, const uint2* tw, uint32_t p) {
   const int64_t half = len / 2;
   const int lh = __ffsll(half) - 1, lp = __ffsll(N / 2) - 1;
   const int64_t total = npoly * (N / 2);
-  const int64_t tstep = tw.nmax / len;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t poly = t >> lp, b = t & (N / 2 - 1);
     const int64_t j = b & (half - 1);
     uint32_t* x = a + poly * N + ((b >> lh) << (lh + 1)) + j;
     const uint32_t u = x[0];
-    const uint32_t v = mul_shoup(x[half], tw.w[j * tstep], tw.ws[j * tstep], p);
+    const uint32_t v = mul_tw(x[half], __ldg(tw + half + j), p);
     x[0] = addmod(u, v, p);
     x[half] = submod(u, v, p);
   }
@@ -109,60 +106,70 @@ __global__ void ntt_inv_stage_kernel(uint32_t* a, int64_t N, int64_t npoly, int6
 
 // Shared-memory NTT of the last (forward) or first (inverse) stages, span up
 // to T = 2^logT <= kNttBlock.  A CTA transforms G = max(1, kNttGroup / T)
-// consecutive T-blocks (several short polynomials per CTA), with the twiddles
-// of span T staged in shared memory (span 2^lg uses entry j << (logT - lg))
-// and power-of-two index arithmetic.  Dynamic shared memory: (G + 1) * T words.
+// consecutive T-blocks (several short polynomials per CTA).  Two stages at a
+// time on four values in registers (an odd stage left over is the one of span
+// 2, whose twiddle is 1): half the shared-memory passes and barriers.  The
+// twiddles of a pass are consecutive words of the table (L1), the values are
+// padded so that the passes of span 4 to 64 meet no bank conflicts, and where a
+// polynomial starts is worked out once per block, not per value.
+// Bound by the latency of the passes at short lengths, by the transforms' traffic
+// at long ones.  Measured, us per launch, mean over the 65536-order generator at
+// b = 16 (1024 polynomials of 128 .. 4096 values): 22.8 forward and 21.7 inverse
+// with one stage per pass and one table strided for every span (up to 32 lanes of
+// a warp on one bank), 12.4 and 11.8 so.
 constexpr int kNttGroup = 2048;
 
-__device__ __forceinline__ void ntt_load_twiddles(uint32_t* W, uint32_t* WS, int logT, const Twiddles& tw) {
-  const int64_t tstep = tw.nmax >> logT;
-  for (int j = threadIdx.x; j < (1 << (logT - 1)); j += blockDim.x) {
-    W[j] = tw.w[j * tstep];
-    WS[j] = tw.ws[j * tstep];
-  }
-}
+__device__ __forceinline__ int ntt_pad(int i) { return i + ((i >> 5) << 2); }
+
+// Dynamic shared memory: G block pointers, then the padded values.
+__device__ __forceinline__ uint32_t* ntt_values(void* sm, int G) { return (uint32_t*)sm + 2 * ((G + 1) & ~1); }
 
 // Forward DIF.  When src.p != nullptr the blocks are first loaded from the
 // polynomials of src (t < src_len, zero padded) -- only valid when N <= kNttBlock.
 __global__ void __launch_bounds__(512) ntt_fwd_smem_kernel(uint32_t* a, int64_t N, int logT, int64_t nblocks,
-                                                           PolyView src, int64_t src_len, Twiddles tw, uint32_t p) {
-  extern __shared__ uint32_t nsm[];
+                                                           PolyView src, int64_t src_len, const uint2* tw, uint32_t p) {
+  extern __shared__ __align__(16) uint64_t nsm[];
   const int T = 1 << logT, G = T >= kNttGroup ? 1 : kNttGroup / T;
-  uint32_t* s = nsm;
-  uint32_t* W = s + G * T;
-  uint32_t* WS = W + T / 2;
+  const uint32_t** const from = (const uint32_t**)nsm;
+  uint32_t* const s = ntt_values(nsm, G);
   const int64_t blk0 = (int64_t)blockIdx.x * G;
-  ntt_load_twiddles(W, WS, logT, tw);
+  for (int g = threadIdx.x; g < G; g += blockDim.x)
+    from[g] = blk0 + g >= nblocks ? nullptr : src.p ? src.at(blk0 + g) : a + ((blk0 + g) << logT);
+  __syncthreads();
+  const int len = src.p ? (int)src_len : T;
   for (int e = threadIdx.x; e < G * T; e += blockDim.x) {
-    const int g = e >> logT, t = e & (T - 1);
-    const int64_t blk = blk0 + g;
-    uint32_t v = 0;
-    if (blk < nblocks) {
-      if (src.p) {  // N == T: block = polynomial; residues mod p < 2^31 < 2q, one subtraction reduces them mod q
-        v = t < src_len ? src.at(blk)[t] : 0u;
-        v = v >= p ? v - p : v;
-      } else {
-        v = a[(blk << logT) + t];
-      }
-    }
-    s[e] = v;
+    const int t = e & (T - 1);
+    const uint32_t* const x = from[e >> logT];
+    const uint32_t v = x != nullptr && t < len ? x[t] : 0u;
+    s[ntt_pad(e)] = v >= p ? v - p : v;  // residues mod the matrix prime < 2^31 < 2p
   }
   __syncthreads();
-  const int nbf = G * T / 2;
-  for (int lg = logT; lg >= 1; --lg) {
-    const int lh = lg - 1, half = 1 << lh, sh = logT - lg;
-    for (int bf = threadIdx.x; bf < nbf; bf += blockDim.x) {
-      const int j = bf & (half - 1);
-      const int i0 = ((bf >> lh) << lg) | j;
-      const uint32_t u = s[i0], v = s[i0 + half];
-      s[i0] = addmod(u, v, p);
-      s[i0 + half] = mul_shoup(submod(u, v, p), W[j << sh], WS[j << sh], p);
+  int lg = logT;
+  for (; lg >= 2; lg -= 2) {
+    const int lq = lg - 2, q = 1 << lq;
+    for (int bf = threadIdx.x; bf < G * T / 4; bf += blockDim.x) {
+      const int j = bf & (q - 1);
+      const int i = ((bf >> lq) << lg) | j;
+      const int i0 = ntt_pad(i), i1 = ntt_pad(i + q), i2 = ntt_pad(i + 2 * q), i3 = ntt_pad(i + 3 * q);
+      const uint2 w1 = __ldg(tw + 2 * q + j), w2 = __ldg(tw + 3 * q + j), w3 = __ldg(tw + q + j);
+      const uint32_t x0 = s[i0], x1 = s[i1], x2 = s[i2], x3 = s[i3];
+      const uint32_t a0 = addmod(x0, x2, p), a2 = mul_tw(submod(x0, x2, p), w1, p);
+      const uint32_t a1 = addmod(x1, x3, p), a3 = mul_tw(submod(x1, x3, p), w2, p);
+      s[i0] = addmod(a0, a1, p);
+      s[i1] = mul_tw(submod(a0, a1, p), w3, p);
+      s[i2] = addmod(a2, a3, p);
+      s[i3] = mul_tw(submod(a2, a3, p), w3, p);
     }
     __syncthreads();
   }
   for (int e = threadIdx.x; e < G * T; e += blockDim.x) {
     const int64_t blk = blk0 + (e >> logT);
-    if (blk < nblocks) a[(blk << logT) + (e & (T - 1))] = s[e];
+    uint32_t v = s[ntt_pad(e)];
+    if (lg == 1) {
+      const uint32_t o = s[ntt_pad(e ^ 1)];
+      v = e & 1 ? submod(o, v, p) : addmod(v, o, p);
+    }
+    if (blk < nblocks) a[(blk << logT) + (e & (T - 1))] = v;
   }
 }
 
@@ -171,44 +178,52 @@ __global__ void __launch_bounds__(512) ntt_fwd_smem_kernel(uint32_t* a, int64_t 
 // the polynomials of dst.
 __global__ void __launch_bounds__(512) ntt_inv_smem_kernel(uint32_t* a, int64_t N, int logT, int64_t nblocks,
                                                            PolyView dst, int64_t lo, int64_t cnt, uint32_t ninv,
-                                                           uint32_t ninv_s, Twiddles tw, uint32_t p) {
-  extern __shared__ uint32_t nsm[];
+                                                           uint32_t ninv_s, const uint2* tw, uint32_t p) {
+  extern __shared__ __align__(16) uint64_t nsm[];
   const int T = 1 << logT, G = T >= kNttGroup ? 1 : kNttGroup / T;
-  uint32_t* s = nsm;
-  uint32_t* W = s + G * T;
-  uint32_t* WS = W + T / 2;
+  uint32_t** const to = (uint32_t**)nsm;
+  uint32_t* const s = ntt_values(nsm, G);
   const int64_t blk0 = (int64_t)blockIdx.x * G;
-  ntt_load_twiddles(W, WS, logT, tw);
+  for (int g = threadIdx.x; g < G; g += blockDim.x)
+    to[g] = blk0 + g >= nblocks ? nullptr : dst.p ? dst.at(blk0 + g) : a + ((blk0 + g) << logT);
   for (int e = threadIdx.x; e < G * T; e += blockDim.x) {
     const int64_t blk = blk0 + (e >> logT);
-    s[e] = blk < nblocks ? a[(blk << logT) + (e & (T - 1))] : 0u;
+    uint32_t v = 0;
+    if (blk < nblocks) {
+      const uint32_t* const x = a + (blk << logT);
+      const int t = e & (T - 1);
+      v = x[t];
+      if (logT & 1) {
+        const uint32_t o = x[t ^ 1];
+        v = t & 1 ? submod(o, v, p) : addmod(v, o, p);
+      }
+    }
+    s[ntt_pad(e)] = v;
   }
   __syncthreads();
-  const int nbf = G * T / 2;
-  for (int lg = 1; lg <= logT; ++lg) {
-    const int lh = lg - 1, half = 1 << lh, sh = logT - lg;
-    for (int bf = threadIdx.x; bf < nbf; bf += blockDim.x) {
-      const int j = bf & (half - 1);
-      const int i0 = ((bf >> lh) << lg) | j;
-      const uint32_t u = s[i0];
-      const uint32_t v = mul_shoup(s[i0 + half], W[j << sh], WS[j << sh], p);
-      s[i0] = addmod(u, v, p);
-      s[i0 + half] = submod(u, v, p);
+  for (int lq = logT & 1; lq < logT; lq += 2) {
+    const int q = 1 << lq;
+    for (int bf = threadIdx.x; bf < G * T / 4; bf += blockDim.x) {
+      const int j = bf & (q - 1);
+      const int i = ((bf >> lq) << (lq + 2)) | j;
+      const int i0 = ntt_pad(i), i1 = ntt_pad(i + q), i2 = ntt_pad(i + 2 * q), i3 = ntt_pad(i + 3 * q);
+      const uint2 w1 = __ldg(tw + 2 * q + j), w2 = __ldg(tw + 3 * q + j), w3 = __ldg(tw + q + j);
+      const uint32_t x0 = s[i0], x1 = mul_tw(s[i1], w3, p), x2 = s[i2], x3 = mul_tw(s[i3], w3, p);
+      const uint32_t a0 = addmod(x0, x1, p), a1 = submod(x0, x1, p);
+      const uint32_t a2 = mul_tw(addmod(x2, x3, p), w1, p), a3 = mul_tw(submod(x2, x3, p), w2, p);
+      s[i0] = addmod(a0, a2, p);
+      s[i1] = addmod(a1, a3, p);
+      s[i2] = submod(a0, a2, p);
+      s[i3] = submod(a1, a3, p);
     }
     __syncthreads();
   }
-  if (dst.p) {
-    for (int e = threadIdx.x; e < G * cnt; e += blockDim.x) {
-      const int g = (int)(e / cnt);
-      const int64_t t = e - (int64_t)g * cnt;
-      const int64_t blk = blk0 + g;
-      if (blk < nblocks) dst.at(blk)[t] = mul_shoup(s[(g << logT) + lo + t], ninv, ninv_s, p);
-    }
-  } else {
-    for (int e = threadIdx.x; e < G * T; e += blockDim.x) {
-      const int64_t blk = blk0 + (e >> logT);
-      if (blk < nblocks) a[(blk << logT) + (e & (T - 1))] = s[e];
-    }
+  const int first = dst.p ? (int)lo : 0, count = dst.p ? (int)cnt : T;
+  for (int e = threadIdx.x; e < G * count; e += blockDim.x) {
+    const int g = e / count, t = e - g * count;
+    uint32_t v = s[ntt_pad((g << logT) + first + t)];
+    if (dst.p) v = mul_shoup(v, ninv, ninv_s, p);
+    if (to[g] != nullptr) to[g][t] = v;
   }
 }
 
@@ -365,24 +380,23 @@ __global__ void unwrap_kernel(PolyView A, PolyView Bm, PolyView dst, int m, int 
   }
 }
 
-// Twiddle tables of a transform prime: w^j and w^-j with their Shoup quotients.
-__global__ void twiddle_kernel(uint32_t* tw, uint32_t* tws, uint32_t* twi, uint32_t* twis, int64_t half, uint32_t w,
-                               uint32_t wi, ModP M) {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= half) return;
+// Twiddle tables (forward w, inverse wi) of a transform prime, entry e = h + j.
+__global__ void twiddle_kernel(uint2* tw, uint2* twi, int64_t nmax, uint32_t w, uint32_t wi, ModP M) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nmax) return;
+  int64_t h = 1;
+  while (2 * h <= e) h *= 2;
   uint32_t x = 1, y = 1, bx = w, by = wi;
-  for (int64_t e = j; e; e >>= 1) {
-    if (e & 1) {
+  for (int64_t k = e < 1 ? 0 : (e - h) * (nmax / (2 * h)); k; k >>= 1) {
+    if (k & 1) {
       x = mulmod(x, bx, M);
       y = mulmod(y, by, M);
     }
     bx = mulmod(bx, bx, M);
     by = mulmod(by, by, M);
   }
-  tw[j] = x;
-  twi[j] = y;
-  tws[j] = (uint32_t)(((uint64_t)x << 32) / M.p);
-  twis[j] = (uint32_t)(((uint64_t)y << 32) / M.p);
+  tw[e] = make_uint2(x, (uint32_t)(((uint64_t)x << 32) / M.p));
+  twi[e] = make_uint2(y, (uint32_t)(((uint64_t)y << 32) / M.p));
 }
 
 // G[i][j][t] = seq[pair(i,j)][t] for i < b; G[b+i][i][0] = 1 (src/sigma_basis.rs:33-46)
@@ -1077,15 +1091,15 @@ int grid_for(int64_t work, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 32));
 }
 
-// An NTT prime q with its twiddle tables (w^j and Shoup quotients, forward
-// and inverse, j < nmax / 2) and the pointwise stage's fold rule.
+// An NTT prime q with its twiddle tables (forward and inverse, nmax entries)
+// and the pointwise stage's fold rule.
 struct NttPrime {
   uint32_t q = 0;
   ModP M{};
   int64_t nmax = 0;
-  DevBuf<uint32_t> tw, tws, twi, twis;
-  Twiddles fwd() const { return Twiddles{tw.ptr, tws.ptr, nmax}; }
-  Twiddles inv() const { return Twiddles{twi.ptr, twis.ptr, nmax}; }
+  DevBuf<uint2> tw, twi;
+  const uint2* fwd() const { return tw.ptr; }
+  const uint2* inv() const { return twi.ptr; }
 };
 
 // Four products fit between folds of a 64-bit accumulator iff
@@ -1151,9 +1165,9 @@ NttShape ntt_shape(int64_t T, int64_t nblocks) {
   sh.logT = 0;
   while ((1ll << sh.logT) < T) ++sh.logT;
   sh.G = T >= kNttGroup ? 1 : (int)(kNttGroup / T);
-  sh.threads = (int)std::min<int64_t>(512, std::max<int64_t>(32, sh.G * T / 2));
+  sh.threads = (int)std::min<int64_t>(512, std::max<int64_t>(32, sh.G * T / 4));
   sh.grid = (unsigned)((nblocks + sh.G - 1) / sh.G);
-  sh.smem = (size_t)(sh.G * T + T) * 4;
+  sh.smem = (size_t)((sh.G + 1) & ~1) * 8 + (size_t)(sh.G * T + sh.G * T / 8) * 4;  // pointers, padded values
   return sh;
 }
 
@@ -1465,12 +1479,10 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
       Q->nmax = nmax;
       const uint32_t g = find_generator(q);
       const uint32_t w = host_powmod(g, (q - 1) / (uint64_t)nmax, q);
-      RR_TRY(Q->tw.alloc_async(nmax / 2, P.s));
-      RR_TRY(Q->tws.alloc_async(nmax / 2, P.s));
-      RR_TRY(Q->twi.alloc_async(nmax / 2, P.s));
-      RR_TRY(Q->twis.alloc_async(nmax / 2, P.s));
-      twiddle_kernel<<<(unsigned)((nmax / 2 + 255) / 256), 256, 0, P.s>>>(
-          Q->tw.ptr, Q->tws.ptr, Q->twi.ptr, Q->twis.ptr, nmax / 2, w, host_invmod(w, q), Q->M);
+      RR_TRY(Q->tw.alloc_async(nmax, P.s));
+      RR_TRY(Q->twi.alloc_async(nmax, P.s));
+      twiddle_kernel<<<(unsigned)((nmax + 255) / 256), 256, 0, P.s>>>(Q->tw.ptr, Q->twi.ptr, nmax, w,
+                                                                      host_invmod(w, q), Q->M);
       RR_CUDA(cudaGetLastError());
       P.nps.push_back(std::move(Q));
     }
