@@ -1139,6 +1139,7 @@ struct Pm {
   DevBuf<int> status;
   int64_t cs = 0;                      // residual coefficient stride of the leaves kernel (words)
   int fold4 = 0;
+  int64_t direct = 0;                  // levels up to this half length take direct products
   bool mma = false;                    // leaf blocks on clusters and tensor cores (pmleaf.cu)
   // per recursion depth: MM, GG, MMM ([nb] each)
   std::vector<std::unique_ptr<DevBuf<uint32_t>>> bufs;
@@ -1282,7 +1283,7 @@ int direct_or_fail(Pm& P, MatView A, int64_t la, MatView B, int k, int64_t lb, M
 int level_product(Pm& P, MatView A, int64_t la, bool a_is_mm, MatView B, int k, int64_t lb, MatView dst, int64_t lo,
                   int64_t cnt, int64_t h, uint32_t* keep) {
   const int m = P.m;
-  if (P.mma && h <= direct_product_max(m)) return direct_or_fail(P, A, la, B, k, lb, dst, lo, cnt);
+  if (h <= P.direct) return direct_or_fail(P, A, la, B, k, lb, dst, lo, cnt);
   const int64_t N = 2 * h;
   if (N > P.nmax) return fail(RR_EINVAL, "internal: NTT length %lld exceeds table %lld", (long long)N, (long long)P.nmax);
   const int64_t ncoef = std::min<int64_t>(cnt, N - lo);  // M's last coefficient is not in the transform
@@ -1449,8 +1450,16 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   // NTT products: modulo p itself when p - 1 is divisible by the transform
   // length, else exact integer products by CRT over two or three NTT primes
   // (whose product must exceed inner dimension x length x (p-1)^2)
-  const int64_t direct = P.mma ? direct_product_max(m) : 0;  // levels up to this half length take direct products
-  P.use_ntt = d > P.K && d / 2 > direct;
+  P.direct = P.mma ? direct_product_max(m) : 0;
+  // The transform path's launches cost the same for many generators, the direct
+  // products grow with them, so in batches of some size the line lies one level
+  // lower (transforms modulo p only: the CRT primes take two or three times the
+  // work).  Measured (ms for the batch, lower / this line): 8 generators b = 16,
+  // d = 1024: 11.4 / 12.2; 16: 21.1 / 23.2; 8 of b = 8, d = 2048: 11.2 / 11.8; 2 of
+  // b = 32, d = 512: 11.6 / 12.2; but alone at b = 16, d = 2^14: 90.7 / 88.6, and 2
+  // of b = 16: 8.7 / 8.5.
+  if ((int64_t)nb * m >= 128 && (uint64_t)(p - 1) % (uint64_t)nmax == 0) P.direct /= 2;
+  P.use_ntt = d > P.K && d / 2 > P.direct;
   if (P.mma && d > P.K) RR_TRY(direct_product_prepare());
   if (P.use_ntt) {
     std::vector<uint32_t> qs;
@@ -1492,7 +1501,7 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
     if (P.crt)
       for (size_t i = 0; i < P.nps.size(); ++i) RR_TRY(P.R[i].alloc_async((size_t)nb * m * m * (d + 1), P.s));
     else
-      for (int64_t dd = d; dd > P.K && dd / 2 > direct; dd /= 2) {
+      for (int64_t dd = d; dd > P.K && dd / 2 > P.direct; dd /= 2) {
         P.FM.emplace_back(new DevBuf<uint32_t>());
         RR_TRY(P.FM.back()->alloc_async((size_t)nb * m * m * dd, P.s));
       }

@@ -28,3 +28,14 @@ def test_lengths(pm_ctx, b, d, p):
     Mo, do = oracle.pm_basis(seq, b, d, p)
     assert np.array_equal(M, Mo.astype(np.uint32))
     assert np.array_equal(delta, do)
+
+
+@pytest.mark.parametrize("b,d,nb", [(8, 512, 7), (8, 512, 8), (13, 256, 5), (16, 128, 4), (32, 64, 2)])
+def test_batches_around_the_direct_products(ctx, b, d, nb):
+    """Batches on both sides of 128 rows, from which the shorter products are transforms too."""
+    p = 2013265921
+    rng = np.random.default_rng(nb)
+    seqs = [rng.integers(0, p, size=(b * (b + 1) // 2, d + 1)).astype(np.uint32) for _ in range(nb)]
+    for seq, (M, delta) in zip(seqs, rr.PM_Basis_batch(seqs, d, p, ctx)):
+        Mo, do = oracle.pm_basis(seq, b, d, p)
+        assert np.array_equal(M, Mo.astype(np.uint32)) and np.array_equal(delta, do)
