@@ -278,9 +278,8 @@ int rr_krylov_create(rr_matrix* mat, int32_t b, const uint32_t* row_precond, con
     RR_TRY(kr->dc_m.alloc_async(n, s));
     RR_TRY(kr->dc_r.alloc_async(n, s));
     RR_TRY(kr->dcinv.alloc_async(n, s));
-    // + 4: the Gram pass copies row scales in 16-byte pieces
-    RR_TRY(kr->drinv_r.alloc_async(m + 4, s));
-    RR_TRY(kr->dcinv_r.alloc_async(n + 4, s));
+    RR_TRY(kr->drinv_r.alloc_async(m, s));
+    RR_TRY(kr->dcinv_r.alloc_async(n + 4, s));  // + 4: the Gram pass copies its row scales in 16-byte pieces
     RR_TRY(rr::upload_host(mat->ctx, {{rp.ptr, row_precond, (size_t)m * 4}, {cp.ptr, col_precond, (size_t)n * 4}}, s));
     RR_TRY(launch_precond(kr.get(), rp.ptr, cp.ptr, mat->d_rowperm.ptr));
   }  // the staging buffers are freed in stream order, after the kernel

@@ -10,8 +10,11 @@
 // the device is x_k = D_c w_k, so A is used with its raw entries and the
 // diagonal preconditioners are applied in the epilogues:
 //
-//   pass 1 (rows of A):   z = A x;  U = D_r z;  Gram_odd  += z (x) U
-//   pass 2 (rows of A^T): t = A^T U; w' = D_c t; x' = D_c w';  Gram_even += w' (x) w'
+//   pass 1 (rows of A):   z = A x;  U = D_r z
+//   pass 2 (rows of A^T): t = A^T U; w' = D_c t; x' = D_c w'
+//   both terms, over the same rows:  w (x) w'  and  w' (x) w',  w = D_c^{-1} x
+//
+// (batches of matrices form the odd term in pass 1, as z (x) U).
 //
 // The block is stored interleaved, X[row][B] uint32 (B = 4..32 lanes); a
 // thread owns 8 lanes (4 when B = 4) and gathers them with 128-bit loads, so a
@@ -21,10 +24,11 @@
 // flight per thread.  Sums are accumulated lazily in 64 bits with a fold every
 // 2 or 4 products and finished with a Montgomery reduction; the factor R^{-1}
 // it leaves is absorbed into the preconditioner scales (d R^2 mod p, d R mod p)
-// and, for the odd term, into one final multiplication by R.
+// and, for an odd term formed in pass 1, into one final multiplication by R.
 //
-// The Gram terms are reduced per CTA in shared memory, then across CTAs with
-// 64-bit atomics; the last CTA to finish writes the finished term and resets
+// At widths up to 8 pass 2 forms the terms, at 16 and 32 a tcgen05 pass after
+// it.  They are reduced per CTA in shared memory, then across CTAs with
+// 64-bit atomics; the last CTA to finish writes the finished terms and resets
 // the accumulators, so no separate reduction kernel and no host round trip is
 // needed.
 //
@@ -507,9 +511,9 @@ constexpr int kLeanLpt = (B == 16) ? 4 : kDefaultLpt<B>;
 // but needs a second pass over U).  Widths up to 8 form them in the even pass
 // (GramDual), wider ones in a tcgen05 pass over the old and the new block
 // (gram_tc_kernel).  Measured (us per application, odd term from the rows of A /
-// both from the columns): 2M x 1.5M Zipf, b = 16: 533 / 516, b = 5: 362 / 326;
-// 1M x 750k Zipf, b = 32: 460 / 451; 600k x 500k incidence, b = 16: 148 / 129;
-// 190k x 150k incidence, b = 32: 104 / 99; 60k x 50k Zipf, b = 4: 28.9 / 23.6.
+// both from the columns): 2M x 1.5M Zipf, b = 16: 533 / 485, b = 5: 362 / 324;
+// 1M x 750k Zipf, b = 32: 460 / 409; 600k x 500k incidence, b = 16: 148 / 110;
+// 190k x 150k incidence, b = 32: 104 / 72; 60k x 50k Zipf, b = 4: 28.9 / 23.0.
 template <int B>
 constexpr bool kGramInPass = B <= 8;
 
