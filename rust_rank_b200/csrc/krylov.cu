@@ -1216,10 +1216,10 @@ static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 b
   // that goes from a Gram pass or a fused pass (200 or 150 KB of shared memory)
   // straight to a gathering kernel keeps its shared-memory carve-out, and the
   // gathers lose most of their L1.  Measured (us per application, overlapped /
-  // not): 1M x 750k Zipf, b = 32: 590 / 453 (its chunks 209 / 144); 190k x 150k,
-  // b = 32: 119 / 104; 600k x 500k, b = 16: 155 / 148; 2M Zipf, b = 16: 543 /
-  // 536, b = 5: 373 / 362; but 60k x 50k Zipf, b = 4 (8 MB gathered a pass):
-  // 28.9 / 30.6.
+  // not): 1M x 750k Zipf, b = 32: 476 / 406; 190k x 150k, b = 32: 78 / 71; 600k x
+  // 500k, b = 16: 143 / 109; 2M Zipf, b = 16: 626 / 484, b = 5: 331 / 319; 190k x
+  // 150k, b = 8 (42 MB gathered a pass): 24.8 / 24.8; 60k x 50k Zipf, b = 4 (8 MB):
+  // 23.9 / 25.6.
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed =
