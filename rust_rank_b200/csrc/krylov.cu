@@ -616,9 +616,9 @@ __device__ __forceinline__ bool mbar_wait_or(uint32_t addr, uint32_t parity, con
 //              store them in operand stage j mod OPS.
 // The reads of the two blocks are the floor (24 / 30 us at the sizes below); what
 // it takes beyond that is the transposers' multiply-adds and stores, and at
-// either end the fill of the ring and one read-out.  So a raw slot is given back
-// as soon as its rows are in registers, the ring is as deep as shared memory
-// allows at 4 or 2 operand stages, and the read-out reduces 64-bit sums of four
+// either end the fill of the ring and one read-out.  So the ring holds two raw
+// tiles per group, the next of which crosses while the group works on one, rows
+// past the end need no selects, and the read-out reduces 64-bit sums of four
 // limbs (2 B reductions per thread and read-out instead of 8 B, and plain adds
 // to words of its own instead of 64-bit atomics).  Measured, us per launch, without
 // these / with: 750k rows, b = 32: 98.5 / 49.6; 150k rows, b = 32: 49.2 / 21.8;
@@ -891,8 +891,6 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
       const uint4 s4 = *reinterpret_cast<const uint4*>(scl + 4 * qd);
       const int64_t left = P.rows - (r0 + 4 * qd);  // rows past the end: scale 0, so 0 whatever y is
       const uint32_t sc[4] = {left > 0 ? s4.x : 0u, left > 1 ? s4.y : 0u, left > 2 ? s4.z : 0u, left > 3 ? s4.w : 0u};
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&raw_empty[slot]);  // the rows are in registers: the next copy may come
       if (j >= T::OPS && !mbar_wait_or(smem_u32(&op_empty[s]), (uint32_t)((j / T::OPS - 1) & 1), &s_fail)) {
         give_up();
         break;
@@ -913,7 +911,13 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // stores visible to the tensor cores
       __syncwarp();
-      if (lane == 0) mbar_arrive(&op_full[s]);
+      if (lane == 0) {
+        mbar_arrive(&op_full[s]);
+        // Only now, when every value read has gone into a store: an arrival right
+        // after the reads was seen to let the next copy overtake some of them
+        // (2 wrong terms in 65,000 at 600k x 408k, b = 16).
+        mbar_arrive(&raw_empty[slot]);
+      }
     }
   }
   griddep_launch();
