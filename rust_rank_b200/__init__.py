@@ -73,6 +73,11 @@ class Context:
         """PM-basis contractions on the int8 tensor cores (True, default) or the CUDA cores (False)."""
         check(lib().rr_ctx_set_pm_tensor_cores(self.handle, 1 if enable else 0))
 
+    def set_waits(self, limit_s: float = 2.0, missing: int = 0):
+        """Limit of the device-side waits of work queued through this context; missing > 0 makes them
+        run out (checks of the error path, see rr_ctx_set_waits)."""
+        check(lib().rr_ctx_set_waits(self.handle, float(limit_s), int(missing)))
+
     def synchronize(self):
         check(lib().rr_ctx_synchronize(self.handle))
 

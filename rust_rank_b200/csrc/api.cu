@@ -183,6 +183,14 @@ int rr_ctx_set_pm_tensor_cores(rr_ctx* ctx, int32_t enable) {
   return RR_OK;
 }
 
+int rr_ctx_set_waits(rr_ctx* ctx, double limit_s, int32_t missing) {
+  if (!ctx) return fail(RR_EINVAL, "NULL context");
+  if (!(limit_s >= 1e-3 && limit_s <= 10) || missing < 0) return fail(RR_EINVAL, "bad argument");
+  ctx->wait_limit_ns = (uint64_t)(limit_s * 1e9);
+  ctx->wait_missing = missing;
+  return RR_OK;
+}
+
 int rr_ctx_synchronize(rr_ctx* ctx) {
   if (!ctx) return fail(RR_EINVAL, "ctx is NULL");
   RR_CUDA(cudaSetDevice(ctx->device));

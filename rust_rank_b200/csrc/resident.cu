@@ -22,7 +22,8 @@
 // latency; the last by the rate at which L2 serves random 64-byte rows
 // (8500 gathers per SM and pass, 4.2 TB/s in all).
 //
-// The grid barrier gives up after 2 s of %globaltimer and sets *status.
+// The grid barrier gives up after a limit (2 s by default) of %globaltimer and
+// sets *status; the CTA's other warps learn of it at their next CTA barrier.
 #include <algorithm>
 #include <mutex>
 
@@ -41,7 +42,6 @@ template <int B>
 constexpr int kResThreads = 32 * (kGatherWarps + kGramWarps<B>);
 constexpr int kMaxBatches = 512;  // row batches of one CTA, per matrix
 constexpr int64_t kResMaxDegree = 64;
-constexpr uint64_t kBarrierNs = 2000000000ull;
 constexpr size_t kResSmem = 227 * 1024 - 2048;
 
 struct ResCsr {
@@ -60,6 +60,8 @@ struct ResParams {
   unsigned long long* gram;  // [2 apps][NP], zero at launch
   unsigned int* bar;         // arrivals, zero at launch
   int* status;
+  uint64_t limit_ns;         // a barrier wait gives up after this long
+  unsigned int missing;      // arrivals the barriers expect beyond those that come (0; checks of the give-up path)
   ModP M;
   uint32_t w4, w5, w6;
 };
@@ -251,7 +253,11 @@ template <int B>
 __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P, int entriesA) {
   constexpr int NP = B * (B + 1) / 2;
   extern __shared__ __align__(16) unsigned char res_smem[];
-  __shared__ int s_stop;
+  // s_stop[p & 1]: the run ends at the CTA barrier of pass p.  Thread 0 sets it
+  // after the barrier of pass p - 1, when a Gram warp may still have to read the
+  // flag of p - 1: with one flag for both, some of the Gram warps could leave and
+  // the others wait for them in gram_bar.
+  __shared__ volatile int s_stop[2];
   uint2* const ellA = reinterpret_cast<uint2*>(res_smem + res_fixed_smem<B>());
   uint2* const ellAt = ellA + entriesA;
   uint32_t* const staging = reinterpret_cast<uint32_t*>(res_smem);
@@ -260,13 +266,13 @@ __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P
   int* const firstAt = firstA + kMaxBatches + 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const ModP M = P.M;
-  if (tid == 0) s_stop = 0;
+  if (tid < 2) s_stop[tid] = 0;
   const int nA = load_entries<B>(P.A, ellA, firstA);
   const int nAt = load_entries<B>(P.At, ellAt, firstAt);
   __syncthreads();
   if (warp < kGatherWarps) {
     int cur = P.cur0;
-    unsigned int target = 0;
+    unsigned int target = P.missing;
     for (int p = 0; p < 2 * P.apps; ++p) {
       if ((p & 1) == 0) {
         res_pass<B, false>(P.A, ellA, firstA, nA, P.X[cur], P.U, P.dr_m, nullptr, M);
@@ -289,17 +295,17 @@ __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P
           if ((spins & 255) == 255) {
             const uint64_t t = res_ns();
             if (t0 == 0) t0 = t;
-            if (*(volatile int*)P.status || t - t0 > kBarrierNs) {
+            if (*(volatile int*)P.status || t - t0 > P.limit_ns) {
               atomicExch(P.status, 1);
-              s_stop = 1;
+              s_stop[(p + 1) & 1] = 1;
               break;
             }
           }
         }
       }
       gather_bar();
-      if (*(volatile int*)&s_stop) {
-        __syncthreads();  // the Gram warps leave here too
+      if (s_stop[(p + 1) & 1]) {
+        __syncthreads();  // the barrier of pass p + 1, after which the Gram warps leave too
         break;
       }
     }
@@ -310,7 +316,7 @@ __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P
     int cur = P.cur0;
     for (int p = 0; p < 2 * P.apps; ++p) {
       __syncthreads();
-      if (*(volatile int*)&s_stop) break;
+      if (s_stop[p & 1]) break;
       unsigned long long* out = P.gram + (size_t)p * NP;
       if ((p & 1) == 0) {
         res_gram<B, false>(gram, P.A.rows, nA, P.U, P.drinv_r, M, W, part, out);
@@ -450,6 +456,8 @@ int run(rr_krylov* kr, int apps, bool* taken) {
   P.gram = kr->res_gram.ptr;
   P.bar = kr->res_bar.ptr;
   P.status = kr->d_status.ptr;
+  P.limit_ns = mat->ctx->wait_limit_ns;
+  P.missing = (unsigned int)mat->ctx->wait_missing;
   P.M = kr->M;
   P.w4 = kr->M.c32;
   P.w5 = (uint32_t)((uint64_t)P.w4 * 256 % kr->M.p);

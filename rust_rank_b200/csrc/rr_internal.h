@@ -133,6 +133,8 @@ struct rr_ctx_s {
   cudaStream_t stream = nullptr;
   int num_sms = 0;
   int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
+  uint64_t wait_limit_ns = 2000000000ull;  // device-side waits of its resident runs (rr_ctx_set_waits)
+  int wait_missing = 0;
   int pm_tensor_cores = 1;  // PM-basis contractions on the int8 tensor cores (0: CUDA cores)
 };
 
@@ -203,7 +205,7 @@ struct rr_krylov_s {
   int64_t len = 0;  // terms queued so far
   int cur = 0;      // index of the current X
   int grid_pass = 0, grid_chunk = 0, grid_lean = 0;
-  rr::DevBuf<int> d_status;  // set by a device-side wait that gave up (tcgen05 Gram pass)
+  rr::DevBuf<int> d_status;  // set by a device-side wait that gave up (resident runs, tcgen05 Gram pass)
   int64_t launches = 0;  // kernels launched by this handle
   // device-indexed sequence output: next slot (len - base) and the S pointer
   rr::DevBuf<unsigned int> d_term;

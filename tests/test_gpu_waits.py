@@ -1,0 +1,91 @@
+"""Device-side waits that run out: the kernel ends by itself, the calls that read its results
+report the time-out, and the context goes on working.  The waits are made to run out by
+expecting more arrivals than come, with a short limit; nothing faults or hangs."""
+import contextlib
+import time
+
+import numpy as np
+import pytest
+
+import oracle
+import rust_rank_b200 as rr
+from rust_rank_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+P = 2013265921
+ETIMEOUT = 5
+
+
+@pytest.fixture(scope="module")
+def module_ctx():
+    return rr.Context(0)
+
+
+@pytest.fixture
+def own_ctx(module_ctx):
+    yield module_ctx
+    module_ctx.set_waits()
+
+
+def _problem(m, b, seed=3):
+    rowptr, col, val, m, n = synth.incidence_fast(m, int(0.8 * m), 3, 10, 2, P, seed)
+    dr, dc = synth.preconditioners(m, n, P, seed + 1)
+    return (rowptr, col, val, m, n), dr, dc, synth.random_vectors(b, n, P, seed + 2)
+
+
+@contextlib.contextmanager
+def _stream(ctx, prob):
+    mat, dr, dc, V = prob
+    dm = rr.CsrMatrix.from_arrays(*mat).to_device(P, ctx)
+    ks = rr.KrylovStream(dm, V, dr, dc, 0)
+    yield ks
+    ks.close()
+    dm.close()
+
+
+def _timed_out(call, *args):
+    try:
+        call(*args)
+    except rr.RRError as e:
+        assert e.status == ETIMEOUT
+    else:
+        pytest.fail("no error")
+
+
+def _works(ctx, prob):
+    """A new handle on the same context computes the oracle's sequence."""
+    mat, dr, dc, V = prob
+    b = V.shape[0]
+    seq = np.zeros((b * (b + 1) // 2, 17), np.uint32)
+    with _stream(ctx, prob) as ks:
+        ks.step_device(8)
+        ks.fetch(0, 17, seq)
+        ref, _, cv = oracle.krylov(*mat, P, dr, dc, V, 0, 16)
+        assert np.array_equal(seq, ref[:, :17])
+        assert np.array_equal(ks.get_curv(), cv)
+
+
+@pytest.mark.parametrize("m,b", [(12, 1), (700, 4), (700, 8), (700, 16), (20000, 8), (20000, 16)])
+def test_grid_barrier_of_a_resident_run(own_ctx, m, b):
+    """Every warp of every CTA leaves the run, whatever it was doing when the wait ran out."""
+    prob = _problem(m, b)
+    seq = np.zeros((b * (b + 1) // 2, 32), np.uint32)
+    with _stream(own_ctx, prob) as ks:
+        own_ctx.set_waits(0.02, 1)
+        t0 = time.perf_counter()
+        for apps in (4, 9, 30):
+            ks.step_device(apps)
+        own_ctx.synchronize()
+        assert time.perf_counter() - t0 < 1.5
+        _timed_out(ks.fetch, 0, 9, seq)
+        own_ctx.set_waits()
+        ks.step_device(5)
+        _timed_out(ks.fetch, 0, 9, seq)  # the handle's state is lost
+    _works(own_ctx, prob)
+
+
+def test_arguments(own_ctx):
+    for limit, missing in ((0.0, 0), (11.0, 0), (float("nan"), 0), (1.0, -1)):
+        with pytest.raises(rr.RRError):
+            own_ctx.set_waits(limit, missing)
