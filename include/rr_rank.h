@@ -130,7 +130,9 @@ int rr_krylov_step_device(rr_krylov* kr, int64_t n_apps);
 int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int64_t seq_stride);
 /* Current sequence length (terms computed so far, including queued work). */
 int rr_krylov_length(const rr_krylov* kr, int64_t* len);
-/* The current block w_k as curv[b][n] (host, original column order). */
+/* The current block w_k as curv[b][n] (host, original column order).
+ * RR_ETIMEOUT when a device-side wait of the handle's kernels had given up:
+ * curv then holds nothing meaningful. */
 int rr_krylov_get_curv(rr_krylov* kr, uint32_t* curv);
 /* Algorithmic bytes of one application of B (both SpMMs: CSR read once,
  * dense blocks read and written once), for bandwidth reporting. */

@@ -171,6 +171,7 @@ int rr_ctx_destroy(rr_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   cudaStreamDestroy(ctx->stream);
   rr::staging_destroy(ctx->staging);
+  if (ctx->curv_status) cudaFreeHost(ctx->curv_status);
   delete ctx;
   return RR_OK;
 }
@@ -540,12 +541,19 @@ int rr_krylov_length(const rr_krylov* kr, int64_t* len) {
 
 int rr_krylov_get_curv(rr_krylov* kr, uint32_t* curv) {
   if (!kr || !curv) return fail(RR_EINVAL, "NULL argument");
-  RR_CUDA(cudaSetDevice(kr->mat->ctx->device));
+  rr_ctx* ctx = kr->mat->ctx;
+  RR_CUDA(cudaSetDevice(ctx->device));
+  // the gathering kernel also writes the handle's status, into a pinned word of
+  // the context: no second copy
+  std::lock_guard<std::mutex> lk(ctx->curv_mu);
+  if (!ctx->curv_status) RR_CUDA(cudaHostAlloc((void**)&ctx->curv_status, sizeof(int), cudaHostAllocMapped));
   DevBuf<uint32_t> out;
-  RR_TRY(out.alloc_async((size_t)kr->b * kr->mat->n, kr->mat->ctx->stream));
-  RR_TRY(krylov_launch_get_curv(kr, out.ptr));
-  RR_TRY(rr::download_host(kr->mat->ctx, {{curv, out.ptr, out.bytes()}}, kr->mat->ctx->stream));
-  RR_CUDA(cudaStreamSynchronize(kr->mat->ctx->stream));
+  RR_TRY(out.alloc_async((size_t)kr->b * kr->mat->n, ctx->stream));
+  RR_TRY(krylov_launch_get_curv(kr, out.ptr, ctx->curv_status));
+  RR_TRY(rr::download_host(ctx, {{curv, out.ptr, out.bytes()}}, ctx->stream));
+  RR_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (*(volatile int*)ctx->curv_status)
+    return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the block is not valid");
   return RR_OK;
 }
 

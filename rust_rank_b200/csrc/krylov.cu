@@ -1124,10 +1124,11 @@ __global__ void scatter_block_kernel(const uint32_t* __restrict__ V, const int32
   }
 }
 
-// curv[l][colperm[c']] = x[c'][l] * dcinv[c']
+// curv[l][colperm[c']] = x[c'][l] * dcinv[c'], and the status beside it
 __global__ void gather_curv_kernel(const uint32_t* __restrict__ x, const uint32_t* __restrict__ dcinv,
                                    const int32_t* __restrict__ colperm, int64_t n, int b, int B, ModP M,
-                                   uint32_t* __restrict__ curv) {
+                                   uint32_t* __restrict__ curv, const int* status, int* status_out) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status_out = *status;
   const int64_t total = n * b;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = i / b;
@@ -1582,13 +1583,14 @@ int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev) {
   return RR_OK;
 }
 
-int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out) {
+int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out, int* status_out) {
   const int64_t n = kr->mat->n;
   const int threads = 256;
   const int64_t want = (n * kr->b + threads - 1) / threads;
   const int blocks = (int)std::min<int64_t>(want, 65535);
   gather_curv_kernel<<<std::max(blocks, 1), threads, 0, kr->mat->ctx->stream>>>(
-      kr->X[kr->cur].ptr, kr->dcinv.ptr, kr->mat->d_colperm.ptr, n, kr->b, kr->B, kr->M, d_out);
+      kr->X[kr->cur].ptr, kr->dcinv.ptr, kr->mat->d_colperm.ptr, n, kr->b, kr->B, kr->M, d_out, kr->d_status.ptr,
+      status_out);
   RR_CUDA(cudaGetLastError());
   return RR_OK;
 }

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -135,6 +136,8 @@ struct rr_ctx_s {
   int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
   uint64_t wait_limit_ns = 2000000000ull;  // device-side waits of its resident runs (rr_ctx_set_waits)
   int wait_missing = 0;
+  std::mutex curv_mu;
+  int* curv_status = nullptr;  // pinned: the status a block was read with (rr_krylov_get_curv)
   int pm_tensor_cores = 1;  // PM-basis contractions on the int8 tensor cores (0: CUDA cores)
 };
 
@@ -231,7 +234,7 @@ namespace rr {
 int krylov_launch_init(rr_krylov* kr, const uint32_t* d_w, bool emit_s0);
 int krylov_reserve(rr_krylov* kr, int64_t terms);
 int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev);
-int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out);
+int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out, int* status_out);  // status_out: kr->d_status with the block
 // Runs of applications in one launch with the CSR in shared memory
 // (resident.cu): resident_prepare sets kr->res_grid where the matrix fits, and
 // resident_run then takes 1 <= apps <= kResMaxApps applications at once, or

@@ -85,6 +85,26 @@ def test_grid_barrier_of_a_resident_run(own_ctx, m, b):
     _works(own_ctx, prob)
 
 
+@pytest.mark.parametrize("m,b", [(700, 8), (700, 16), (90000, 16)])
+def test_block_of_a_run_that_gave_up(own_ctx, m, b):
+    """A block that a given-up run left half advanced is not returned as valid: neither by get_curv nor
+    by next(), which at width 16 is a resident run of its own."""
+    prob = _problem(m, b)
+    with _stream(own_ctx, prob) as ks:
+        own_ctx.set_waits(0.02, 1)
+        ks.step_device(4)
+        _timed_out(ks.get_curv)
+        own_ctx.set_waits()
+        _timed_out(ks.get_curv)
+        _timed_out(ks.next)
+    if b == 16:
+        with _stream(own_ctx, prob) as ks:
+            own_ctx.set_waits(0.02, 1)
+            _timed_out(ks.next)
+            own_ctx.set_waits()
+    _works(own_ctx, prob)
+
+
 def test_arguments(own_ctx):
     for limit, missing in ((0.0, 0), (11.0, 0), (float("nan"), 0), (1.0, -1)):
         with pytest.raises(rr.RRError):
