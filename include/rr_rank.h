@@ -296,12 +296,15 @@ int rr_server_submit(rr_server* server, int64_t m, int64_t n, const int64_t* row
                      const uint32_t* val, const uint32_t* row_precond, const uint32_t* col_precond, const uint32_t* V,
                      uint64_t* id);
 /* Waits for request id (timeout_s < 0: no limit; RR_ETIMEOUT when it runs out);
- * *rank as rr_rank, *latency_ms = submit to completion (may be NULL). */
+ * *rank as rr_rank, *latency_ms = submit to completion (may be NULL).  A request
+ * that failed returns its own status, RR_ECUDA where a device-side wait gave up. */
 int rr_server_wait(rr_server* server, uint64_t id, double timeout_s, int64_t* rank, double* latency_ms);
 /* Requests submitted and completed, latency percentiles of the completed
  * ones and completions per second between the first submit and the last completion. */
 int rr_server_stats(rr_server* server, int64_t* submitted, int64_t* completed, double* p50_ms, double* p99_ms,
                     double* ranks_per_s);
+/* rr_ctx_set_waits for the requests of one lane (0 .. lanes - 1). */
+int rr_server_set_waits(rr_server* server, int32_t lane, double limit_s, int32_t missing);
 int rr_server_destroy(rr_server* server);
 
 /* ---------------------------------------------------------------- several GPUs */

@@ -574,6 +574,10 @@ class Server:
         return {"submitted": a.value, "completed": b.value, "p50_ms": p50.value, "p99_ms": p99.value,
                 "ranks_per_s": rps.value}
 
+    def set_waits(self, lane: int, limit_s: float = 2.0, missing: int = 0):
+        """:meth:`Context.set_waits` for the requests of one lane."""
+        check(lib().rr_server_set_waits(self.handle, int(lane), float(limit_s), int(missing)))
+
     def close(self):
         if getattr(self, "handle", None):
             lib().rr_server_destroy(self.handle)

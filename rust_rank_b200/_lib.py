@@ -75,6 +75,7 @@ SIGNATURES = {
     "rr_server_wait": (C.c_int, [_vp, C.c_uint64, C.c_double, _pi64, C.POINTER(C.c_double)]),
     "rr_server_stats": (C.c_int, [_vp, _pi64, _pi64, C.POINTER(C.c_double), C.POINTER(C.c_double),
                                   C.POINTER(C.c_double)]),
+    "rr_server_set_waits": (C.c_int, [_vp, _i32, C.c_double, _i32]),
     "rr_server_destroy": (C.c_int, [_vp]),
     "rr_footprint": (C.c_int, [_i64, _i64, _i64, _i32, C.POINTER(C.c_uint64)]),
     "rr_place_by_footprint": (C.c_int, [_i32, _vp, _i32, _vp, _vp, _vp]),

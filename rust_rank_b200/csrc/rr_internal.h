@@ -134,8 +134,8 @@ struct rr_ctx_s {
   cudaStream_t stream = nullptr;
   int num_sms = 0;
   int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
-  uint64_t wait_limit_ns = 2000000000ull;  // device-side waits of its resident runs (rr_ctx_set_waits)
-  int wait_missing = 0;
+  std::atomic<uint64_t> wait_limit_ns{2000000000ull};  // device-side waits of its resident runs (rr_ctx_set_waits)
+  std::atomic<int> wait_missing{0};
   std::mutex curv_mu;
   int* curv_status = nullptr;  // pinned: the status a block was read with (rr_krylov_get_curv)
   int pm_tensor_cores = 1;  // PM-basis contractions on the int8 tensor cores (0: CUDA cores)

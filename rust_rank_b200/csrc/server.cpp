@@ -190,28 +190,41 @@ struct rr_server_s {
   }
 
   // Worker: sequences -> generators (in lockstep) -> ranks, on the worker's
-  // own context, for requests of equal sequence length.
-  int solve(std::vector<Request*>& rs, rr_ctx* wctx) {
-    const int b = cfg.b, np = b * (b + 1) / 2, cnt = (int)rs.size();
+  // own context, for requests of equal generator order.  A request whose device-side
+  // waits gave up fails (RR_ECUDA: RR_ETIMEOUT from rr_server_wait means a request
+  // that is not finished) and is left out.
+  int solve(const std::vector<Request*>& all, rr_ctx* wctx) {
+    const int b = cfg.b, np = b * (b + 1) / 2;
     // one order d for the batch; the generator reads the first d + 1 terms
-    const int64_t d = rs[0]->order, L = d + 1;
+    const int64_t d = all[0]->order, L = d + 1;
     RR_CUDA(cudaSetDevice(device));
     // every chunk's event has completed (the scheduler saw them), so the
-    // sequences are final in device memory
+    // sequences are final in device memory, with the status of their waits
+    cudaStream_t st = (cudaStream_t)rr_ctx_stream(wctx);
     std::vector<uint32_t> raw((size_t)L * np);
-    std::vector<std::vector<uint32_t>> seq(cnt);
-    for (int z = 0; z < cnt; ++z) {
-      RR_CUDA(cudaMemcpyAsync(raw.data(), rs[z]->kr->S.ptr, raw.size() * 4, cudaMemcpyDeviceToHost,
-                              (cudaStream_t)rr_ctx_stream(wctx)));
-      RR_CUDA(cudaStreamSynchronize((cudaStream_t)rr_ctx_stream(wctx)));
-      seq[z].resize((size_t)np * L);
+    std::vector<Request*> rs;  // the requests whose sequences are valid
+    std::vector<std::vector<uint32_t>> seq;
+    for (Request* r : all) {
+      int dstat = 0;
+      RR_CUDA(cudaMemcpyAsync(&dstat, r->kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+      RR_CUDA(cudaMemcpyAsync(raw.data(), r->kr->S.ptr, raw.size() * 4, cudaMemcpyDeviceToHost, st));
+      RR_CUDA(cudaStreamSynchronize(st));
+      rr_krylov_destroy(r->kr);
+      r->kr = nullptr;
+      rr_matrix_destroy(r->mat);
+      r->mat = nullptr;
+      if (dstat) {
+        r->status = RR_ECUDA;
+        r->error = "a device-side wait of the Krylov kernels gave up; the terms are not valid";
+        continue;
+      }
+      rs.push_back(r);
+      seq.emplace_back((size_t)np * L);
       for (int64_t t = 0; t < L; ++t)
-        for (int q = 0; q < np; ++q) seq[z][(size_t)q * L + t] = raw[(size_t)t * np + q];
-      rr_krylov_destroy(rs[z]->kr);
-      rs[z]->kr = nullptr;
-      rr_matrix_destroy(rs[z]->mat);
-      rs[z]->mat = nullptr;
+        for (int q = 0; q < np; ++q) seq.back()[(size_t)q * L + t] = raw[(size_t)t * np + q];
     }
+    const int cnt = (int)rs.size();
+    if (cnt == 0) return RR_OK;
     std::vector<std::vector<uint32_t>> M(cnt);
     std::vector<std::vector<int64_t>> delta(cnt);
     std::vector<const uint32_t*> sp(cnt);
@@ -303,6 +316,7 @@ struct rr_server_s {
       if (rc == RR_OK) {
         rc = loading ? load(*batch[0]) : solve(batch, wctx);
         if (rc != RR_OK) err = rr_last_error();
+        if (rc == RR_ETIMEOUT) rc = RR_ECUDA;  // of the generator's waits: as for the sequence's
       }
       std::lock_guard<std::mutex> lk(mu);
       for (Request* r : batch) {
@@ -316,7 +330,7 @@ struct rr_server_s {
           cv_sched.notify_one();
         } else {
           release(*r);
-          finish_locked(*r, RR_OK);
+          finish_locked(*r, r->status);
         }
       }
     }
@@ -511,6 +525,11 @@ int rr_server_stats(rr_server* s, int64_t* submitted, int64_t* completed, double
     *ranks_per_s = (s->completed > 0 && span > 0) ? (double)s->completed / span : 0.0;
   }
   return RR_OK;
+}
+
+int rr_server_set_waits(rr_server* s, int32_t lane, double limit_s, int32_t missing) {
+  if (!s || lane < 0 || lane >= (int)s->lanes.size()) return fail(RR_EINVAL, "bad argument");
+  return rr_ctx_set_waits(s->lanes[lane], limit_s, missing);
 }
 
 int rr_server_destroy(rr_server* s) {

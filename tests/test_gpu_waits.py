@@ -44,6 +44,13 @@ def _stream(ctx, prob):
     dm.close()
 
 
+@contextlib.contextmanager
+def rr_server(b):
+    srv = rr.Server(b, P, lanes=2, workers=2)
+    yield srv
+    srv.close()
+
+
 def _timed_out(call, *args):
     try:
         call(*args)
@@ -103,6 +110,25 @@ def test_block_of_a_run_that_gave_up(own_ctx, m, b):
             _timed_out(ks.next)
             own_ctx.set_waits()
     _works(own_ctx, prob)
+
+
+@pytest.mark.parametrize("b", [8, 16])
+def test_served_request_whose_run_gave_up(b):
+    """The request fails instead of returning a rank of terms that were never computed; the one solved
+    together with it, and later ones of the same lane, return theirs."""
+    (rowptr, col, val, m, n), dr, dc, V = _problem(700, b)
+    with rr_server(b) as srv:
+        want = rr.block_wiedemann_rank(rr.CsrMatrix.from_arrays(rowptr, col, val, m, n), b, P, dr, dc, V)
+        srv.set_waits(0, 0.02, 1)
+        ids = [srv.submit(rowptr, col, val, m, n, dr, dc, V) for _ in range(2)]  # one per lane
+        with pytest.raises(rr.RRError, match="gave up") as e:
+            srv.result(ids[0])
+        assert e.value.status != ETIMEOUT  # which would say that it is not finished
+        assert srv.result(ids[1])[0] == want
+        srv.set_waits(0)
+        ids = [srv.submit(rowptr, col, val, m, n, dr, dc, V) for _ in range(4)]
+        assert [srv.result(i)[0] for i in ids] == [want] * 4
+        assert srv.stats()["completed"] == 6
 
 
 def test_arguments(own_ctx):
