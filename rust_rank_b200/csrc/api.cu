@@ -436,24 +436,28 @@ int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int6
   cudaStream_t st = kr->mat->ctx->stream;
   const uint32_t* terms = kr->S.ptr + (size_t)(from - kr->base) * np;
   int dstat = 0;
-  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   std::vector<uint32_t> tmp;
-  if (cnt >= kTransposeTerms) {  // pair-major on the device, then one strided copy
-    DevBuf<uint32_t> pairs;
+  DevBuf<uint32_t> pairs;
+  const bool transpose = cnt >= kTransposeTerms;  // pair-major on the device, then one strided copy
+  if (transpose) {
     RR_TRY(pairs.alloc_async((size_t)cnt * np, st));
     RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr));
-    RR_CUDA(cudaMemcpy2DAsync(seq + from, (size_t)seq_stride * 4, pairs.ptr, (size_t)cnt * 4, (size_t)cnt * 4, np,
-                              cudaMemcpyDeviceToHost, st));
-    RR_CUDA(cudaStreamSynchronize(st));
   } else {
     tmp.resize((size_t)cnt * np);
     RR_CUDA(cudaMemcpyAsync(tmp.data(), terms, tmp.size() * 4, cudaMemcpyDeviceToHost, st));
-    RR_CUDA(cudaStreamSynchronize(st));
   }
+  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  RR_CUDA(cudaStreamSynchronize(st));
+  // seq is written only once the terms are known to be valid
   if (dstat) return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the terms are not valid");
-  if (!tmp.empty())
-    for (int64_t t = 0; t < cnt; ++t)
-      for (int q = 0; q < np; ++q) seq[(size_t)q * seq_stride + from + t] = tmp[(size_t)t * np + q];
+  if (transpose) {
+    RR_CUDA(cudaMemcpy2DAsync(seq + from, (size_t)seq_stride * 4, pairs.ptr, (size_t)cnt * 4, (size_t)cnt * 4, np,
+                              cudaMemcpyDeviceToHost, st));
+    RR_CUDA(cudaStreamSynchronize(st));
+    return RR_OK;
+  }
+  for (int64_t t = 0; t < cnt; ++t)
+    for (int q = 0; q < np; ++q) seq[(size_t)q * seq_stride + from + t] = tmp[(size_t)t * np + q];
   return RR_OK;
 }
 

@@ -112,6 +112,23 @@ def test_block_of_a_run_that_gave_up(own_ctx, m, b):
     _works(own_ctx, prob)
 
 
+@pytest.mark.parametrize("terms", [9, 1023, 1024, 5001])
+def test_terms_of_a_run_that_gave_up(own_ctx, terms):
+    """The caller's array keeps what it held, whatever the length of the fetch."""
+    b = 8
+    prob = _problem(700, b)
+    with _stream(own_ctx, prob) as ks:
+        ks.step_device(4)
+        seq = np.full((b * (b + 1) // 2, terms + 2), 7, np.uint32)
+        ks.fetch(0, 9, seq)
+        head = seq[:, :9].copy()
+        own_ctx.set_waits(0.02, 1)
+        ks.step_device(terms // 2)
+        _timed_out(ks.fetch, 0, terms, seq)
+        own_ctx.set_waits()
+        assert np.array_equal(seq[:, :9], head) and (seq[:, 9:] == 7).all()
+
+
 @pytest.mark.parametrize("b", [8, 16])
 def test_served_request_whose_run_gave_up(b):
     """The request fails instead of returning a rank of terms that were never computed; the one solved
