@@ -58,12 +58,13 @@ int rr_ctx_synchronize(rr_ctx* ctx);
  * generator is the same bit for bit; this selects the path, e.g. to compare
  * them.  No counterpart in the reference. */
 int rr_ctx_set_pm_tensor_cores(rr_ctx* ctx, int32_t enable);
-/* Device-side waits of the resident Krylov runs queued through ctx from now on
- * (one launch per run, the matrix in shared memory): each gives up after
- * limit_s seconds (2 by default, 0.001 to 10).  missing > 0 makes them run
- * out, for checks of the error path: the grid barriers then expect that many
- * arrivals more than there are.  The calls that read the run's results return
- * RR_ETIMEOUT, and go on doing so for that handle; the context stays usable. */
+/* Device-side waits of the resident Krylov runs (one launch per run, the matrix
+ * in shared memory) and of the PM-basis leaf blocks queued through ctx from now
+ * on: each gives up after limit_s seconds (2 by default, 0.001 to 10).  missing >
+ * 0 makes them run out, for checks of the error path: the grid barriers of a run
+ * then expect that many arrivals, the first hand-off of a leaf block that many
+ * words more than come.  The calls that return the results give RR_ETIMEOUT, and
+ * go on doing so for that Krylov handle; the context stays usable. */
 int rr_ctx_set_waits(rr_ctx* ctx, double limit_s, int32_t missing);
 
 /* ---------------------------------------------------------------- checks */

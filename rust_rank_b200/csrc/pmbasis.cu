@@ -1140,6 +1140,8 @@ struct Pm {
   int64_t cs = 0;                      // residual coefficient stride of the leaves kernel (words)
   int fold4 = 0;
   int64_t direct = 0;                  // levels up to this half length take direct products
+  uint64_t wait_ns = 0;                // of the leaf blocks (rr_ctx_set_waits)
+  int wait_missing = 0;
   bool mma = false;                    // leaf blocks on clusters and tensor cores (pmleaf.cu)
   // per recursion depth: MM, GG, MMM ([nb] each)
   std::vector<std::unique_ptr<DevBuf<uint32_t>>> bufs;
@@ -1316,7 +1318,7 @@ int level_product(Pm& P, MatView A, int64_t la, bool a_is_mm, MatView B, int k, 
 int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
   if (P.mma)
     return leaf_block_launch(LeafBlock{G.p, G.rs, G.cs, G.bs, P.m, P.n, nleaves, P.delta.ptr, Mout.p, Mout.rs, Mout.cs,
-                                       Mout.bs, P.M, P.status.ptr, 0, 0, 0},
+                                       Mout.bs, P.M, P.status.ptr, P.wait_ns, P.wait_missing, 0, 0, 0},
                              P.nb, P.s);
   LeafParams L;
   L.G = G.p;
@@ -1439,6 +1441,8 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   P.p = p;
   P.M = make_modp(p);
   size_t leaves_smem = 0;
+  P.wait_ns = ctx->wait_limit_ns;
+  P.wait_missing = ctx->wait_missing;
   P.mma = ctx->pm_tensor_cores;
   P.K = P.mma ? (int)std::min<int64_t>(d, leaf_block_max(P.m)) : pick_block_leaves(P.m, P.n, d, &leaves_smem);
   P.cs = leaf_coeff_stride(P.m, P.n);

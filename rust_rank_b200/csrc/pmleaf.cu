@@ -50,8 +50,9 @@
 // Hand-offs: a finished transform goes from the leaf CTA's registers to the
 // other CTAs' shared memory with st.async, and coefficient 1 comes back the
 // same way; each message completes bytes on an mbarrier of its own (one per
-// leaf), so no side needs a fence.  Every wait gives up after 2 s and sets
-// *status = 3; all CTAs meet in a cluster barrier before any of them exits.
+// leaf), so no side needs a fence.  Every wait gives up after a limit (2 s by
+// default) and sets *status = 3, after which the blocks that follow do not wait
+// at all; all CTAs meet in a cluster barrier before any of them exits.
 // Measured (us per leaf, blocks of the largest K on one B200; before: one CTA
 // per generator with 8 elimination and 8 update warps, then a second kernel for
 // the block's basis -- 13.1 at n = 16 and 9.3 at n = 8, and the CUDA-core
@@ -74,7 +75,7 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 8;      // portable cluster size
 constexpr int kMaxLeaves = 64;
-constexpr uint64_t kWaitNs = 2000000000ull;
+constexpr uint64_t kLandNs = 1000000ull;  // in which the messages in flight have long landed
 
 // Words of the shared-memory regions; RL = rows per lane (m <= 32 RL), CPW =
 // columns per elimination warp, EW = elimination warps (n <= CPW EW).
@@ -171,18 +172,18 @@ __device__ __forceinline__ bool bar_try(uint32_t a) {
       : "memory");
   return done != 0;
 }
-// Waits for the message of mbarrier q; gives up after kWaitNs or once another
+// Waits for the message of mbarrier q; gives up after wait_ns or once another
 // wait of this CTA did.
-__device__ __forceinline__ bool bar_wait(uint32_t* sm, int q, volatile int* abort, int* status) {
+__device__ __forceinline__ bool bar_wait(uint32_t* sm, int q, volatile int* abort, const LeafBlock& P) {
   const uint32_t a = smem_addr(sm + 2 * q);
   if (bar_try(a)) return true;
   const uint64_t t0 = now_ns();
   for (;;) {
     if (bar_try(a)) return true;
     if (*abort) return false;
-    if (now_ns() - t0 > kWaitNs) {
+    if (now_ns() - t0 > P.wait_ns) {
       *abort = 1;
-      atomicExch(status, 3);
+      atomicExch(P.status, 3);
       return false;
     }
   }
@@ -704,14 +705,14 @@ __device__ void leaf_help(const LeafBlock& P, uint32_t* sm, volatile int* s_abor
       if (sender) X.slot[(peer - 1) * MP + i] = 255;
     }
     if (warp == kWaitWarp && leaf > 0 && leaf + 1 < K) {
-      const bool ok = bar_wait(sm, leaf - 1, s_abort, P.status);
+      const bool ok = bar_wait(sm, leaf - 1, s_abort, P);
       if (!__all_sync(0xffffffffu, ok) && lane == 0) *s_ok = 0;
     }
     if (S::kRinged && leaf >= S::slots(K) && sender) {
       // the ring slot this transform goes to (handed back long ago)
       const uint64_t t0 = now_ns();
       while (ld_acquire(sm + S::OFF_USED + peer) < (uint32_t)(leaf - S::slots(K) + 1)) {
-        if (*s_abort || now_ns() - t0 > kWaitNs) {
+        if (*s_abort || now_ns() - t0 > P.wait_ns) {
           *s_abort = 1;
           atomicExch(P.status, 3);
           *s_ok = 0;
@@ -830,7 +831,7 @@ __device__ bool receive_transform(const LeafBlock& P, uint32_t* sm, int leaf, in
                                   unsigned long long& mask) {
   using S = LeafShape<RL, CPW, EW>;
   constexpr int MP = S::MP, KW = S::KW;
-  const bool ok = bar_wait(sm, leaf, s_abort, P.status);
+  const bool ok = bar_wait(sm, leaf, s_abort, P);
   __syncwarp();
   const uint32_t* L = sm + S::OFF_RING + (leaf % S::slots(P.K)) * S::LW;
   uint32_t* Tp = sm + S::OFF_T + (leaf & 1) * S::TW;
@@ -972,7 +973,7 @@ __device__ void update_cta(const LeafBlock& P, uint32_t* sm, int rank, volatile 
   }
   if (!BASIS) return;
   // normalise by the row scales
-  const bool ok = bar_wait(sm, K, s_abort, P.status);
+  const bool ok = bar_wait(sm, K, s_abort, P);
   __syncwarp();
   if (!__syncthreads_and(ok)) return;
   uint32_t* inv = sm + S::OFF_T;
@@ -1002,13 +1003,13 @@ __global__ void __launch_bounds__(kThreads, 1) pm_leaf_block_kernel(LeafBlock P)
   P.Mout += (int64_t)z * P.out_bs;
   const int m = P.m, n = P.n, K = P.K;
   if (tid == 0) {
-    s_abort = 0;
+    s_abort = *(volatile int*)P.status == 3;  // an earlier block gave up: its basis is not there
     s_ok = 1;
   }
   if (tid < 8) sm[S::OFF_USED + tid] = 0;
   // one mbarrier per message: transforms (and the row scales) in, coefficient 1 back
   if (tid <= K)
-    bar_arm(sm, tid, rank == 0 ? (uint32_t)(4 * m * n) : tid == K ? 4u * S::MP : (uint32_t)(4 * ((n + 2) * S::MP + 2)));
+    bar_arm(sm, tid, (rank != 0 && tid == 0 ? 4u * (uint32_t)P.missing : 0u) + (rank == 0 ? (uint32_t)(4 * m * n) : tid == K ? 4u * S::MP : (uint32_t)(4 * ((n + 2) * S::MP + 2))));
   if (rank == 0) {
     for (int e = S::OFF_R1 + tid; e < S::OFF_FB; e += kThreads) sm[e] = 0;
     __syncthreads();
@@ -1054,14 +1055,13 @@ __global__ void __launch_bounds__(kThreads, 1) pm_leaf_block_kernel(LeafBlock P)
   }
   __syncwarp();
   // No CTA leaves while another may still write into its shared memory.  Every
-  // message has been waited for, unless a wait gave up; then the messages in
-  // flight get 10 ms to land.
+  // message has been waited for, unless a wait of this CTA gave up: then those
+  // still in flight, which all have been sent by now, get time to land.
+  cluster_sync();
   if (*(volatile int*)&s_abort) {
     const uint64_t t0 = now_ns();
-    while (now_ns() - t0 < 10000000ull) __nanosleep(1000);
-    __syncwarp();
+    while (now_ns() - t0 < kLandNs) __nanosleep(1000);
   }
-  cluster_sync();
 }
 
 template <int RL, int CPW, int EW>

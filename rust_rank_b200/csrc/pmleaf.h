@@ -16,6 +16,8 @@ struct LeafBlock {
   int64_t out_rs, out_cs, out_bs;
   ModP M;
   int* status;            // 2: a zero row scale; 3: a wait gave up
+  uint64_t wait_ns;       // a wait gives up after this long
+  int missing;            // words the first hand-off expects beyond those that come (0; checks of the give-up path)
   // set by leaf_block_launch
   int nres, nbas;         // residual and basis CTAs of a cluster
   uint32_t two16;         // 2^16

@@ -148,6 +148,22 @@ def test_served_request_whose_run_gave_up(b):
         assert srv.stats()["completed"] == 6
 
 
+@pytest.mark.parametrize("b,d", [(1, 1), (2, 2), (4, 64), (8, 256), (16, 4), (16, 256), (32, 16), (32, 128)])
+def test_hand_offs_of_leaf_blocks(own_ctx, b, d):
+    """Every CTA of the cluster ends, the blocks after the first do not wait again, and the context's
+    next generator is the oracle's."""
+    rng = np.random.default_rng(b + d)
+    seqs = [rng.integers(0, P, size=(b * (b + 1) // 2, d + 1)).astype(np.uint32) for _ in range(2)]
+    own_ctx.set_waits(0.1, 1)
+    t0 = time.perf_counter()
+    _timed_out(rr.PM_Basis_batch, seqs, d, P, own_ctx)
+    assert time.perf_counter() - t0 < 1.0
+    own_ctx.set_waits()
+    M, delta = rr.PM_Basis(seqs[0], d, P, own_ctx)
+    Mo, do = oracle.pm_basis(seqs[0], b, d, P)
+    assert np.array_equal(M, Mo.astype(np.uint32)) and np.array_equal(delta, do)
+
+
 def test_arguments(own_ctx):
     for limit, missing in ((0.0, 0), (11.0, 0), (float("nan"), 0), (1.0, -1)):
         with pytest.raises(rr.RRError):
