@@ -395,7 +395,7 @@ static int queue_apps(rr_krylov* kr, int64_t n_apps) {
   int64_t i = 0;
   if (kr->res_grid > 0 && n_apps >= resident_min_run(kr)) {
     for (bool taken = true; taken && i < n_apps;) {
-      const int k = (int)std::min<int64_t>(kResMaxApps, n_apps - i);
+      const int k = (int)std::min<int64_t>(kr->res_apps, n_apps - i);
       RR_TRY(resident_run(kr, k, &taken));
       if (taken) i += k;
     }

@@ -67,7 +67,7 @@ struct rr_fleet_s {
   std::map<uint64_t, Placed> placed;
   std::vector<uint64_t> outstanding;  // bytes of submitted, not yet waited-for requests per shard
   uint64_t next_id = 1;
-  int b = 0;
+  int b = 0, run_apps = 0;
 };
 
 extern "C" {
@@ -80,7 +80,7 @@ int rr_place_by_footprint(int32_t nitems, const uint64_t* footprint, int32_t nde
 
 int rr_footprint(int64_t m, int64_t n, int64_t nnz, int32_t b, uint64_t* bytes) {
   if (!bytes || m < 1 || n < 1 || nnz < 0 || b < 1 || b > 32) return fail(RR_EINVAL, "bad argument");
-  *bytes = footprint_of(m, n, nnz, b, max_nlen_for(m, n, b));
+  *bytes = footprint_of(m, n, nnz, b, max_nlen_for(m, n, b), kResMaxApps);
   return RR_OK;
 }
 
@@ -100,6 +100,9 @@ int rr_fleet_create(const int32_t* devices, int32_t ndev, const rr_server_config
     f->shards.push_back(s);
     f->outstanding.push_back(0);
   }
+  ServerSnapshot snap;
+  server_snapshot(f->shards[0], &snap);
+  f->run_apps = snap.run_apps;
   *out = f.release();
   return RR_OK;
 }
@@ -108,7 +111,7 @@ int rr_fleet_submit(rr_fleet* f, int64_t m, int64_t n, const int64_t* rowptr, co
                     const uint32_t* row_precond, const uint32_t* col_precond, const uint32_t* V, uint64_t* id) {
   if (!f || !rowptr || !id) return fail(RR_EINVAL, "NULL argument");
   if (m < 1 || n < 1) return fail(RR_EINVAL, "bad shape %lld x %lld", (long long)m, (long long)n);
-  const uint64_t fp = footprint_of(m, n, rowptr[m], f->b, max_nlen_for(m, n, f->b));
+  const uint64_t fp = footprint_of(m, n, rowptr[m], f->b, max_nlen_for(m, n, f->b), f->run_apps);
   int shard = 0;
   {
     std::lock_guard<std::mutex> lk(f->mu);
@@ -216,7 +219,7 @@ int rr_batch_ranks_multi(const int32_t* devices, int32_t ndev, int32_t nmat, con
   std::vector<uint64_t> fp(nmat), room(ndev);
   for (int i = 0; i < nmat; ++i) {
     if (m[i] < 1 || n[i] < 1 || !rowptr[i]) return fail(RR_EINVAL, "matrix %d: bad shape or NULL rowptr", i);
-    fp[i] = footprint_of(m[i], n[i], rowptr[i][m[i]], b, max_nlen_for(m[i], n[i], b));
+    fp[i] = footprint_of(m[i], n[i], rowptr[i][m[i]], b, max_nlen_for(m[i], n[i], b), 0);  // batches have no resident runs
   }
   int dev0 = 0;
   RR_CUDA(cudaGetDevice(&dev0));

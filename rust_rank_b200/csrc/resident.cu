@@ -429,7 +429,8 @@ int prepare(rr_krylov* kr) {
   // the limit is per kernel, shared by every thread of the process: always the largest
   RR_CUDA(cudaFuncSetAttribute(resident_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
   cudaStream_t s = mat->ctx->stream;
-  RR_TRY(kr->res_gram.alloc_async((size_t)2 * kResMaxApps * (B * (B + 1) / 2), s));
+  kr->res_apps = std::min(mat->ctx->run_apps, kResMaxApps);
+  RR_TRY(kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps), s));
   RR_CUDA(cudaMemsetAsync(kr->res_gram.ptr, 0, kr->res_gram.bytes(), s));
   RR_TRY(kr->res_bar.alloc_async(1, s));
   RR_CUDA(cudaMemsetAsync(kr->res_bar.ptr, 0, kr->res_bar.bytes(), s));

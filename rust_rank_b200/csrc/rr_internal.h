@@ -133,6 +133,7 @@ struct rr_ctx_s {
   int device = 0;
   cudaStream_t stream = nullptr;
   int num_sms = 0;
+  int run_apps = 512;       // most applications of one resident run of its handles (at most kResMaxApps)
   int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
   std::atomic<uint64_t> wait_limit_ns{2000000000ull};  // device-side waits of its resident runs (rr_ctx_set_waits)
   std::atomic<int> wait_missing{0};
@@ -221,7 +222,7 @@ struct rr_krylov_s {
   int64_t graph_launches = 0;
   // runs with the CSR in shared memory (resident.cu): CTAs (0 = the matrix does
   // not fit), entries of A per CTA, dynamic shared memory, Gram sums, barrier
-  int res_grid = 0, res_entriesA = 0, res_share = -1;
+  int res_grid = 0, res_entriesA = 0, res_share = -1, res_apps = 0;  // res_apps: most applications of a run
   size_t res_smem = 0;
   rr::DevBuf<unsigned long long> res_gram;
   rr::DevBuf<unsigned int> res_bar;
@@ -237,10 +238,13 @@ int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev);
 int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out, int* status_out);  // status_out: kr->d_status with the block
 // Runs of applications in one launch with the CSR in shared memory
 // (resident.cu): resident_prepare sets kr->res_grid where the matrix fits, and
-// resident_run then takes 1 <= apps <= kResMaxApps applications at once, or
+// resident_run then takes 1 <= apps <= kr->res_apps applications at once, or
 // none (*taken = false) while a batch holds the device.
 constexpr int kResMaxApps = 512;
 constexpr int kCoopShares = 4;  // shares of a device for runs side by side (rr_ctx::coop_share)
+// Gram slots of its runs: two 64-bit sums per pair and application (no pass of
+// width 32 runs resident).
+inline size_t resident_gram_words(int B, int64_t apps) { return B <= 16 ? (size_t)apps * B * (B + 1) : 0; }
 int resident_prepare(rr_krylov* kr);
 int resident_run(rr_krylov* kr, int apps, bool* taken);
 // Held while persistent launches of a batch may be in flight on stream s: no
@@ -258,8 +262,9 @@ int krylov_occupancy(rr_krylov* kr);
 // bytes a matrix and its Krylov state hold while resident (server.cpp).
 int64_t max_nlen_for(int64_t m, int64_t n, int b);
 int padded(int b);
-size_t footprint_of(int64_t m, int64_t n, int64_t nnz, int b, int64_t max_nlen);
+size_t footprint_of(int64_t m, int64_t n, int64_t nnz, int b, int64_t max_nlen, int64_t run_apps);
 struct ServerSnapshot {
+  int run_apps = 0;  // most applications of one resident run
   std::vector<double> latencies_ms;
   int64_t submitted = 0, completed = 0;
   double t_first = 0, t_last = 0;  // seconds on the steady clock

@@ -38,6 +38,7 @@
 #include <thread>
 #include <vector>
 
+#include "krylov_params.h"
 #include "rr_internal.h"
 
 namespace {
@@ -95,15 +96,18 @@ int64_t max_nlen_for(int64_t m, int64_t n, int b) {
 int padded(int b) { return b <= 4 ? 4 : b <= 8 ? 8 : b <= 16 ? 16 : 32; }
 
 // Device bytes a request holds while resident: both CSR copies, the Krylov
-// blocks and preconditioner forms, and its device sequence.
-size_t footprint_of(int64_t m, int64_t n, int64_t nnz, int b, int64_t max_nlen) {
+// blocks and preconditioner forms, its device sequence, and the Gram sums of
+// the passes and of resident runs of up to run_apps applications.
+size_t footprint_of(int64_t m, int64_t n, int64_t nnz, int b, int64_t max_nlen, int64_t run_apps) {
   const int B = padded(b);
   const size_t np = (size_t)b * (b + 1) / 2;
   const size_t csr = 2 * 8 * (size_t)nnz + 8 * (size_t)(m + n + 2) + 4 * (size_t)n;
   const size_t blocks = 4 * (size_t)B * (2 * (size_t)n + (size_t)m) + 4 * (size_t)(m + 3 * n);
   const size_t heavy = 8 * (size_t)B * (size_t)std::max(m, n) / 16;  // generous bound on split rows
   const size_t seq = 4 * np * (size_t)(max_nlen + 2);
-  return (size_t)((double)(csr + blocks + heavy + seq) * 1.1) + (1u << 20);
+  const size_t gram = 8 * (resident_gram_words(B, run_apps) + (size_t)kGramReplicas * B * (B + 1));
+  // beside what grows with the matrix, 1 MiB, of which 256 KiB is for small buffers and rounding
+  return (size_t)((double)(csr + blocks + heavy + seq) * 1.1) + std::max<size_t>(1u << 20, gram + (256u << 10));
 }
 
 }  // namespace rr
@@ -417,6 +421,7 @@ void rr::server_snapshot(rr_server* s, ServerSnapshot* out) {
   out->t_first = std::chrono::duration<double>(s->t_first.time_since_epoch()).count();
   out->t_last = std::chrono::duration<double>(s->t_last.time_since_epoch()).count();
   out->hbm_budget = s->cfg.hbm_budget;
+  out->run_apps = s->lanes[0]->run_apps;
 }
 
 extern "C" {
@@ -446,6 +451,7 @@ int rr_server_create(int device, const rr_server_config* cfg, rr_server** out) {
       for (rr_ctx* x : s->lanes) rr_ctx_destroy(x);
       return rc;
     }
+    c->run_apps = (int)std::min<int64_t>(s->cfg.chunk_apps, rr::kResMaxApps);  // what the scheduler queues at once
     if (s->cfg.lanes > 1) c->coop_share = l % rr::kCoopShares;  // the lanes' runs side by side
     s->lanes.push_back(c);
     s->lane_load.push_back(0);
@@ -473,7 +479,7 @@ int rr_server_submit(rr_server* s, int64_t m, int64_t n, const int64_t* rowptr, 
   r->rp.assign(row_precond, row_precond + m);
   r->cp.assign(col_precond, col_precond + n);
   r->V.assign(V, V + (size_t)s->cfg.b * n);
-  r->footprint = footprint_of(m, n, nnz, s->cfg.b, max_nlen_for(m, n, s->cfg.b));
+  r->footprint = footprint_of(m, n, nnz, s->cfg.b, max_nlen_for(m, n, s->cfg.b), s->lanes[0]->run_apps);
   if (r->footprint > s->cfg.hbm_budget)
     return fail(RR_ENOMEM, "request needs about %zu bytes of device memory, over the budget of %llu", r->footprint,
                 (unsigned long long)s->cfg.hbm_budget);
