@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -100,13 +101,21 @@ int staging_of(rr_ctx* ctx, Staging** out) {
   return RR_OK;
 }
 
-// work(w) on nt threads, the calling one among them; the first error wins.
+// work(w) for every w < nt, on a thread each as far as the system gives them, the
+// calling thread doing the rest (an exception must not leave through the C
+// entry points); the first error wins.
 template <class F>
 int run_copies(int nt, const char* what, F work) {
   std::vector<cudaError_t> cerr(nt, cudaSuccess);
   std::vector<std::thread> pool;
-  for (int w = 1; w < nt; ++w) pool.emplace_back([&, w] { cerr[w] = work(w); });
+  pool.reserve(nt);
+  int started = 1;
+  try {
+    for (; started < nt; ++started) pool.emplace_back([&cerr, &work, w = started] { cerr[w] = work(w); });
+  } catch (const std::system_error&) {
+  }
   cerr[0] = work(0);
+  for (int w = started; w < nt; ++w) cerr[w] = work(w);
   for (std::thread& t : pool) t.join();
   for (int w = 0; w < nt; ++w)
     if (cerr[w] != cudaSuccess) return fail(RR_ECUDA, "staged %s copy failed: %s", what, cudaGetErrorString(cerr[w]));
