@@ -438,9 +438,9 @@ int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int6
   int dstat = 0;
   std::vector<uint32_t> tmp;
   DevBuf<uint32_t> pairs;
-  const bool transpose = cnt >= kTransposeTerms;  // pair-major on the device, then one strided copy
+  // pair-major on the device, then one strided copy, where the device has room for it
+  const bool transpose = cnt >= kTransposeTerms && pairs.alloc_async((size_t)cnt * np, st) == RR_OK;
   if (transpose) {
-    RR_TRY(pairs.alloc_async((size_t)cnt * np, st));
     RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr));
   } else {
     tmp.resize((size_t)cnt * np);

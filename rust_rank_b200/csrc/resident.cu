@@ -430,7 +430,10 @@ int prepare(rr_krylov* kr) {
   RR_CUDA(cudaFuncSetAttribute(resident_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
   cudaStream_t s = mat->ctx->stream;
   kr->res_apps = std::min(mat->ctx->run_apps, kResMaxApps);
-  RR_TRY(kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps), s));
+  if (kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps), s) != RR_OK) {  // no room: the pass kernels
+    kr->res_grid = 0;
+    return RR_OK;
+  }
   RR_CUDA(cudaMemsetAsync(kr->res_gram.ptr, 0, kr->res_gram.bytes(), s));
   RR_TRY(kr->res_bar.alloc_async(1, s));
   RR_CUDA(cudaMemsetAsync(kr->res_bar.ptr, 0, kr->res_bar.bytes(), s));
