@@ -393,7 +393,7 @@ static int queue_apps(rr_krylov* kr, int64_t n_apps) {
   if (kr->len == 0) kr->len = 1;  // publish S_0
   RR_TRY(ensure_capacity(kr, kr->len - kr->base + 2 * n_apps + 1));
   int64_t i = 0;
-  if (kr->res_grid > 0 && n_apps >= resident_min_run(kr)) {
+  if (kr->res_deepest >= 0 && n_apps >= resident_min_run(kr)) {
     for (bool taken = true; taken && i < n_apps;) {
       const int k = (int)std::min<int64_t>(kr->res_apps, n_apps - i);
       RR_TRY(resident_run(kr, k, &taken));

@@ -330,52 +330,138 @@ __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P
 
 // Cooperative grids of one device.  Grids that together need more SMs than
 // there are must not be in flight together: each could hold some SMs and wait
-// for the rest.  Runs of the whole device follow one another through an event;
-// runs of a share of it (the lanes of a rank service, 1 / kCoopShares of the
-// SMs at most) follow the runs of the same share and of the whole device.  None
-// is queued while a batch holds the device.
+// for the rest.  So a run takes a share of the device, 1 / 2^level of its SMs
+// (slot j of level l is [j, j + 1) sms / 2^l), and waits, through events, for
+// the last runs of the parts it takes; two runs in flight never share a part,
+// and waits only go back to runs queued earlier.  None is queued while a batch
+// holds the device.
+//
+// Level: a run alone on the device takes all the SMs it has row batches for;
+// when the streams of k other contexts have runs in flight, 1 / (k + 1) of
+// them, as far down as the matrix still fits the share's shared memory.  These
+// runs are bound by latency, so side by side they lose little each.  Measured
+// (ms for 256 applications in each of 8 contexts; pass kernels / runs of the
+// whole device one after the other / side by side): 700 rows, b = 4: 4.1 / 11.2 /
+// 2.2; 5000 rows, b = 8: 5.5 / 14.0 / 3.7; 20,000 rows, b = 8: 8.2 / 15.7 / 7.8;
+// 64 applications, 60,000 rows, b = 16: 14.8 / 10.1 / 8.8.
+//
+// Runs of fewer than kResShort applications (width 16 only, see queue_apps) are
+// taken alone on the device only: among others the pass kernels are as good or
+// better (8 contexts, 64 applications of 2000 rows one by one: 6.0 ms with runs,
+// 5.2 without; 32 of 20,000 rows: 3.4 / 3.2).
+constexpr int kResShort = 4;
+constexpr int kCoopLevels = 4;               // the smallest share: 1/16, 9 SMs
+constexpr int kCoopParts = 1 << kCoopLevels;
+
 struct CoopChain {
+  struct Run {
+    cudaEvent_t done = nullptr;
+    cudaStream_t stream = nullptr;
+    uint64_t seq = 0;        // order of queuing
+    int parts = 0;           // parts whose last run this is; 0 = a free record
+    bool finished = false;   // seen complete
+  };
   std::mutex m;
-  cudaEvent_t done[kCoopShares + 1] = {};  // the last run of each share, and of the whole device
-  int holds = 0;                           // batches with persistent launches in flight
-  // stream s waits for the last run of share q (an event never recorded does not wait)
-  int wait(cudaStream_t s, int q) {
-    if (done[q]) RR_CUDA(cudaStreamWaitEvent(s, done[q], 0));
+  Run runs[kCoopParts + 1];  // as many as can be the last run of a part, and one to fill in
+  Run* last[kCoopParts] = {};
+  uint64_t seq = 0;
+  int holds = 0;             // batches with persistent launches in flight
+
+  bool pending(const Run& r, cudaStream_t s) const { return r.parts > 0 && !r.finished && r.stream != s; }
+  // stream s waits for run r
+  int wait(cudaStream_t s, const Run& r) {
+    if (pending(r, s)) RR_CUDA(cudaStreamWaitEvent(s, r.done, 0));
     return RR_OK;
+  }
+  // Streams other than s with runs in flight.
+  int others(cudaStream_t s) {
+    int n = 0;
+    // an event query is not allowed while any thread captures in the global mode
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    bool asked = false;
+    for (Run& r : runs) {
+      if (!pending(r, s)) continue;
+      if (!asked) cudaThreadExchangeStreamCaptureMode(&mode);
+      asked = true;
+      const cudaError_t e = cudaEventQuery(r.done);
+      r.finished = e == cudaSuccess;
+      if (r.finished) continue;
+      cudaGetLastError();  // not ready is not an error
+      bool seen = false;
+      for (const Run* q = runs; q != &r && !seen; ++q) seen = pending(*q, s) && q->stream == r.stream;
+      n += !seen;
+    }
+    if (asked) cudaThreadExchangeStreamCaptureMode(&mode);
+    return n;
   }
 };
 constexpr int kMaxDevices = 64;
 CoopChain g_coop[kMaxDevices];
 
+// A run's turn: its level and the wait for the parts it takes, held until the
+// run is queued.
 class CoopTurn {
  public:
-  // share < 0: the whole device
-  int begin(int device, cudaStream_t s, int share, bool* taken) {
-    *taken = false;
+  // The run may go from level `top` (it has no use for more SMs) to `deepest`
+  // (it does not fit fewer); *level = the one it takes, -1 = none: a batch holds
+  // the device, or (alone_only) other streams have runs in flight.
+  int begin(int device, cudaStream_t s, int top, int deepest, bool alone_only, int* level) {
+    *level = -1;
     if (device < 0 || device >= kMaxDevices) return RR_OK;
-    chain_ = &g_coop[device];
-    chain_->m.lock();
-    if (chain_->holds > 0) return RR_OK;
-    share_ = share < 0 ? kCoopShares : share;
-    if (!chain_->done[share_]) RR_CUDA(cudaEventCreateWithFlags(&chain_->done[share_], cudaEventDisableTiming));
-    for (int q = 0; q <= kCoopShares; ++q)
-      if (share < 0 || q == share_ || q == kCoopShares) RR_TRY(chain_->wait(s, q));
+    c_ = &g_coop[device];
+    c_->m.lock();
+    if (c_->holds > 0) return RR_OK;
+    const int streams = c_->others(s) + 1;
+    if (alone_only && streams > 1) return RR_OK;
+    int l = top;
+    while ((1 << l) < streams && l < deepest) ++l;
+    const int width = kCoopParts >> l;
+    // the slot whose runs of other streams were queued the longest ago, or that has none
+    uint64_t best = ~0ull;
+    for (int j = 0; j < kCoopParts; j += width) {
+      uint64_t newest = 0;
+      for (int q = j; q < j + width; ++q)
+        if (c_->last[q] && c_->pending(*c_->last[q], s)) newest = std::max(newest, c_->last[q]->seq);
+      if (newest < best) {
+        best = newest;
+        first_ = j;
+      }
+    }
+    width_ = width;
+    for (int q = first_; q < first_ + width; ++q)
+      if (c_->last[q] && (q == first_ || c_->last[q] != c_->last[q - 1])) RR_TRY(c_->wait(s, *c_->last[q]));
     stream_ = s;
-    *taken = true;
+    *level = l;
     return RR_OK;
   }
+  // The run is queued.
   int end() {
-    RR_CUDA(cudaEventRecord(chain_->done[share_], stream_));
+    CoopChain::Run* r = c_->runs;
+    while (r->parts > 0) ++r;
+    cudaError_t e = r->done ? cudaSuccess : cudaEventCreateWithFlags(&r->done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(r->done, stream_);
+    if (e != cudaSuccess) {  // nobody could wait for the run
+      cudaStreamSynchronize(stream_);
+      RR_CUDA(e);
+    }
+    for (int q = first_; q < first_ + width_; ++q) {
+      if (c_->last[q]) --c_->last[q]->parts;
+      c_->last[q] = r;
+    }
+    r->stream = stream_;
+    r->seq = ++c_->seq;
+    r->parts = width_;
+    r->finished = false;
     return RR_OK;
   }
   ~CoopTurn() {
-    if (chain_) chain_->m.unlock();
+    if (c_) c_->m.unlock();
   }
 
  private:
-  CoopChain* chain_ = nullptr;
+  CoopChain* c_ = nullptr;
   cudaStream_t stream_ = nullptr;
-  int share_ = 0;
+  int first_ = 0, width_ = 0;
 };
 
 // Gram sums of `terms` terms -> sequence terms (real pairs); the sums, the
@@ -403,35 +489,44 @@ int64_t entry_bound(int64_t nnz, int64_t max_degree, int rpw, int grid) {
   return rpw * max_degree + (nnz + rpw * max_degree) / grid + 1;
 }
 
+// The grid of a matrix at a level, its entries of A per CTA and its dynamic
+// shared memory (0 = it does not fit).
+struct ResShape {
+  int grid, entriesA;
+  size_t smem;
+};
+template <int B>
+ResShape shape_at(const rr_matrix* mat, int level) {
+  constexpr int RPW = 128 / B;
+  const int64_t batches = (std::max(mat->m, mat->n) + RPW - 1) / RPW;
+  ResShape r{(int)std::min<int64_t>(batches, mat->ctx->num_sms >> level), 0, 0};
+  if (r.grid == 0 || (batches + r.grid - 1) / r.grid > kMaxBatches) return r;
+  const int64_t ea = entry_bound(mat->nnz, mat->max_row_nnz, RPW, r.grid);
+  const size_t smem = res_fixed_smem<B>() + 8 * (size_t)(ea + entry_bound(mat->nnz, mat->max_col_nnz, RPW, r.grid));
+  if (smem > kResSmem) return r;
+  r.entriesA = (int)ea;
+  r.smem = smem;
+  return r;
+}
+
 template <int B>
 int prepare(rr_krylov* kr) {
   constexpr int RPW = 128 / B;
   const rr_matrix* mat = kr->mat;
-  const int64_t degA = mat->max_row_nnz, degAt = mat->max_col_nnz;
-  kr->res_grid = 0;
-  if (degA > kResMaxDegree || degAt > kResMaxDegree) return RR_OK;
+  kr->res_deepest = -1;
+  if (mat->max_row_nnz > kResMaxDegree || mat->max_col_nnz > kResMaxDegree) return RR_OK;
+  for (int l = 0; l <= kCoopLevels && shape_at<B>(mat, l).smem > 0; ++l) kr->res_deepest = l;
+  if (kr->res_deepest < 0) return RR_OK;
   const int64_t batches = (std::max(mat->m, mat->n) + RPW - 1) / RPW;
-  // a share of the device where the context has one and the matrix fits it
-  const int sms = mat->ctx->num_sms, share = mat->ctx->coop_share;
-  for (int cap : {share < 0 ? sms : sms / kCoopShares, sms}) {
-    const int grid = (int)std::min<int64_t>(batches, cap);
-    if ((batches + grid - 1) / grid > kMaxBatches) continue;
-    const int64_t ea = entry_bound(mat->nnz, degA, RPW, grid), et = entry_bound(mat->nnz, degAt, RPW, grid);
-    const size_t smem = res_fixed_smem<B>() + 8 * (size_t)(ea + et);
-    if (smem > kResSmem) continue;
-    kr->res_grid = grid;
-    kr->res_entriesA = (int)ea;
-    kr->res_smem = smem;
-    kr->res_share = cap < sms ? share : -1;
-    break;
-  }
-  if (kr->res_grid == 0) return RR_OK;
+  kr->res_top = 0;
+  while (kr->res_top < kr->res_deepest && (mat->ctx->num_sms >> (kr->res_top + 1)) >= batches) ++kr->res_top;
+  if (mat->ctx->coop_level <= kr->res_deepest) kr->res_top = std::max(kr->res_top, mat->ctx->coop_level);
   // the limit is per kernel, shared by every thread of the process: always the largest
   RR_CUDA(cudaFuncSetAttribute(resident_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
   cudaStream_t s = mat->ctx->stream;
   kr->res_apps = std::min(mat->ctx->run_apps, kResMaxApps);
   if (kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps), s) != RR_OK) {  // no room: the pass kernels
-    kr->res_grid = 0;
+    kr->res_deepest = -1;
     return RR_OK;
   }
   RR_CUDA(cudaMemsetAsync(kr->res_gram.ptr, 0, kr->res_gram.bytes(), s));
@@ -468,9 +563,7 @@ int run(rr_krylov* kr, int apps, bool* taken) {
   P.w6 = (uint32_t)((uint64_t)P.w5 * 256 % kr->M.p);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.gridDim = dim3((unsigned)kr->res_grid);
   cfg.blockDim = dim3(kResThreads<B>);
-  cfg.dynamicSmemBytes = kr->res_smem;
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
@@ -478,9 +571,14 @@ int run(rr_krylov* kr, int apps, bool* taken) {
   attr[0].val.cooperative = 1;
   {
     CoopTurn turn;
-    RR_TRY(turn.begin(mat->ctx->device, s, kr->res_share, taken));
+    int level;
+    RR_TRY(turn.begin(mat->ctx->device, s, kr->res_top, kr->res_deepest, apps < kResShort, &level));
+    *taken = level >= 0;
     if (!*taken) return RR_OK;
-    RR_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel<B>, P, kr->res_entriesA));
+    const ResShape shape = shape_at<B>(mat, level);
+    cfg.gridDim = dim3((unsigned)shape.grid);
+    cfg.dynamicSmemBytes = shape.smem;
+    RR_CUDA(cudaLaunchKernelEx(&cfg, resident_kernel<B>, P, shape.entriesA));
     RR_TRY(turn.end());
   }
   const int np = kr->b * (kr->b + 1) / 2, NP = B * (B + 1) / 2;
@@ -500,7 +598,7 @@ int CoopHold::begin(int device, cudaStream_t s) {
   if (device < 0 || device >= kMaxDevices) return RR_OK;
   CoopChain& c = g_coop[device];
   std::lock_guard<std::mutex> lk(c.m);
-  for (int q = 0; q <= kCoopShares; ++q) RR_TRY(c.wait(s, q));
+  for (const CoopChain::Run& r : c.runs) RR_TRY(c.wait(s, r));
   device_ = device;
   ++c.holds;
   return RR_OK;
@@ -518,7 +616,7 @@ int resident_prepare(rr_krylov* kr) {
     case 8: return prepare<8>(kr);
     case 16: return prepare<16>(kr);
   }
-  kr->res_grid = 0;
+  kr->res_deepest = -1;
   return RR_OK;
 }
 

@@ -134,7 +134,7 @@ struct rr_ctx_s {
   cudaStream_t stream = nullptr;
   int num_sms = 0;
   int run_apps = 512;       // most applications of one resident run of its handles (at most kResMaxApps)
-  int coop_share = -1;      // share of the device its resident runs take (resident.cu); -1 = all of it
+  int coop_level = 0;       // its resident runs take 2^-coop_level of the device at most, where they fit (resident.cu)
   std::atomic<uint64_t> wait_limit_ns{2000000000ull};  // device-side waits of its resident runs (rr_ctx_set_waits)
   std::atomic<int> wait_missing{0};
   std::mutex curv_mu;
@@ -220,10 +220,10 @@ struct rr_krylov_s {
   cudaStream_t launch_stream = nullptr;  // set while capturing (a private stream), else the context's
   int graph_cur = 0;
   int64_t graph_launches = 0;
-  // runs with the CSR in shared memory (resident.cu): CTAs (0 = the matrix does
-  // not fit), entries of A per CTA, dynamic shared memory, Gram sums, barrier
-  int res_grid = 0, res_entriesA = 0, res_share = -1, res_apps = 0;  // res_apps: most applications of a run
-  size_t res_smem = 0;
+  // runs with the CSR in shared memory (resident.cu): the shares of the device
+  // they may take (2^-res_top down to 2^-res_deepest; -1 = the matrix does not
+  // fit), most applications of a run, Gram sums, barrier
+  int res_top = 0, res_deepest = -1, res_apps = 0;
   rr::DevBuf<unsigned long long> res_gram;
   rr::DevBuf<unsigned int> res_bar;
   ~rr_krylov_s() {
@@ -237,11 +237,10 @@ int krylov_reserve(rr_krylov* kr, int64_t terms);
 int krylov_launch_application(rr_krylov* kr, cudaEvent_t* ev);
 int krylov_launch_get_curv(rr_krylov* kr, uint32_t* d_out, int* status_out);  // status_out: kr->d_status with the block
 // Runs of applications in one launch with the CSR in shared memory
-// (resident.cu): resident_prepare sets kr->res_grid where the matrix fits, and
+// (resident.cu): resident_prepare sets kr->res_deepest where the matrix fits, and
 // resident_run then takes 1 <= apps <= kr->res_apps applications at once, or
 // none (*taken = false) while a batch holds the device.
 constexpr int kResMaxApps = 512;
-constexpr int kCoopShares = 4;  // shares of a device for runs side by side (rr_ctx::coop_share)
 // Gram slots of its runs: two 64-bit sums per pair and application (no pass of
 // width 32 runs resident).
 inline size_t resident_gram_words(int B, int64_t apps) { return B <= 16 ? (size_t)apps * B * (B + 1) : 0; }
