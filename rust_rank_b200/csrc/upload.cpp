@@ -9,7 +9,13 @@
 // Arrays already in pinned memory go straight to cudaMemcpyAsync.  Results leave
 // the device the same way: a 96 MB block took 21 ms as one pageable copy (which
 // also touches the fresh pages of the caller's array on one thread), 5 ms through
-// the staging buffers.
+// the staging buffers.  Below 8 MB that pays only where the array's pages are
+// still to be touched: into touched ones the driver's copy takes 0.29 ms for
+// 4.5 MB and 0.36 for 6, the staged one anything from 0.29 to 0.66 (its threads'
+// start is most of it); into fresh ones 2.5 and 3.3 ms against 1.5 and 1.9.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -24,6 +30,7 @@ namespace rr {
 namespace {
 constexpr size_t kPiece = 2u << 20;     // bytes per staged piece
 constexpr size_t kStageMin = 4u << 20;  // smaller copies go straight to the driver
+constexpr size_t kStageTouched = 8u << 20;  // downloads into touched pages: staged from here on
 constexpr int kMaxStageThreads = 8;
 constexpr size_t kStageNew = 32u << 20;  // downloads a context creates its buffers for
 }  // namespace
@@ -56,6 +63,19 @@ static bool is_pinned(const void* p) {
 
 namespace {
 
+// Whether at least half of the pages of [p, p + bytes) are there already (bytes
+// below kStageTouched).
+bool touched(const void* p, size_t bytes) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  unsigned char there[kStageTouched / 4096 + 2];
+  const uintptr_t lo = (uintptr_t)p / page * page, hi = (uintptr_t)p + bytes;
+  const size_t n = (hi - lo + page - 1) / page;
+  if (n > sizeof(there) || mincore((void*)lo, hi - lo, there) != 0) return false;
+  size_t count = 0;
+  for (size_t i = 0; i < n; ++i) count += there[i] & 1;
+  return 2 * count >= n;
+}
+
 struct Piece {
   char* dst;
   const char* src;
@@ -67,7 +87,9 @@ struct Piece {
 int split_segments(const std::vector<HostSegment>& segs, cudaMemcpyKind kind, cudaStream_t s, std::vector<Piece>* pieces) {
   for (const HostSegment& g : segs) {
     if (g.bytes == 0) continue;
-    if (g.bytes < kStageMin || is_pinned(kind == cudaMemcpyHostToDevice ? g.src : g.dst)) {
+    const bool down = kind == cudaMemcpyDeviceToHost;
+    if (g.bytes < kStageMin || is_pinned(down ? g.dst : g.src) ||
+        (down && g.bytes < kStageTouched && touched(g.dst, g.bytes))) {
       RR_CUDA(cudaMemcpyAsync(g.dst, g.src, g.bytes, kind, s));
       continue;
     }
