@@ -67,8 +67,11 @@ ModP make_modp(uint32_t p) {
 
 int launch_scatter_block(rr_krylov* kr, const uint32_t* d_V, uint32_t* d_out);
 int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out);
-// Terms from which a fetch transposes on the device: below, the host loop is shorter than the launch and the strided copy.
-constexpr int64_t kTransposeTerms = 1024;
+// Terms and words from which a fetch transposes on the device: below, the host
+// loop is shorter than the launch and the strided copy.  Measured (us, host loop /
+// device): b = 1, 2048 terms 36 / 39.5, 6000 terms 45 / 41; b = 2, 1400 terms 40.5 /
+// 43.8, 3000 terms 50.6 / 46.5; b = 3, 1024 terms 45 / 42; b = 16, 1024 terms 550 / 78.
+constexpr int64_t kTransposeTerms = 1024, kTransposeWords = 6 * 1024;
 int launch_precond(rr_krylov* kr, const uint32_t* d_rp, const uint32_t* d_cp, const int32_t* d_rowperm);
 
 }  // namespace rr
@@ -439,7 +442,8 @@ int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int6
   std::vector<uint32_t> tmp;
   DevBuf<uint32_t> pairs;
   // pair-major on the device, then one strided copy, where the device has room for it
-  const bool transpose = cnt >= kTransposeTerms && pairs.alloc_async((size_t)cnt * np, st) == RR_OK;
+  const bool transpose =
+      cnt >= kTransposeTerms && cnt * np >= kTransposeWords && pairs.alloc_async((size_t)cnt * np, st) == RR_OK;
   if (transpose) {
     RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr));
   } else {
