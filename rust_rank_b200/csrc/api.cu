@@ -66,7 +66,8 @@ ModP make_modp(uint32_t p) {
 }
 
 int launch_scatter_block(rr_krylov* kr, const uint32_t* d_V, uint32_t* d_out);
-int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out);
+int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out, const int* status,
+                      int* status_out);
 // Terms and words from which a fetch transposes on the device: below, the host
 // loop is shorter than the launch and the strided copy.  Measured (us, host loop /
 // device): b = 1, 2048 terms 36 / 39.5, 6000 terms 45 / 41; b = 2, 1400 terms 40.5 /
@@ -174,7 +175,7 @@ int rr_ctx_destroy(rr_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   cudaStreamDestroy(ctx->stream);
   rr::staging_destroy(ctx->staging);
-  if (ctx->curv_status) cudaFreeHost(ctx->curv_status);
+  if (ctx->status_word) cudaFreeHost(ctx->status_word);
   delete ctx;
   return RR_OK;
 }
@@ -426,6 +427,18 @@ int rr_krylov_step_device(rr_krylov* kr, int64_t n_apps) {
   return queue_apps(kr, n_apps);
 }
 
+// The context's pinned word for a handle's status; the caller holds ctx->status_mu.
+static int status_word(rr_ctx* ctx, int** word) {
+  if (!ctx->status_word) RR_CUDA(cudaHostAlloc((void**)&ctx->status_word, sizeof(int), cudaHostAllocMapped));
+  *word = ctx->status_word;
+  return RR_OK;
+}
+
+static int waits_ended(int status, const char* what) {
+  if (status) return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the %s not valid", what);
+  return RR_OK;
+}
+
 int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int64_t seq_stride) {
   if (!kr || (!seq && to > from)) return fail(RR_EINVAL, "NULL argument");
   if (from < kr->base || to > kr->len || from > to)
@@ -438,28 +451,28 @@ int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int6
   if (cnt == 0) return RR_OK;
   cudaStream_t st = kr->mat->ctx->stream;
   const uint32_t* terms = kr->S.ptr + (size_t)(from - kr->base) * np;
-  int dstat = 0;
-  std::vector<uint32_t> tmp;
+  // pair-major on the device, then one strided copy, where the device has room
+  // for it.  Either way seq is written only once the terms are known to be valid.
   DevBuf<uint32_t> pairs;
-  // pair-major on the device, then one strided copy, where the device has room for it
-  const bool transpose =
-      cnt >= kTransposeTerms && cnt * np >= kTransposeWords && pairs.alloc_async((size_t)cnt * np, st) == RR_OK;
-  if (transpose) {
-    RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr));
-  } else {
-    tmp.resize((size_t)cnt * np);
-    RR_CUDA(cudaMemcpyAsync(tmp.data(), terms, tmp.size() * 4, cudaMemcpyDeviceToHost, st));
-  }
-  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-  RR_CUDA(cudaStreamSynchronize(st));
-  // seq is written only once the terms are known to be valid
-  if (dstat) return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the terms are not valid");
-  if (transpose) {
+  if (cnt >= kTransposeTerms && cnt * np >= kTransposeWords && pairs.alloc_async((size_t)cnt * np, st) == RR_OK) {
+    std::unique_lock<std::mutex> lk(kr->mat->ctx->status_mu);
+    int* status;
+    RR_TRY(status_word(kr->mat->ctx, &status));
+    RR_TRY(launch_pair_major(st, terms, cnt, np, pairs.ptr, kr->d_status.ptr, status));
+    RR_CUDA(cudaStreamSynchronize(st));
+    RR_TRY(waits_ended(*(volatile int*)status, "terms are"));
+    lk.unlock();
     RR_CUDA(cudaMemcpy2DAsync(seq + from, (size_t)seq_stride * 4, pairs.ptr, (size_t)cnt * 4, (size_t)cnt * 4, np,
                               cudaMemcpyDeviceToHost, st));
     RR_CUDA(cudaStreamSynchronize(st));
     return RR_OK;
   }
+  std::vector<uint32_t> tmp((size_t)cnt * np);
+  int dstat = 0;
+  RR_CUDA(cudaMemcpyAsync(tmp.data(), terms, tmp.size() * 4, cudaMemcpyDeviceToHost, st));
+  RR_CUDA(cudaMemcpyAsync(&dstat, kr->d_status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  RR_CUDA(cudaStreamSynchronize(st));
+  RR_TRY(waits_ended(dstat, "terms are"));
   for (int64_t t = 0; t < cnt; ++t)
     for (int q = 0; q < np; ++q) seq[(size_t)q * seq_stride + from + t] = tmp[(size_t)t * np + q];
   return RR_OK;
@@ -553,16 +566,15 @@ int rr_krylov_get_curv(rr_krylov* kr, uint32_t* curv) {
   RR_CUDA(cudaSetDevice(ctx->device));
   // the gathering kernel also writes the handle's status, into a pinned word of
   // the context: no second copy
-  std::lock_guard<std::mutex> lk(ctx->curv_mu);
-  if (!ctx->curv_status) RR_CUDA(cudaHostAlloc((void**)&ctx->curv_status, sizeof(int), cudaHostAllocMapped));
+  std::lock_guard<std::mutex> lk(ctx->status_mu);
+  int* status;
+  RR_TRY(status_word(ctx, &status));
   DevBuf<uint32_t> out;
   RR_TRY(out.alloc_async((size_t)kr->b * kr->mat->n, ctx->stream));
-  RR_TRY(krylov_launch_get_curv(kr, out.ptr, ctx->curv_status));
+  RR_TRY(krylov_launch_get_curv(kr, out.ptr, status));
   RR_TRY(rr::download_host(ctx, {{curv, out.ptr, out.bytes()}}, ctx->stream));
   RR_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (*(volatile int*)ctx->curv_status)
-    return fail(RR_ETIMEOUT, "a device-side wait of the Krylov kernels gave up; the block is not valid");
-  return RR_OK;
+  return waits_ended(*(volatile int*)status, "block is");
 }
 
 int rr_krylov_bytes_per_application(const rr_krylov* kr, double* bytes) {

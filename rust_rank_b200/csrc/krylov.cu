@@ -1641,8 +1641,10 @@ int launch_precond(rr_krylov* kr, const uint32_t* d_rp, const uint32_t* d_cp, co
   return RR_OK;
 }
 
-// out[q][t] = terms[t][q] (32 x 32 tiles through shared memory)
-__global__ void pair_major_kernel(const uint32_t* __restrict__ terms, int64_t count, int np, uint32_t* __restrict__ out) {
+// out[q][t] = terms[t][q] (32 x 32 tiles through shared memory), and the status beside it
+__global__ void pair_major_kernel(const uint32_t* __restrict__ terms, int64_t count, int np, uint32_t* __restrict__ out,
+                                  const int* status, int* status_out) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *status_out = *status;
   __shared__ uint32_t tile[32][33];
   const int64_t t0 = (int64_t)blockIdx.x * 32;
   const int q0 = blockIdx.y * 32;
@@ -1653,9 +1655,10 @@ __global__ void pair_major_kernel(const uint32_t* __restrict__ terms, int64_t co
     if (q0 + y < np && t0 + threadIdx.x < count) out[(int64_t)(q0 + y) * count + t0 + threadIdx.x] = tile[threadIdx.x][y];
 }
 
-int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out) {
+int launch_pair_major(cudaStream_t s, const uint32_t* terms, int64_t count, int np, uint32_t* out, const int* status,
+                      int* status_out) {
   const dim3 grid((unsigned)((count + 31) / 32), (unsigned)((np + 31) / 32));
-  pair_major_kernel<<<grid, dim3(32, 8), 0, s>>>(terms, count, np, out);
+  pair_major_kernel<<<grid, dim3(32, 8), 0, s>>>(terms, count, np, out, status, status_out);
   RR_CUDA(cudaGetLastError());
   return RR_OK;
 }
