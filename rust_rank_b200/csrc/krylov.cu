@@ -909,13 +909,16 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
             *reinterpret_cast<uint32_t*>(buf + tc_off(T::N, h * T::H + a * B + c4 * T::GROUPS + gw, 4 * qd)) = wz[a];
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // stores visible to the tensor cores
+      // Orders this thread's accesses before what the async proxy does after the
+      // arrivals below: its stores before the tensor cores' reads of the operands,
+      // and its reads of the raw tile before the bulk copy that overwrites it.  Both
+      // arrivals have to stay behind it: with raw_empty's right after the reads the
+      // next copy overtook some of them (2 wrong terms in 65,000 at 600k x 408k,
+      // b = 16).
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&op_full[s]);
-        // Only now, when every value read has gone into a store: an arrival right
-        // after the reads was seen to let the next copy overtake some of them
-        // (2 wrong terms in 65,000 at 600k x 408k, b = 16).
         mbar_arrive(&raw_empty[slot]);
       }
     }
