@@ -137,8 +137,8 @@ struct rr_ctx_s {
   int coop_level = 0;       // its resident runs take 2^-coop_level of the device at most, where they fit (resident.cu)
   std::atomic<uint64_t> wait_limit_ns{2000000000ull};  // device-side waits of its resident runs (rr_ctx_set_waits)
   std::atomic<int> wait_missing{0};
-  std::mutex status_mu;
-  int* status_word = nullptr;  // pinned: the status that a kernel writes beside the results it prepares for the host
+  std::mutex pinned_mu;
+  uint32_t* pinned = nullptr;  // host buffer for small results and a status word (api.cu), created at first use
   int pm_tensor_cores = 1;  // PM-basis contractions on the int8 tensor cores (0: CUDA cores)
 };
 
