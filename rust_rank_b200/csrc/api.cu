@@ -274,12 +274,6 @@ int rr_krylov_create(rr_matrix* mat, int32_t b, const uint32_t* row_precond, con
   kr->b = b;
   kr->B = padded_width(b);
   kr->M = make_modp(p);
-  {
-    // four products fit between folds iff (2^32-1)*c32 + 2^32 - 1 + 4 (p-1)^2 < 2^64
-    const unsigned __int128 F = (unsigned __int128)0xffffffffull * kr->M.c32 + 0xffffffffull;
-    const unsigned __int128 q = (unsigned __int128)(p - 1) * (p - 1);
-    kr->fold4 = (F + 4 * q) < ((unsigned __int128)1 << 64);
-  }
   // preconditioners in device order, in the forms the epilogues use:
   // d_r R^2, d_c R^2, d_c R and d_c^{-1} (all mod p), computed on the device
   // from the caller's arrays and the row renumbering

@@ -39,7 +39,6 @@ struct rr_batch_s {
   int nmat = 0, b = 0, B = 0, np = 0;
   uint32_t p = 0;
   rr::ModP M{};
-  int fold4 = 0;
   int grid = 0;
   std::vector<int> order;        // stack position -> caller's index
   std::vector<int> pos_of;       // caller's index -> stack position
@@ -220,7 +219,7 @@ int launch_phase(rr_batch* bt, int ph, int var, int grid, const int32_t* d_ra, c
                  int64_t t_end, int cur0) {
   PersistParams Q = phase_params(bt, ph, var, d_ra, d_rt, t_begin, t_end, cur0);
   RR_CUDA(cudaMemsetAsync(bt->bar.ptr, 0, 2 * sizeof(unsigned int), bt->stream));
-  return launch_persistent_raw(bt->stream, bt->B, bt->fold4, grid, bt->lpt[var], Q);
+  return launch_persistent_raw(bt->stream, bt->B, grid, bt->lpt[var], Q);
 }
 
 // Autotuner: for every phase, time a persistent launch of three
@@ -323,7 +322,7 @@ int krylov_queue(rr_batch* bt, cudaEvent_t* ev) {
     P.seg_begin = 0;
     P.seg_end = nmat;
     P.term = 0;
-    RR_TRY(launch_pass_raw(st, bt->B, bt->fold4, bt->grid, P, kModeInit));
+    RR_TRY(launch_init_raw(st, bt->B, bt->grid, P));
   }
   RR_CUDA(cudaMemsetAsync(bt->error.ptr, 0, sizeof(int), st));
   const int64_t max_apps = bt->apps[nmat - 1];
@@ -415,11 +414,6 @@ int rr_batch_create(rr_ctx* ctx, int32_t nmat, const int64_t* m, const int64_t* 
   bt->np = b * (b + 1) / 2;
   bt->p = p;
   bt->M = make_modp(p);
-  {
-    const unsigned __int128 F = (unsigned __int128)0xffffffffull * bt->M.c32 + 0xffffffffull;
-    const unsigned __int128 q = (unsigned __int128)(p - 1) * (p - 1);
-    bt->fold4 = (F + 4 * q) < ((unsigned __int128)1 << 64);
-  }
   // validate (in parallel over matrices) and order by sequence length
   std::vector<int64_t> len(nmat);
   std::vector<std::string> bad(nmat);
@@ -589,8 +583,8 @@ int rr_batch_create(rr_ctx* ctx, int32_t nmat, const int64_t* m, const int64_t* 
   RR_CUDA(cudaMemsetAsync(bt->bar.ptr, 0, bt->bar.bytes(), st));
   RR_CUDA(cudaMemsetAsync(bt->error.ptr, 0, bt->error.bytes(), st));
   int blocks = 1, pblocks[2] = {1, 1};
-  RR_TRY(pass_blocks_per_sm(bt->B, bt->fold4, &blocks));
-  for (int v = 0; v < bt->nvar; ++v) RR_TRY(persistent_blocks_per_sm(bt->B, bt->fold4, bt->lpt[v], &pblocks[v]));
+  RR_TRY(init_blocks_per_sm(bt->B, &blocks));
+  for (int v = 0; v < bt->nvar; ++v) RR_TRY(persistent_blocks_per_sm(bt->B, bt->lpt[v], &pblocks[v]));
   bt->grid = std::max(1, blocks) * ctx->num_sms;
   // phases: one per distinct set of running matrices
   bt->phase_of.assign(nmat, -1);

@@ -51,9 +51,9 @@ static_assert(kWarps == kPassWarps, "host-side run tables assume this many warps
 
 // acc[l] += sum over entries k = beg, beg+stride, ... < end of val * X[col][lane l]
 // for this thread's LPT lanes (lane block `sub`).  Four entries per step, all
-// loads issued before the multiplies; acc is folded after every FE products,
+// loads issued before the multiplies; acc is folded after every kFold products,
 // so it leaves folded (< p * 2^32).
-template <int B, int FE, int L = kDefaultLpt<B>>
+template <int B, int L = kDefaultLpt<B>>
 __device__ __forceinline__ void mac_step(const uint2 (&e)[4], const uint4 (&g)[4][Shape<B, L>::NV], const ModP& M,
                                          uint64_t (&acc)[Shape<B, L>::LPT]) {
 #pragma unroll
@@ -66,7 +66,7 @@ __device__ __forceinline__ void mac_step(const uint2 (&e)[4], const uint4 (&g)[4
       acc[4 * v + 2] = mad_wide(val, g[u][v].z, acc[4 * v + 2]);
       acc[4 * v + 3] = mad_wide(val, g[u][v].w, acc[4 * v + 3]);
     }
-    if ((u % FE) == FE - 1) {
+    if ((u % kFold) == kFold - 1) {
 #pragma unroll
       for (int l = 0; l < Shape<B, L>::LPT; ++l) acc[l] = fold(acc[l], M);
     }
@@ -86,7 +86,7 @@ __device__ __forceinline__ uint4 ld_block(const uint4* p) {
   return __ldg(p);
 }
 
-template <int B, int FE, bool COH = false, int L = kDefaultLpt<B>>
+template <int B, bool COH = false, int L = kDefaultLpt<B>>
 __device__ __forceinline__ void gather_sum(const uint2* __restrict__ cv, uint32_t beg, uint32_t end, uint32_t stride,
                                            const uint4* __restrict__ X, int sub, const ModP& M,
                                            uint64_t (&acc)[Shape<B, L>::LPT]) {
@@ -112,7 +112,7 @@ __device__ __forceinline__ void gather_sum(const uint2* __restrict__ cv, uint32_
 #pragma unroll
         for (int u = 0; u < 4; ++u) en[u] = __ldg(cv + k + u * stride);
       }
-      mac_step<B, FE, L>(e, g, M, acc);
+      mac_step<B, L>(e, g, M, acc);
       if (!more) break;
 #pragma unroll
       for (int u = 0; u < 4; ++u) e[u] = en[u];
@@ -131,7 +131,7 @@ __device__ __forceinline__ void gather_sum(const uint2* __restrict__ cv, uint32_
     for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int v = 0; v < NV; ++v) g[u][v] = ld_block<COH>(Xs + (size_t)e[u].x * RW + v * Shape<B, L>::TPR);
-    mac_step<B, FE, L>(e, g, M, acc);
+    mac_step<B, L>(e, g, M, acc);
   }
 }
 
@@ -139,7 +139,7 @@ __device__ __forceinline__ void gather_sum(const uint2* __restrict__ cv, uint32_
 // thread): with 4 lanes per thread a whole 64- or 128-byte block row is one
 // warp load instruction (one L1 wavefront per gathered row instead of two),
 // and the eight loads keep as many bytes in flight as four steps of 8 lanes.
-template <int B, int FE, int L>
+template <int B, int L>
 __device__ __forceinline__ void gather_sum8(const uint2* __restrict__ cv, uint32_t beg, uint32_t end, uint32_t stride,
                                             const uint4* __restrict__ X, int sub, const ModP& M,
                                             uint64_t (&acc)[Shape<B, L>::LPT]) {
@@ -173,8 +173,8 @@ __device__ __forceinline__ void gather_sum8(const uint2* __restrict__ cv, uint32
           n1[u] = __ldg(cv + k + (u + 4) * stride);
         }
       }
-      mac_step<B, FE, L>(e0, g0, M, acc);
-      mac_step<B, FE, L>(e1, g1, M, acc);
+      mac_step<B, L>(e0, g0, M, acc);
+      mac_step<B, L>(e1, g1, M, acc);
       if (!more) break;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -196,7 +196,7 @@ __device__ __forceinline__ void gather_sum8(const uint2* __restrict__ cv, uint32
     for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int v = 0; v < NV; ++v) g[u][v] = __ldg(Xs + (size_t)e[u].x * RW + v * TPR);
-    mac_step<B, FE, L>(e, g, M, acc);
+    mac_step<B, L>(e, g, M, acc);
     k += 4 * stride;
   }
 }
@@ -233,19 +233,19 @@ __device__ __forceinline__ unsigned long long* seg_target(const PassParams& P, u
 // terms of the application.
 enum GramForm { kGramNone = 0, kGramOwn = 1, kGramBoth = 2 };
 
-template <int B, int FE, int L, int GRAM>
+template <int B, int L, int GRAM>
 struct GramOf {
-  using type = typename std::conditional<(B >= 8), GramMma<B, FE, L>, GramCore<B, FE, L>>::type;
+  using type = typename std::conditional<(B >= 8), GramMma<B, L>, GramCore<B, L>>::type;
 };
-template <int B, int FE, int L>
-struct GramOf<B, FE, L, kGramBoth> {
-  using type = GramDual<B, FE, L>;
+template <int B, int L>
+struct GramOf<B, L, kGramBoth> {
+  using type = GramDual<B, L>;
 };
 
 // One pass over the rows of A (MODE odd), of A^T (even) or the initial
 // scaling (init), by the whole CTA: gram_smem is the per-warp Gram staging,
 // red[NP] (2 NP with kGramBoth) the CTA's Gram reduction, is_last a shared flag.
-template <int B, int MODE, int FE, bool COH, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
+template <int B, int MODE, bool COH, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
 __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_smem, unsigned long long* red,
                                           bool& is_last) {
   using S = Shape<B, L>;
@@ -254,7 +254,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
   constexpr bool kBoth = GRAM == kGramBoth;
   constexpr bool kSym = MODE != kModeOdd && !kBoth;  // both Gram factors are the same rows: one set of byte planes
   constexpr int kSums = kBoth ? 2 * NP : NP;
-  using Gram = typename GramOf<B, FE, L, GRAM>::type;
+  using Gram = typename GramOf<B, L, GRAM>::type;
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -346,7 +346,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
             h[S::lane_of(sub, l)] = 0;
           }
         } else {
-          gather_sum<B, FE, COH, L>(P.cv, P.rowptr[r], P.rowptr[r + 1], 1u, P.X, sub, M, acc);
+          gather_sum<B, COH, L>(P.cv, P.rowptr[r], P.rowptr[r + 1], 1u, P.X, sub, M, acc);
         }
 #pragma unroll
         for (int l = 0; l < LPT; ++l) t[l] = redc(acc[l], M);  // t = (row sum) R^{-1}
@@ -490,13 +490,13 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
 template <int B, int GRAM>
 constexpr int kPassMinBlocks = (B >= 32 && GRAM) ? 2 : ((!GRAM && B == 16) ? 5 : 4);
 
-template <int B, int MODE, int FE, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
+template <int B, int MODE, int GRAM = kGramOwn, int L = kDefaultLpt<B>>
 __global__ void __launch_bounds__(kThreads, kPassMinBlocks<B, GRAM>) pass_kernel(PassParams P) {
   extern __shared__ __align__(16) uint32_t gram_smem[];
   __shared__ unsigned long long red[(GRAM == kGramBoth ? 2 : 1) * (B * (B + 1) / 2)];
   __shared__ bool is_last;
   griddep_wait();
-  pass_body<B, MODE, FE, false, GRAM, L>(P, gram_smem, red, is_last);
+  pass_body<B, MODE, false, GRAM, L>(P, gram_smem, red, is_last);
 }
 
 // Lanes per thread of the single-matrix odd and even passes: 4 (a whole
@@ -1026,7 +1026,7 @@ __device__ bool grid_barrier(unsigned int* bar, int* error, uint64_t limit_ns, u
 // over the stacked rows of A, grid barrier, pass over the rows of A^T, grid
 // barrier.  The blocks are read with coherent loads (they change between
 // barriers); the Gram partials go to the per-(matrix, term) slots.
-template <int B, int FE, int L>
+template <int B, int L>
 __global__ void __launch_bounds__(kThreads, (B >= 32 ? 2 : 4)) persistent_kernel(PersistParams Q) {
   extern __shared__ __align__(16) uint32_t gram_smem[];
   __shared__ unsigned long long red[B * (B + 1) / 2];
@@ -1037,13 +1037,13 @@ __global__ void __launch_bounds__(kThreads, (B >= 32 ? 2 : 4)) persistent_kernel
     P.X = Q.X[cur];
     P.Y = Q.U;
     P.term = 2 * t + 1;
-    pass_body<B, kModeOdd, FE, true, true, L>(P, gram_smem, red, is_last);
+    pass_body<B, kModeOdd, true, kGramOwn, L>(P, gram_smem, red, is_last);
     if (!grid_barrier(Q.bar, Q.error, Q.limit_ns, gridDim.x)) return;
     P = Q.even;
     P.X = Q.U;
     P.Y = Q.X[cur ^ 1];
     P.term = 2 * t + 2;
-    pass_body<B, kModeEven, FE, true, true, L>(P, gram_smem, red, is_last);
+    pass_body<B, kModeEven, true, kGramOwn, L>(P, gram_smem, red, is_last);
     if (!grid_barrier(Q.bar, Q.error, Q.limit_ns, gridDim.x)) return;
     cur ^= 1;
   }
@@ -1068,7 +1068,7 @@ __global__ void barrier_check_kernel(unsigned int* bar, int* error, uint64_t lim
 template <int B>
 constexpr int kChunkLpt = (B >= 16) ? 4 : kDefaultLpt<B>;
 
-template <int B, int FE, int L = kChunkLpt<B>>
+template <int B, int L = kChunkLpt<B>>
 __global__ void __launch_bounds__(kThreads, 3) chunk_kernel(ChunkParams P) {
   using S = Shape<B, L>;
   constexpr int LPT = S::LPT, TPR = S::TPR, RPW = S::RPW;
@@ -1096,9 +1096,9 @@ __global__ void __launch_bounds__(kThreads, 3) chunk_kernel(ChunkParams P) {
 #pragma unroll
     for (int l = 0; l < LPT; ++l) acc[l] = 0;
     if constexpr (L == 4 && B >= 16)
-      gather_sum8<B, FE, L>(P.cv, beg + slot, end, (uint32_t)RPW, P.X, sub, M, acc);
+      gather_sum8<B, L>(P.cv, beg + slot, end, (uint32_t)RPW, P.X, sub, M, acc);
     else
-      gather_sum<B, FE, false, L>(P.cv, beg + slot, end, (uint32_t)RPW, P.X, sub, M, acc);
+      gather_sum<B, false, L>(P.cv, beg + slot, end, (uint32_t)RPW, P.X, sub, M, acc);
     uint32_t y[LPT];
 #pragma unroll
     for (int l = 0; l < LPT; ++l) y[l] = reduce(acc[l], M);
@@ -1178,14 +1178,14 @@ int launch_batch_finalize(cudaStream_t s, const unsigned long long* gram_all, co
 // memory is L1 for their gathers.
 template <int B, bool SYM = false>
 constexpr size_t pass_smem_bytes() {
-  if (B >= 8) return (size_t)kWarps * 4 * (SYM ? GramMma<B, 4>::kWordsSym : GramMma<B, 4>::kWords);
-  return (size_t)kWarps * 4 * GramCore<B, 4>::kWords;
+  if (B >= 8) return (size_t)kWarps * 4 * (SYM ? GramMma<B>::kWordsSym : GramMma<B>::kWords);
+  return (size_t)kWarps * 4 * GramCore<B>::kWords;
 }
 
 // of the even pass that forms both terms
 template <int B>
 constexpr size_t both_smem_bytes() {
-  return (size_t)kWarps * 4 * GramDual<B, 4>::kWords;
+  return (size_t)kWarps * 4 * GramDual<B>::kWords;
 }
 
 // CTAs for a pass over `rows` rows: the resident maximum, but no more CTAs
@@ -1242,18 +1242,18 @@ static int launch_ex(const rr_krylov* kr, void (*fn)(Args...), dim3 grid, dim3 b
 // is lean (no Gram staging, no tensor-core flush, so fewer registers and no
 // shared memory); so is the even pass at widths 16 and 32, whose two terms
 // follow in a Gram pass (kModeGram), while at widths 4 and 8 it adds both.
-template <int B, int FE>
-static int launch_pass_BF(rr_krylov* kr, const PassParams& P, int mode, dim3 grid, cudaStream_t s) {
+template <int B>
+static int launch_pass_kernel(rr_krylov* kr, const PassParams& P, int mode, dim3 grid, cudaStream_t s) {
   const dim3 block(kThreads);
   switch (mode) {
     case kModeInit:
-      return launch_ex(kr, pass_kernel<B, kModeInit, FE>, grid, block, pass_smem_bytes<B, true>(), s, P);
+      return launch_ex(kr, pass_kernel<B, kModeInit>, grid, block, pass_smem_bytes<B, true>(), s, P);
     case kModeOdd:
-      return launch_ex(kr, pass_kernel<B, kModeOdd, FE, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
+      return launch_ex(kr, pass_kernel<B, kModeOdd, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
     case kModeEven:
       if constexpr (kGramInPass<B>)
-        return launch_ex(kr, pass_kernel<B, kModeEven, FE, kGramBoth>, grid, block, both_smem_bytes<B>(), s, P);
-      else return launch_ex(kr, pass_kernel<B, kModeEven, FE, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
+        return launch_ex(kr, pass_kernel<B, kModeEven, kGramBoth>, grid, block, both_smem_bytes<B>(), s, P);
+      else return launch_ex(kr, pass_kernel<B, kModeEven, kGramNone, kLeanLpt<B>>, grid, block, (size_t)0, s, P);
   }
   return fail(RR_EINVAL, "pass mode %d has no pass kernel at width %d", mode, B);
 }
@@ -1278,16 +1278,7 @@ static int launch_pass_B(rr_krylov* kr, const PassParams& P, int mode) {
   const bool lean = mode == kModeOdd || (mode == kModeEven && !kGramInPass<B>);
   const dim3 grid(lean ? pass_grid_lean<B>(kr, P.rows) : pass_grid<B>(kr, P.rows));
   cudaStream_t s = kr->launch_stream ? kr->launch_stream : kr->mat->ctx->stream;
-  return kr->fold4 ? launch_pass_BF<B, 4>(kr, P, mode, grid, s) : launch_pass_BF<B, 2>(kr, P, mode, grid, s);
-}
-
-template <int B, int FE>
-static int set_pass_smem() {
-  const int sm = (int)pass_smem_bytes<B>();
-  RR_CUDA(cudaFuncSetAttribute(pass_kernel<B, kModeInit, FE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  RR_CUDA(cudaFuncSetAttribute(pass_kernel<B, kModeOdd, FE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  RR_CUDA(cudaFuncSetAttribute(pass_kernel<B, kModeEven, FE>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  return RR_OK;
+  return launch_pass_kernel<B>(kr, P, mode, grid, s);
 }
 
 static int launch_pass(rr_krylov* kr, const PassParams& P, int mode) {
@@ -1306,8 +1297,7 @@ static int launch_chunk_B(rr_krylov* kr, const ChunkParams& P) {
   const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(kr->grid_chunk, (P.nchunks + kWarps - 1) / kWarps))),
       block(kThreads);
   cudaStream_t s = kr->launch_stream ? kr->launch_stream : kr->mat->ctx->stream;
-  if (kr->fold4) return launch_ex(kr, chunk_kernel<B, 4>, grid, block, 0, s, P);
-  return launch_ex(kr, chunk_kernel<B, 2>, grid, block, 0, s, P);
+  return launch_ex(kr, chunk_kernel<B>, grid, block, 0, s, P);
 }
 
 static int launch_chunk(rr_krylov* kr, const ChunkParams& P) {
@@ -1322,71 +1312,58 @@ static int launch_chunk(rr_krylov* kr, const ChunkParams& P) {
 }
 
 template <int B>
-static int occupancy_B(rr_krylov* kr, int* pass_blocks, int* chunk_blocks, int* lean_blocks) {
-  const size_t sm = pass_smem_bytes<B>();
-  if (kr->fold4) {
-    RR_TRY((set_pass_smem<B, 4>()));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(pass_blocks, pass_kernel<B, kModeOdd, 4>, kThreads, sm));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(chunk_blocks, chunk_kernel<B, 4>, kThreads, 0));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 4, kGramNone, kLeanLpt<B>>,
-                                                          kThreads, 0));
-  } else {
-    RR_TRY((set_pass_smem<B, 2>()));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(pass_blocks, pass_kernel<B, kModeOdd, 2>, kThreads, sm));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(chunk_blocks, chunk_kernel<B, 2>, kThreads, 0));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(lean_blocks, pass_kernel<B, kModeOdd, 2, kGramNone, kLeanLpt<B>>,
-                                                          kThreads, 0));
-  }
+static int init_blocks_B(int* blocks) {
+  constexpr size_t sm = pass_smem_bytes<B, true>();
+  RR_CUDA(cudaFuncSetAttribute(pass_kernel<B, kModeInit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, pass_kernel<B, kModeInit>, kThreads, sm));
+  return RR_OK;
+}
+
+// Resident CTAs per SM: of the pass with Gram work (the even one at widths up to
+// 8, else only the initial one), of the lean passes and of the chunk kernel.
+template <int B>
+static int occupancy_B(int* pass_blocks, int* chunk_blocks, int* lean_blocks) {
+  RR_TRY(init_blocks_B<B>(pass_blocks));
+  if constexpr (kGramInPass<B>)
+    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(pass_blocks, pass_kernel<B, kModeEven, kGramBoth>, kThreads,
+                                                          both_smem_bytes<B>()));
+  RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(chunk_blocks, chunk_kernel<B>, kThreads, 0));
+  RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      lean_blocks, pass_kernel<B, kModeOdd, kGramNone, kLeanLpt<B>>, kThreads, 0));
   return RR_OK;
 }
 
 template <int B>
-static int launch_pass_raw_B(cudaStream_t s, int fold4, int grid, const PassParams& P, int mode) {
-  const size_t sm = pass_smem_bytes<B>();
-  const dim3 g(grid), block(kThreads);
-  if (fold4) {
-    if (mode == kModeInit) pass_kernel<B, kModeInit, 4><<<g, block, sm, s>>>(P);
-    else if (mode == kModeOdd) pass_kernel<B, kModeOdd, 4><<<g, block, sm, s>>>(P);
-    else pass_kernel<B, kModeEven, 4><<<g, block, sm, s>>>(P);
-  } else {
-    if (mode == kModeInit) pass_kernel<B, kModeInit, 2><<<g, block, sm, s>>>(P);
-    else if (mode == kModeOdd) pass_kernel<B, kModeOdd, 2><<<g, block, sm, s>>>(P);
-    else pass_kernel<B, kModeEven, 2><<<g, block, sm, s>>>(P);
-  }
+static int launch_init_B(cudaStream_t s, int grid, const PassParams& P) {
+  pass_kernel<B, kModeInit><<<dim3(grid), dim3(kThreads), pass_smem_bytes<B, true>(), s>>>(P);
   RR_CUDA(cudaGetLastError());
   return RR_OK;
 }
 
-int launch_pass_raw(cudaStream_t s, int B, int fold4, int grid, const PassParams& P, int mode) {
+int launch_init_raw(cudaStream_t s, int B, int grid, const PassParams& P) {
   switch (B) {
-    case 4: return launch_pass_raw_B<4>(s, fold4, grid, P, mode);
-    case 8: return launch_pass_raw_B<8>(s, fold4, grid, P, mode);
-    case 16: return launch_pass_raw_B<16>(s, fold4, grid, P, mode);
-    case 32: return launch_pass_raw_B<32>(s, fold4, grid, P, mode);
+    case 4: return launch_init_B<4>(s, grid, P);
+    case 8: return launch_init_B<8>(s, grid, P);
+    case 16: return launch_init_B<16>(s, grid, P);
+    case 32: return launch_init_B<32>(s, grid, P);
   }
   return fail(RR_EINVAL, "unsupported padded block width %d", B);
 }
 
 template <int B, int L>
-static int launch_persistent_BL(cudaStream_t s, int fold4, int grid, PersistParams& Q) {
-  const size_t sm = pass_smem_bytes<B>();
+static int launch_persistent_BL(cudaStream_t s, int grid, PersistParams& Q) {
   void* args[] = {&Q};
   // the shared-memory limit was raised by persistent_blocks_per_sm at set-up
-  const void* fn = fold4 ? (const void*)persistent_kernel<B, 4, L> : (const void*)persistent_kernel<B, 2, L>;
-  RR_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, sm, s));
+  RR_CUDA(cudaLaunchCooperativeKernel((const void*)persistent_kernel<B, L>, dim3(grid), dim3(kThreads), args,
+                                      pass_smem_bytes<B>(), s));
   return RR_OK;
 }
 
 template <int B, int L>
-static int persistent_blocks_BL(int fold4, int* blocks) {
+static int persistent_blocks_BL(int* blocks) {
   const size_t sm = pass_smem_bytes<B>();
-  if (fold4) {
-    RR_CUDA(cudaFuncSetAttribute(persistent_kernel<B, 4, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, persistent_kernel<B, 4, L>, kThreads, sm));
-  } else {
-    RR_CUDA(cudaFuncSetAttribute(persistent_kernel<B, 2, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, persistent_kernel<B, 2, L>, kThreads, sm));
-  }
+  RR_CUDA(cudaFuncSetAttribute(persistent_kernel<B, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, persistent_kernel<B, L>, kThreads, sm));
   return RR_OK;
 }
 
@@ -1401,28 +1378,28 @@ int persistent_lane_options(int B, int* opts) {
   return 2;
 }
 
-int launch_persistent_raw(cudaStream_t s, int B, int fold4, int grid, int lpt, PersistParams& Q) {
+int launch_persistent_raw(cudaStream_t s, int B, int grid, int lpt, PersistParams& Q) {
   switch (B * 100 + lpt) {
-    case 404: return launch_persistent_BL<4, 4>(s, fold4, grid, Q);
-    case 804: return launch_persistent_BL<8, 4>(s, fold4, grid, Q);
-    case 808: return launch_persistent_BL<8, 8>(s, fold4, grid, Q);
-    case 1604: return launch_persistent_BL<16, 4>(s, fold4, grid, Q);
-    case 1608: return launch_persistent_BL<16, 8>(s, fold4, grid, Q);
-    case 3204: return launch_persistent_BL<32, 4>(s, fold4, grid, Q);
-    case 3208: return launch_persistent_BL<32, 8>(s, fold4, grid, Q);
+    case 404: return launch_persistent_BL<4, 4>(s, grid, Q);
+    case 804: return launch_persistent_BL<8, 4>(s, grid, Q);
+    case 808: return launch_persistent_BL<8, 8>(s, grid, Q);
+    case 1604: return launch_persistent_BL<16, 4>(s, grid, Q);
+    case 1608: return launch_persistent_BL<16, 8>(s, grid, Q);
+    case 3204: return launch_persistent_BL<32, 4>(s, grid, Q);
+    case 3208: return launch_persistent_BL<32, 8>(s, grid, Q);
   }
   return fail(RR_EINVAL, "no persistent kernel for width %d and %d lanes per thread", B, lpt);
 }
 
-int persistent_blocks_per_sm(int B, int fold4, int lpt, int* blocks) {
+int persistent_blocks_per_sm(int B, int lpt, int* blocks) {
   switch (B * 100 + lpt) {
-    case 404: return persistent_blocks_BL<4, 4>(fold4, blocks);
-    case 804: return persistent_blocks_BL<8, 4>(fold4, blocks);
-    case 808: return persistent_blocks_BL<8, 8>(fold4, blocks);
-    case 1604: return persistent_blocks_BL<16, 4>(fold4, blocks);
-    case 1608: return persistent_blocks_BL<16, 8>(fold4, blocks);
-    case 3204: return persistent_blocks_BL<32, 4>(fold4, blocks);
-    case 3208: return persistent_blocks_BL<32, 8>(fold4, blocks);
+    case 404: return persistent_blocks_BL<4, 4>(blocks);
+    case 804: return persistent_blocks_BL<8, 4>(blocks);
+    case 808: return persistent_blocks_BL<8, 8>(blocks);
+    case 1604: return persistent_blocks_BL<16, 4>(blocks);
+    case 1608: return persistent_blocks_BL<16, 8>(blocks);
+    case 3204: return persistent_blocks_BL<32, 4>(blocks);
+    case 3208: return persistent_blocks_BL<32, 8>(blocks);
   }
   return fail(RR_EINVAL, "no persistent kernel for width %d and %d lanes per thread", B, lpt);
 }
@@ -1434,25 +1411,12 @@ int launch_barrier_check(cudaStream_t s, int grid, unsigned int* bar, int* error
   return RR_OK;
 }
 
-template <int B>
-static int pass_blocks_B(int fold4, int* blocks) {
-  const size_t sm = pass_smem_bytes<B>();
-  if (fold4) {
-    RR_TRY((set_pass_smem<B, 4>()));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, pass_kernel<B, kModeEven, 4>, kThreads, sm));
-  } else {
-    RR_TRY((set_pass_smem<B, 2>()));
-    RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, pass_kernel<B, kModeEven, 2>, kThreads, sm));
-  }
-  return RR_OK;
-}
-
-int pass_blocks_per_sm(int B, int fold4, int* blocks) {
+int init_blocks_per_sm(int B, int* blocks) {
   switch (B) {
-    case 4: return pass_blocks_B<4>(fold4, blocks);
-    case 8: return pass_blocks_B<8>(fold4, blocks);
-    case 16: return pass_blocks_B<16>(fold4, blocks);
-    case 32: return pass_blocks_B<32>(fold4, blocks);
+    case 4: return init_blocks_B<4>(blocks);
+    case 8: return init_blocks_B<8>(blocks);
+    case 16: return init_blocks_B<16>(blocks);
+    case 32: return init_blocks_B<32>(blocks);
   }
   return fail(RR_EINVAL, "unsupported padded block width %d", B);
 }
@@ -1471,10 +1435,10 @@ int krylov_occupancy(rr_krylov* kr) {
                                  (int)gram_tc_smem_bytes<32>()));
   int pb = 1, cb = 1, lb = 1;
   switch (kr->B) {
-    case 4: RR_TRY(occupancy_B<4>(kr, &pb, &cb, &lb)); break;
-    case 8: RR_TRY(occupancy_B<8>(kr, &pb, &cb, &lb)); break;
-    case 16: RR_TRY(occupancy_B<16>(kr, &pb, &cb, &lb)); break;
-    case 32: RR_TRY(occupancy_B<32>(kr, &pb, &cb, &lb)); break;
+    case 4: RR_TRY(occupancy_B<4>(&pb, &cb, &lb)); break;
+    case 8: RR_TRY(occupancy_B<8>(&pb, &cb, &lb)); break;
+    case 16: RR_TRY(occupancy_B<16>(&pb, &cb, &lb)); break;
+    case 32: RR_TRY(occupancy_B<32>(&pb, &cb, &lb)); break;
     default: return fail(RR_EINVAL, "unsupported padded block width %d", kr->B);
   }
   const int sms = kr->mat->ctx->num_sms;

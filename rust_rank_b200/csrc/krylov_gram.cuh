@@ -45,7 +45,7 @@ __device__ __forceinline__ int pair_index(int i, int j, int B) { return i * B - 
 
 // CUDA cores (B = 4): the batch is staged in shared memory and every lane
 // accumulates a few (i, j) pairs over the staged rows.
-template <int B, int FE, int L = kDefaultLpt<B>>
+template <int B, int L = kDefaultLpt<B>>
 struct GramCore {
   static constexpr int LPT = Shape<B, L>::LPT, RPW = Shape<B, L>::RPW;
   static constexpr int NP = B * (B + 1) / 2, PPL = (NP + 31) / 32;
@@ -83,7 +83,7 @@ struct GramCore {
 #pragma unroll
         for (int rr = 0; rr < RPW; ++rr) {
           a = mad_wide(zs[rr * B + i], us[rr * B + j], a);
-          if ((rr % FE) == FE - 1) a = fold(a, M);
+          if ((rr % kFold) == kFold - 1) a = fold(a, M);
         }
         acc[t] = a;
       }
@@ -135,7 +135,7 @@ __device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint
 // pair's product is < 32 * 255^2 < 2^21, so the shift classes s = a + c stay
 // exact in int32; classes 0..3 are recombined exactly in 64 bits (< 2^48) and
 // classes 4..6 are added with their weights 2^{8s} mod p.
-template <int B, int FE, int L = kDefaultLpt<B>>
+template <int B, int L = kDefaultLpt<B>>
 struct GramMma {
   static constexpr int LPT = Shape<B, L>::LPT, TPR = Shape<B, L>::TPR, RPW = Shape<B, L>::RPW;
   static constexpr int TB = 32 / RPW;           // batches per K tile
@@ -328,12 +328,12 @@ struct GramMma {
 // term w' (x) w' and the odd term w (x) w' (w the block before the application),
 // which together need one set of operands: no Gram work and no second block of
 // multiply-adds in the odd pass.  Sums: [0, NP) odd, [NP, 2 NP) even.
-template <int B, int FE, int L = kDefaultLpt<B>>
+template <int B, int L = kDefaultLpt<B>>
 struct GramDual;
 
 // B = 4: the lanes take the 10 pairs of either term.
-template <int FE>
-struct GramDual<4, FE, 4> {
+template <>
+struct GramDual<4, 4> {
   static constexpr int B = 4, RPW = 32, NP = 10;
   static constexpr int kWords = 2 * RPW * B;
   uint32_t *zs, *us;  // rows of w' and of w
@@ -360,7 +360,7 @@ struct GramDual<4, FE, 4> {
 #pragma unroll
       for (int rr = 0; rr < RPW; ++rr) {
         acc = mad_wide(a[rr * B + pi], zs[rr * B + pj], acc);
-        if ((rr % FE) == FE - 1) acc = fold(acc, M);
+        if ((rr % kFold) == kFold - 1) acc = fold(acc, M);
       }
     }
     __syncwarp();
@@ -370,19 +370,15 @@ struct GramDual<4, FE, 4> {
   __device__ __forceinline__ void emit(unsigned long long* red, int lane, const ModP& M) {
     if (lane < 2 * NP) atomicAdd(&red[lane], (unsigned long long)reduce(acc, M));
   }
-  // the warp's sums as residues, part[pair or NP + pair]
-  __device__ __forceinline__ void store(uint32_t* part, int lane, const ModP& M) {
-    if (lane < 2 * NP) part[lane] = reduce(acc, M);
-  }
 };
 
 // B = 8 on the tensor cores: the 16 rows of an MMA's A operand are the 8 lanes
 // of w' and the 8 of w, so both terms take the products of one.
-template <int FE>
-struct GramDual<8, FE, 4> {
+template <>
+struct GramDual<8, 4> {
   static constexpr int B = 8, LPT = 4, TPR = 2, RPW = 16, TB = 2, RS = 9, NP = 36;
   static constexpr int kWords = 4 * 16 * RS;
-  using Single = GramMma<8, FE, 4>;
+  using Single = GramMma<8, 4>;
   uint32_t* pl;  // planes [limb][w' lanes 0..7, w lanes 8..15][RS]
   unsigned long long acc[4];
   int bt;
@@ -462,12 +458,6 @@ struct GramDual<8, FE, 4> {
       const int j = j0 + (v & 1);
       if (i <= j) atomicAdd(&red[(v < 2 ? NP : 0) + pair_index(i, j, B)], (unsigned long long)reduce(acc[v], M));
     }
-  }
-  // the warp's sums as residues, part[term][i * B + j] for i <= j (others undefined)
-  __device__ __forceinline__ void store(uint32_t* part, int lane, const ModP& M) {
-    const int e = (lane >> 2) * B + 2 * (lane & 3);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) part[(v < 2 ? B * B : 0) + e + (v & 1)] = reduce(acc[v], M);
   }
 };
 

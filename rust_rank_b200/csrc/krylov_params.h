@@ -87,9 +87,9 @@ struct PersistParams {
   uint64_t limit_ns;
 };
 // lpt: lanes of the block per thread (4 or 8; persistent_lane_options).
-int launch_persistent_raw(cudaStream_t s, int B, int fold4, int grid, int lpt, PersistParams& Q);
+int launch_persistent_raw(cudaStream_t s, int B, int grid, int lpt, PersistParams& Q);
 // Largest co-resident CTAs per SM of the persistent kernel (sets its shared-memory limit).
-int persistent_blocks_per_sm(int B, int fold4, int lpt, int* blocks);
+int persistent_blocks_per_sm(int B, int lpt, int* blocks);
 // The lanes-per-thread variants of the persistent kernel at padded width B
 // (into opts[2]); returns their count.
 int persistent_lane_options(int B, int* opts);
@@ -102,10 +102,10 @@ int launch_barrier_check(cudaStream_t s, int grid, unsigned int* bar, int* error
 int launch_batch_finalize(cudaStream_t s, const unsigned long long* gram_all, const int64_t* d_seg_G_off,
                           uint32_t* S_all, const int64_t* d_seg_S_off, const int64_t* d_seg_terms, int seg_begin,
                           int seg_end, int64_t max_terms, int b, int B, const ModP& M);
-// Launch one pass kernel for padded width B on stream s (grid = CTAs).
-int launch_pass_raw(cudaStream_t s, int B, int fold4, int grid, const PassParams& P, int mode);
-// CTAs per SM of the pass kernel for padded width B (also sets its shared-memory limit).
-int pass_blocks_per_sm(int B, int fold4, int* blocks);
+// Launch the initial pass for padded width B on stream s (grid = CTAs).
+int launch_init_raw(cudaStream_t s, int B, int grid, const PassParams& P);
+// CTAs per SM of the initial pass for padded width B (also sets its shared-memory limit).
+int init_blocks_per_sm(int B, int* blocks);
 // Rows per warp batch for padded width B with lpt lanes per thread (0: the
 // default shape of the pass kernels).
 int rows_per_batch(int B, int lpt = 0);

@@ -774,7 +774,7 @@ __device__ __forceinline__ void leaf_select(LeafParams& P) {
   P.sigma_inv += (int64_t)z * P.m;
 }
 
-template <int CT, int FE>
+template <int CT>
 __global__ void __launch_bounds__(kLeafThreads) pm_leaves_kernel(LeafParams P) {
   leaf_select(P);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -916,9 +916,9 @@ __global__ void __launch_bounds__(kLeafThreads) pm_leaves_kernel(LeafParams P) {
 #pragma unroll
           for (int v = 0; v < CT; ++v) acc[r][v] = 0;
         int s = 0;
-        for (; s + FE <= m; s += FE) {
+        for (; s + kFold <= m; s += kFold) {
 #pragma unroll
-          for (int u = 0; u < FE; ++u) {
+          for (int u = 0; u < kFold; ++u) {
             const uint4 wv = *reinterpret_cast<const uint4*>(w);
             uint32_t xv[CT];
             if (CT == 4) {
@@ -980,7 +980,6 @@ __global__ void __launch_bounds__(kLeafThreads) pm_leaves_kernel(LeafParams P) {
 // Mout[i][j][t] = V_K[t][i] sigma_inv[i].  Rows are taken in the grouped slot
 // order of the leaves kernel, four per thread, so the four rows of a thread
 // read one source coefficient.
-template <int FE>
 __global__ void __launch_bounds__(256) pm_block_basis_kernel(const uint32_t* __restrict__ Tt,
                                                              const unsigned long long* __restrict__ mask,
                                                              const uint32_t* __restrict__ sigma_inv, int m, int K,
@@ -1026,9 +1025,9 @@ __global__ void __launch_bounds__(256) pm_block_basis_kernel(const uint32_t* __r
         const uint32_t* w = Ts + q0;
         const uint32_t* x = Vc + st * S;
         int s = 0;
-        for (; s + FE <= m; s += FE) {
+        for (; s + kFold <= m; s += kFold) {
 #pragma unroll
-          for (int u = 0; u < FE; ++u) {
+          for (int u = 0; u < kFold; ++u) {
             const uint4 wv = *reinterpret_cast<const uint4*>(w);
             const uint32_t xv = x[s + u];
             acc[0] = mad_wide(wv.x, xv, acc[0]);
@@ -1091,8 +1090,7 @@ int grid_for(int64_t work, int threads = 256) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, 148 * 32));
 }
 
-// An NTT prime q with its twiddle tables (forward and inverse, nmax entries)
-// and the pointwise stage's fold rule.
+// An NTT prime q with its twiddle tables (forward and inverse, nmax entries).
 struct NttPrime {
   uint32_t q = 0;
   ModP M{};
@@ -1101,14 +1099,6 @@ struct NttPrime {
   const uint2* fwd() const { return tw.ptr; }
   const uint2* inv() const { return twi.ptr; }
 };
-
-// Four products fit between folds of a 64-bit accumulator iff
-// (2^32 - 1) * c32 + 2^32 - 1 + 4 (q - 1)^2 < 2^64.
-int fold4_ok(uint32_t q, const ModP& M) {
-  const unsigned __int128 F = (unsigned __int128)0xffffffffull * M.c32 + 0xffffffffull;
-  const unsigned __int128 sq = (unsigned __int128)(q - 1) * (q - 1);
-  return (F + 4 * sq) < ((unsigned __int128)1 << 64);
-}
 
 // The three largest NTT primes below 2^31 (2-adic orders 27, 25, 24): the
 // exact-integer products of primes without a suitable NTT are taken modulo
@@ -1138,7 +1128,6 @@ struct Pm {
   DevBuf<int64_t> delta;                // [nb][m]
   DevBuf<int> status;
   int64_t cs = 0;                      // residual coefficient stride of the leaves kernel (words)
-  int fold4 = 0;
   int64_t direct = 0;                  // levels up to this half length take direct products
   uint64_t wait_ns = 0;                // of the leaf blocks (rr_ctx_set_waits)
   int wait_missing = 0;
@@ -1336,26 +1325,15 @@ int run_base(Pm& P, MatView G, int nleaves, MatView Mout) {
   L.M = P.M;
   L.status = P.status.ptr;
   const unsigned nb = (unsigned)P.nb;
-  if (P.n % 4 == 0) {
-    const size_t smem = leaves_smem_bytes(P.m, P.n, nleaves, P.cs);
-    if (P.fold4) pm_leaves_kernel<4, 4><<<nb, kLeafThreads, smem, P.s>>>(L);
-    else pm_leaves_kernel<4, 2><<<nb, kLeafThreads, smem, P.s>>>(L);
-  } else {
-    const size_t smem = leaves_smem_bytes(P.m, P.n, nleaves, P.cs);
-    if (P.fold4) pm_leaves_kernel<1, 4><<<nb, kLeafThreads, smem, P.s>>>(L);
-    else pm_leaves_kernel<1, 2><<<nb, kLeafThreads, smem, P.s>>>(L);
-  }
+  const size_t smem = leaves_smem_bytes(P.m, P.n, nleaves, P.cs);
+  if (P.n % 4 == 0) pm_leaves_kernel<4><<<nb, kLeafThreads, smem, P.s>>>(L);
+  else pm_leaves_kernel<1><<<nb, kLeafThreads, smem, P.s>>>(L);
   RR_CUDA(cudaGetLastError());
   // the leaves kernel indexes its transforms with the block's own K; the
   // block basis reads them with the same K
   const dim3 grid((unsigned)P.m, nb);
-  const size_t bsm = block_basis_smem_bytes(P.m, nleaves);
-  if (P.fold4)
-    pm_block_basis_kernel<4><<<grid, 256, bsm, P.s>>>(P.Tt.ptr, P.leafmask.ptr, P.sigma_inv.ptr, P.m, nleaves, Mout.p,
-                                                      Mout.rs, Mout.cs, Mout.bs, P.M);
-  else
-    pm_block_basis_kernel<2><<<grid, 256, bsm, P.s>>>(P.Tt.ptr, P.leafmask.ptr, P.sigma_inv.ptr, P.m, nleaves, Mout.p,
-                                                      Mout.rs, Mout.cs, Mout.bs, P.M);
+  pm_block_basis_kernel<<<grid, 256, block_basis_smem_bytes(P.m, nleaves), P.s>>>(
+      P.Tt.ptr, P.leafmask.ptr, P.sigma_inv.ptr, P.m, nleaves, Mout.p, Mout.rs, Mout.cs, Mout.bs, P.M);
   RR_CUDA(cudaGetLastError());
   return RR_OK;
 }
@@ -1378,12 +1356,9 @@ int pick_block_leaves(int m, int n, int64_t d, size_t* smem) {
 
 int set_leaves_smem_limit(size_t bytes, size_t basis_bytes) {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<4, 4>, attr, (int)bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<4, 2>, attr, (int)bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<1, 4>, attr, (int)bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<1, 2>, attr, (int)bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_block_basis_kernel<4>, attr, (int)basis_bytes));
-  RR_CUDA(cudaFuncSetAttribute(pm_block_basis_kernel<2>, attr, (int)basis_bytes));
+  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<4>, attr, (int)bytes));
+  RR_CUDA(cudaFuncSetAttribute(pm_leaves_kernel<1>, attr, (int)bytes));
+  RR_CUDA(cudaFuncSetAttribute(pm_block_basis_kernel, attr, (int)basis_bytes));
   return RR_OK;
 }
 
@@ -1446,7 +1421,6 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   P.mma = ctx->pm_tensor_cores;
   P.K = P.mma ? (int)std::min<int64_t>(d, leaf_block_max(P.m)) : pick_block_leaves(P.m, P.n, d, &leaves_smem);
   P.cs = leaf_coeff_stride(P.m, P.n);
-  P.fold4 = fold4_ok(p, P.M);
   const int m = P.m, n = P.n;
   // the largest transform: length 2h = d
   const int64_t nmax = std::max<int64_t>(d, 2);

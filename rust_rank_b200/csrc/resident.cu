@@ -242,7 +242,7 @@ __device__ __forceinline__ void res_gram(Gram& gram, int64_t rows, int count, co
 }
 
 template <int B>
-using ResGram = typename std::conditional<(B >= 8), GramMma<B, 4, 4>, GramCore<B, 4, 4>>::type;
+using ResGram = typename std::conditional<(B >= 8), GramMma<B, 4>, GramCore<B, 4>>::type;
 
 template <int B>
 constexpr size_t res_fixed_smem() {  // Gram staging, the Gram warps' sums, batch offsets

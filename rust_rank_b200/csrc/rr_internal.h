@@ -193,7 +193,6 @@ struct rr_krylov_s {
   int b = 0;   // real block width
   int B = 0;   // padded width (4, 8, 16, 32)
   rr::ModP M{};
-  int fold4 = 0;  // 1 when four products fit between folds
   // preconditioners in device order, in the forms the epilogues use:
   // d_r R^2, d_c R^2, d_c R (mod p, R = 2^32), d_c^{-1}, and the Gram passes'
   // d_r^{-1} R and d_c^{-1} R

@@ -24,6 +24,12 @@ struct ModP {
 // mad.lo.cc / madc.hi pair takes 5.0 (CUDA 12.9, B200).
 __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)a * b + c; }
 
+// Products of residues that fit a 64-bit accumulator between two folds, for every
+// p < 2^31.  A folded accumulator is below 2^32 (c32 + 1).  For p = 2^31 - e > 2^32 / 3,
+// c32 = 2e and 4 (p - 1)^2 = 2^64 - 2^32 (4e + 4) + (2e + 2)^2, together below 2^64
+// because (2e + 2)^2 < 2^32 (2e + 3); for smaller p, 4 p^2 <= 4/9 2^64 and c32 < p.
+constexpr int kFold = 4;
+
 // Fold a 64-bit accumulator: result == x (mod p) and result < 2^32 * c32 + 2^32.
 // Here the carry chain wins (mad_wide and fold of one accumulator 10.2 cycles
 // against 11.8): the addend is half an accumulator, which the wide form has to
