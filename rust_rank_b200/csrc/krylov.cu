@@ -543,7 +543,6 @@ constexpr bool kGramInPass = B <= 8;
 constexpr int kTcDrain = 64;        // tiles between drains of the int32 accumulators
 constexpr uint64_t kTcWaitLimitNs = 2000000000ull;  // 2 s of %globaltimer
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // K-major, no swizzle: start >> 4, LBO = 128 B (K-direction core stride),
 // SBO = 256 B (8-row group stride), descriptor version 1 (sm_100).
@@ -566,12 +565,6 @@ __device__ __forceinline__ uint32_t tc_off(int R, int row, int k) {
   return (uint32_t)((k >> 5) * (R / 8) * 256 + (row >> 3) * 256 + ((k & 31) >> 4) * 128 + (row & 7) * 16 + (k & 15));
 }
 
-__device__ __forceinline__ uint64_t tc_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
   uint32_t done;
   asm volatile(
@@ -587,18 +580,18 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
 // Waits read the timer only once a try has failed.
 __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
   if (mbar_try(addr, parity)) return true;
-  const uint64_t t0 = tc_ns();
+  const uint64_t t0 = now_ns();
   while (!mbar_try(addr, parity))
-    if (tc_ns() - t0 > kTcWaitLimitNs) return false;
+    if (now_ns() - t0 > kTcWaitLimitNs) return false;
   return true;
 }
 
 // A bounded wait that also ends when another role of the CTA gave up.
 __device__ __forceinline__ bool mbar_wait_or(uint32_t addr, uint32_t parity, const volatile int* abort) {
   if (mbar_try(addr, parity)) return true;
-  const uint64_t t0 = tc_ns();
+  const uint64_t t0 = now_ns();
   while (!mbar_try(addr, parity))
-    if (*abort || tc_ns() - t0 > kTcWaitLimitNs) return false;
+    if (*abort || now_ns() - t0 > kTcWaitLimitNs) return false;
   return true;
 }
 
@@ -664,16 +657,6 @@ constexpr size_t gram_tc_smem_bytes() {
 static_assert(gram_tc_smem_bytes<16>() + 4 * TcShape<16>::SUMS + 512 <= 232448, "Gram stages too large");
 static_assert(gram_tc_smem_bytes<32>() + 4 * TcShape<32>::SUMS + 512 <= 232448, "Gram stages too large");
 
-__device__ __forceinline__ void byte_transpose4(const uint32_t (&v)[4], uint32_t (&w)[4]) {
-  // w[a] = bytes a of v[0..3]: limb a of four consecutive rows
-  const uint32_t t0 = __byte_perm(v[0], v[1], 0x5140), t1 = __byte_perm(v[2], v[3], 0x5140);
-  const uint32_t t2 = __byte_perm(v[0], v[1], 0x7362), t3 = __byte_perm(v[2], v[3], 0x7362);
-  w[0] = __byte_perm(t0, t1, 0x5410);
-  w[1] = __byte_perm(t0, t1, 0x7632);
-  w[2] = __byte_perm(t2, t3, 0x5410);
-  w[3] = __byte_perm(t2, t3, 0x7632);
-}
-
 // y * s * 2^-32 mod p without the final correction: a value in [0, 2p) < 2^32
 // congruent to the Montgomery product.  The Gram pass only needs the value
 // mod p (its limb products are exact for any 32-bit operand and its sums are
@@ -684,7 +667,7 @@ __device__ __forceinline__ uint32_t redc_lazy(uint32_t y, uint32_t s, const ModP
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 // Thread 0 of the producer: the rows of `tile` of both blocks and their scales
@@ -698,12 +681,12 @@ __device__ __forceinline__ void tc_fetch(const PassParams& P, int64_t tile, unsi
   const int rows = (int)(P.rows - r0 < T::TILE ? P.rows - r0 : T::TILE);
   const uint32_t ybytes = (uint32_t)rows * B * 4;
   const uint32_t sbytes = (uint32_t)((rows * 4 + 15) & ~15);
-  const uint32_t mb = smem_u32(mbar);
+  const uint32_t mb = smem_addr(mbar);
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(2 * ybytes + sbytes)
                : "memory");
   auto copy = [mb](unsigned char* to, const uint32_t* from, uint32_t bytes) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(to)),
+                     smem_addr(to)),
                  "l"(from), "r"(bytes), "r"(mb)
                  : "memory");
   };
@@ -734,7 +717,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     s_fail = 0;
     s_issued = 0;
     auto init = [](uint64_t* bar, int count) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
     };
     for (int i = 0; i < T::RING; ++i) {
       init(&raw_full[i], 1);
@@ -752,7 +735,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_s)),
                  "r"(T::COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -775,7 +758,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     if (lane == 0) {
       for (int64_t j = 0; j < mine; ++j) {
         const int slot = (int)(j % T::RING);
-        if (j >= T::RING && !mbar_wait_or(smem_u32(&raw_empty[slot]), (uint32_t)((j / T::RING - 1) & 1), &s_fail)) {
+        if (j >= T::RING && !mbar_wait_or(smem_addr(&raw_empty[slot]), (uint32_t)((j / T::RING - 1) & 1), &s_fail)) {
           give_up();
           break;
         }
@@ -791,16 +774,16 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
         const int64_t grp = j / kTcDrain;
         const int a = (int)(grp & 1);
         const bool first = j % kTcDrain == 0;
-        if (first && grp >= 2 && !mbar_wait_or(smem_u32(&acc_empty[a]), (uint32_t)((grp / 2 - 1) & 1), &s_fail)) {
+        if (first && grp >= 2 && !mbar_wait_or(smem_addr(&acc_empty[a]), (uint32_t)((grp / 2 - 1) & 1), &s_fail)) {
           give_up();
           break;
         }
-        if (!mbar_wait_or(smem_u32(&op_full[s]), (uint32_t)((j / T::OPS) & 1), &s_fail)) {
+        if (!mbar_wait_or(smem_addr(&op_full[s]), (uint32_t)((j / T::OPS) & 1), &s_fail)) {
           give_up();
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t b0 = smem_u32(tc_smem + s * T::STAGE), a0 = b0 + (T::A_ROW / 8) * 256;
+        const uint32_t b0 = smem_addr(tc_smem + s * T::STAGE), a0 = b0 + (T::A_ROW / 8) * 256;
 #pragma unroll
         for (int kb = 0; kb < T::TILE / 32; ++kb) {
           const uint64_t da = umma_desc(a0 + kb * (T::N / 8) * 256);
@@ -816,11 +799,11 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
               : "memory");
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_u32(&op_empty[s]))
+                         smem_addr(&op_empty[s]))
                      : "memory");
         if (j % kTcDrain == kTcDrain - 1 || j == mine - 1)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           smem_u32(&acc_full[a]))
+                           smem_addr(&acc_full[a]))
                        : "memory");
       }
     }
@@ -834,7 +817,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     const int64_t ngrp = (mine + kTcDrain - 1) / kTcDrain;
     for (int64_t G = 0; G < ngrp; ++G) {
       const int a = (int)(G & 1);
-      if (!mbar_wait_or(smem_u32(&acc_full[a]), (uint32_t)((G / 2) & 1), &s_fail)) {
+      if (!mbar_wait_or(smem_addr(&acc_full[a]), (uint32_t)((G / 2) & 1), &s_fail)) {
         give_up();
         break;
       }
@@ -874,7 +857,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
     const int gw = task % T::GROUPS, qd = task / T::GROUPS;  // word gw of rows 4 qd .. 4 qd + 3
     for (int64_t j = g; j < mine; j += T::NG) {
       const int slot = (int)(j % T::RING), s = (int)(j % T::OPS);
-      if (!mbar_wait_or(smem_u32(&raw_full[slot]), (uint32_t)((j / T::RING) & 1), &s_fail)) {
+      if (!mbar_wait_or(smem_addr(&raw_full[slot]), (uint32_t)((j / T::RING) & 1), &s_fail)) {
         give_up();
         break;
       }
@@ -891,7 +874,7 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
       const uint4 s4 = *reinterpret_cast<const uint4*>(scl + 4 * qd);
       const int64_t left = P.rows - (r0 + 4 * qd);  // rows past the end: scale 0, so 0 whatever y is
       const uint32_t sc[4] = {left > 0 ? s4.x : 0u, left > 1 ? s4.y : 0u, left > 2 ? s4.z : 0u, left > 3 ? s4.w : 0u};
-      if (j >= T::OPS && !mbar_wait_or(smem_u32(&op_empty[s]), (uint32_t)((j / T::OPS - 1) & 1), &s_fail)) {
+      if (j >= T::OPS && !mbar_wait_or(smem_addr(&op_empty[s]), (uint32_t)((j / T::OPS - 1) & 1), &s_fail)) {
         give_up();
         break;
       }
@@ -928,14 +911,14 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
   if (s_fail) {  // let what was committed or fetched finish before the memory goes away
     if (tid == 32) {
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&fin))
+                       smem_addr(&fin))
                    : "memory");
-      mbar_wait(smem_u32(&fin), 0);
+      mbar_wait(smem_addr(&fin), 0);
     }
     if (tid == 0) {  // the last RING fetches issued, one per slot
       const int64_t hi = s_issued;
       for (int64_t j = hi > T::RING ? hi - T::RING : 0; j < hi; ++j)
-        mbar_wait(smem_u32(&raw_full[(int)(j % T::RING)]), (uint32_t)((j / T::RING) & 1));
+        mbar_wait(smem_addr(&raw_full[(int)(j % T::RING)]), (uint32_t)((j / T::RING) & 1));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -985,12 +968,6 @@ __global__ void __launch_bounds__(TcShape<B>::THREADS, 1) gram_tc_kernel(PassPar
 // others wait for the generation to move, at most limit_ns of wall time
 // (%globaltimer), after which they set *error and every CTA returns false at
 // this or the next barrier.  `expected` is the number of CTAs that arrive.
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ bool grid_barrier(unsigned int* bar, int* error, uint64_t limit_ns, unsigned int expected) {
   __shared__ int s_ok;
   __syncthreads();
@@ -1004,10 +981,10 @@ __device__ bool grid_barrier(unsigned int* bar, int* error, uint64_t limit_ns, u
       __threadfence();
       atomicAdd(bar + 1, 1u);
     } else {
-      const uint64_t t0 = global_ns();
+      const uint64_t t0 = now_ns();
       while (*gen == g) {
         if (*(volatile int*)error) { ok = 0; break; }
-        if (global_ns() - t0 > limit_ns) {
+        if (now_ns() - t0 > limit_ns) {
           atomicExch(error, 1);
           ok = 0;
           break;

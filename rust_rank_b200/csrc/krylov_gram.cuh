@@ -2,6 +2,7 @@
 // shared by the Krylov kernels (krylov.cu, resident.cu).
 #pragma once
 #include "krylov_params.h"
+#include "rr_device.cuh"
 
 namespace rr {
 
@@ -116,14 +117,6 @@ struct GramCore {
     }
   }
 };
-
-// D += A * B with A 16x32 u8 (row-major fragments), B 32x8 u8, D 16x8 s32.
-__device__ __forceinline__ void mma_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // Tensor cores (B >= 8): exact integer Gram by byte limbs.  Residues are
 // < 2^31, so z = sum_a z_a 256^a with bytes z_a, and

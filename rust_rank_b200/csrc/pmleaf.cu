@@ -122,12 +122,6 @@ struct LeafShape {
   static_assert(LW % 4 == 0 && OFF_RING % 4 == 0 && OFF_BAR % 2 == 0 && MAP % 4 == 0, "alignment");
 };
 
-__device__ __forceinline__ uint64_t now_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // the same address in the shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
   uint32_t r;
@@ -282,7 +276,7 @@ __device__ __forceinline__ void join_classes(const int (&C)[7][4], const uint32_
                  (uint32_t)((uint32_t)C[1][v] * 256u + (uint32_t)C[0][v]);
     x += (uint64_t)((uint32_t)C[3][v] * 256u + (uint32_t)C[2][v]) * Wt[2];  // 2^16: one instruction, where a shift takes four
     x += (uint64_t)(uint32_t)C[6][v] * Wt[1];
-    val[v] = redc64(x, M);
+    val[v] = redc(x, M);
   }
 }
 
@@ -422,7 +416,7 @@ __device__ __forceinline__ void leaf_products(const LeafBlock& P, const LeafScra
     }
 #pragma unroll
     for (int cl = 0; cl < PC; ++cl) {
-      uint32_t y = redc64(fold(x[cl], M), M);
+      uint32_t y = redc(fold(x[cl], M), M);
       y = addmod(y, __shfl_xor_sync(0xffffffffu, y, 16), M.p);
       if (j < nn && half == 0) R0n[i * S::RS0 + cl] = y;
     }

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) direct_product_kernel(DirectProdu
     x += (uint64_t)(uint32_t)C[4][v] * P.w[0];
     x += (uint64_t)(uint32_t)C[5][v] * P.w[1];
     x += (uint64_t)(uint32_t)C[6][v] * P.w[2];
-    red[((sp * 16 + g + 8 * (v >> 1)) * 8 + 2 * t4 + (v & 1)) * TC + tl] = redc64(fold(x, M), M);
+    red[((sp * 16 + g + 8 * (v >> 1)) * 8 + 2 * t4 + (v & 1)) * TC + tl] = redc(fold(x, M), M);
   }
   __syncthreads();
   for (int e = tid; e < TC * 128; e += kThreads) {

@@ -66,21 +66,10 @@ struct ResParams {
   uint32_t w4, w5, w6;
 };
 
-__device__ __forceinline__ uint64_t res_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 __device__ __forceinline__ void gather_bar() { __barrier_sync_count(1, 32 * kGatherWarps); }
 template <int B>
 __device__ __forceinline__ void gram_bar() {
   __barrier_sync_count(2, 32 * kGramWarps<B>);
-}
-
-__device__ __forceinline__ uint32_t redc_c(uint64_t T, const ModP& M) {  // T < p 2^32
-  const uint32_t q = (uint32_t)T * M.pinv;
-  const uint32_t t = (uint32_t)(((uint64_t)q * M.p + T) >> 32);
-  return min(t, t - M.p);
 }
 
 // The entries of a CTA's row batches (batch j of the CTA = batch blockIdx.x +
@@ -186,8 +175,8 @@ __device__ __forceinline__ void res_pass(const ResCsr& C, const uint2* ell, cons
       uint32_t o[4];
 #pragma unroll
       for (int l = 0; l < 4; ++l) {
-        o[l] = redc_c((uint64_t)redc_c(fold(acc[l], M), M) * s1, M);  // d_r z, or w'
-        if (EVEN) o[l] = redc_c((uint64_t)o[l] * s2, M);              // d_c w'
+        o[l] = redc((uint64_t)redc(fold(acc[l], M), M) * s1, M);  // d_r z, or w'
+        if (EVEN) o[l] = redc((uint64_t)o[l] * s2, M);              // d_c w'
       }
       __stcg(Y + r * TPR + sub, make_uint4(o[0], o[1], o[2], o[3]));
     }
@@ -219,7 +208,7 @@ __device__ __forceinline__ void res_gram(Gram& gram, int64_t rows, int count, co
       const uint32_t v[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
       uint32_t z[4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) z[l] = redc_c((uint64_t)v[l] * s[u], M);
+      for (int l = 0; l < 4; ++l) z[l] = redc((uint64_t)v[l] * s[u], M);
       if (EVEN) gram.add_sym(z, slot, sub, lane, M, W);
       else gram.add(z, v, slot, sub, lane, M, W);
     }
@@ -293,7 +282,7 @@ __global__ void __launch_bounds__(kResThreads<B>, 1) resident_kernel(ResParams P
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(P.bar) : "memory");
           if (seen >= target) break;
           if ((spins & 255) == 255) {
-            const uint64_t t = res_ns();
+            const uint64_t t = now_ns();
             if (t0 == 0) t0 = t;
             if (*(volatile int*)P.status || t - t0 > P.limit_ns) {
               atomicExch(P.status, 1);
