@@ -22,7 +22,7 @@
 // (column, value) pairs read with one 64-bit load.  Each thread issues the
 // loads of four entries before it multiplies, so eight (or four) gathers are in
 // flight per thread.  Sums are accumulated lazily in 64 bits with a fold every
-// 2 or 4 products and finished with a Montgomery reduction; the factor R^{-1}
+// four products (kFold) and finished with a Montgomery reduction; the factor R^{-1}
 // it leaves is absorbed into the preconditioner scales (d R^2 mod p, d R mod p)
 // and, for an odd term formed in pass 1, into one final multiplication by R.
 //
@@ -486,7 +486,7 @@ __device__ __forceinline__ void pass_body(const PassParams& P, uint32_t* gram_sm
 //
 // Resident CTAs per SM the register budget is set for: 5 for the lean pass at
 // width 16 (48 registers; one more CTA of latency hiding measured 1.3 % faster
-// than 4 with 62 registers), 2 for fused passes at width 32, else 4.
+// than 4 with 62 registers), 2 for the initial pass at width 32, else 4.
 template <int B, int GRAM>
 constexpr int kPassMinBlocks = (B >= 32 && GRAM) ? 2 : ((!GRAM && B == 16) ? 5 : 4);
 

@@ -7,8 +7,9 @@
 // With exact arithmetic, _PM_Basis(G, d) equals the ordered product of d
 // order-1 bases m_{d-1} ... m_0, where m_k = M_Basis(coefficient k of
 // (m_{k-1}...m_0) G).  The engine keeps the reference's divide and conquer
-// above blocks of K leaves and runs each block of K leaves iteratively inside
-// one CTA:
+// above blocks of K leaves and runs each block of K leaves iteratively, on one
+// thread-block cluster (pmleaf.cu) or, for contexts that have the tensor cores
+// switched off, in one CTA and a kernel for the block's basis (below):
 //
 //   * a leaf sorts delta stably (descending), eliminates the permuted
 //     coefficient matrix row by row with the reference's pivot rule (first
@@ -1403,7 +1404,8 @@ size_t pm_workspace_bytes(int b, int64_t d) {
 }
 
 // PM-basis of nb generators with the same b, d and p, solved in lockstep: one
-// leaf-kernel CTA per generator, one launch per NTT / product step for all.
+// cluster (or leaf-kernel CTA) per generator and block of leaves, one launch per
+// NTT / product step for all.
 int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, const int64_t* seq_strides, int b,
                           int64_t d, uint32_t p, uint32_t* const* Mh, int64_t* const* deltah) {
   if (nb < 1) return RR_OK;
@@ -1428,6 +1430,7 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   // NTT products: modulo p itself when p - 1 is divisible by the transform
   // length, else exact integer products by CRT over two or three NTT primes
   // (whose product must exceed inner dimension x length x (p-1)^2)
+  const bool native = (uint64_t)(p - 1) % (uint64_t)nmax == 0;
   P.direct = P.mma ? direct_product_max(m) : 0;
   // The transform path's launches cost the same for many generators, the direct
   // products grow with them, so in batches of some size the line lies one level
@@ -1436,10 +1439,13 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   // d = 1024: 11.4 / 12.2; 16: 21.1 / 23.2; 8 of b = 8, d = 2048: 11.2 / 11.8; 2 of
   // b = 32, d = 512: 11.6 / 12.2; but alone at b = 16, d = 2^14: 90.7 / 88.6, and 2
   // of b = 16: 8.7 / 8.5.
-  if ((int64_t)nb * m >= 128 && (uint64_t)(p - 1) % (uint64_t)nmax == 0) P.direct /= 2;
+  if ((int64_t)nb * m >= 128 && native) P.direct /= 2;
   P.use_ntt = d > P.K && d / 2 > P.direct;
   if (P.mma && d > P.K) RR_TRY(direct_product_prepare());
   if (P.use_ntt) {
+    // Orders are refused as for transforms of length 2 nmax, which full products
+    // take, though the cyclic ones here need only nmax: beyond that (d = 2^24 and
+    // more) nothing has been run.
     std::vector<uint32_t> qs;
     if ((uint64_t)(p - 1) % (uint64_t)(2 * nmax) != 0) {
       const long double bound = (long double)m * (long double)(d + 1) * (long double)(p - 1) * (long double)(p - 1);
@@ -1453,12 +1459,9 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
       }
       if (prod <= bound) return fail(RR_EUNSUPPORTED, "d = %lld too large for a three-prime CRT at p = %u", (long long)d, p);
       if (qs.size() < 2) qs.push_back(kCrtPrimes[1]);  // Garner needs two residues
-      P.crt = true;
     }
-    if ((uint64_t)(p - 1) % (uint64_t)nmax == 0) {
-      P.crt = false;
-      qs.assign(1, p);
-    }
+    if (native) qs.assign(1, p);
+    P.crt = !native;
     for (uint32_t q : qs) {
       std::unique_ptr<NttPrime> Q(new NttPrime());
       Q->q = q;
@@ -1537,7 +1540,7 @@ int pm_basis_batch_device(rr_ctx* ctx, int nb, const uint32_t* const* seqs, cons
   outs.push_back({&status, P.status.ptr, sizeof(int)});
   RR_TRY(download_host(ctx, outs, P.s));
   RR_CUDA(cudaStreamSynchronize(P.s));
-  if (status == 3) return fail(RR_ETIMEOUT, "PM-basis leaf kernel: a hand-off between its warp groups gave up");
+  if (status == 3) return fail(RR_ETIMEOUT, "PM-basis leaf block: a hand-off between the CTAs of its cluster gave up");
   if (status) return fail(RR_ECUDA, "PM-basis device status %d (zero row scale)", status);
   return RR_OK;
 }
@@ -1550,10 +1553,9 @@ int pm_basis_device(rr_ctx* ctx, const uint32_t* seq, int64_t seq_stride, int b,
 
 // ---------------------------------------------------------------- no-allocation variant
 // rr_pm_basis_short_noalloc builds G (build_G_kernel) and runs one block of
-// leaves in one CTA of pm_base_kernel -- the original single-kernel block,
-// kept for this entry point; rr_pm_basis now runs the leaves and the block
-// basis as two kernels.  tests/test_zz_no_alloc.py checks both against each
-// other and against the oracle.  Its scratch -- the matrix G, the base
+// leaves in one CTA of pm_base_kernel, which keeps the whole block in one kernel
+// and needs no scratch of its own; rr_pm_basis takes the leaf blocks of pmleaf.cu.
+// tests/test_zz_no_alloc.py checks both against each other and against the oracle.  Its scratch -- the matrix G, the base
 // kernel's double-buffered basis and the status word -- comes from the
 // file-scope array below instead of an allocation.
 // Limits: b <= 16 and d (rounded up to a power of two) <= 32.
