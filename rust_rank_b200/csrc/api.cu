@@ -345,10 +345,16 @@ int rr_krylov_destroy(rr_krylov* kr) {
 constexpr int64_t kGraphApps = 16;
 constexpr int64_t kGraphMinRun = 2 * kGraphApps;
 // Shortest run worth a resident launch, which reads the CSR into shared memory
-// first.  One application at width 16 is three other launches (2000 x 1500: 42 us
-// against 26 resident); narrower ones are two, which overlap (5003 x 4001, b = 3:
-// 25 us against 30).
-static int64_t resident_min_run(const rr_krylov* kr) { return kr->B >= 16 ? 1 : 4; }
+// first.  Widths 4 and 8: an application is two other launches, which overlap
+// (5003 x 4001, b = 3, one application: 25 us against 30 resident).  At width 16 it
+// is three, and the line depends on the entries to read (us, resident / launches;
+// 6.5 entries per row): one application of 20,000 rows 34.3 / 37.8, of 40,000 40.6 /
+// 40.2, of 60,000 46.8 / 42.1, of 194,000 81.5 / 68; two of 150,000 106 / 110, of
+// 194,000 127 / 123; three of 194,000 172.6 / 176.8.
+static int64_t resident_min_run(const rr_krylov* kr) {
+  if (kr->B < 16) return 4;
+  return kr->mat->nnz <= 200000 ? 1 : kr->mat->nnz <= 1100000 ? 2 : 3;
+}
 
 // Captures kGraphApps applications (they are recorded, not run: the host
 // state the launches advance is restored afterwards).  The capture runs on a
