@@ -154,10 +154,10 @@ def test_hand_offs_of_leaf_blocks(own_ctx, b, d):
     next generator is the oracle's."""
     rng = np.random.default_rng(b + d)
     seqs = [rng.integers(0, P, size=(b * (b + 1) // 2, d + 1)).astype(np.uint32) for _ in range(2)]
-    own_ctx.set_waits(0.1, 1)
+    own_ctx.set_waits(0.3, 1)
     t0 = time.perf_counter()
     _timed_out(rr.PM_Basis_batch, seqs, d, P, own_ctx)
-    assert time.perf_counter() - t0 < 1.0
+    assert time.perf_counter() - t0 < 1.5  # up to eight blocks
     own_ctx.set_waits()
     M, delta = rr.PM_Basis(seqs[0], d, P, own_ctx)
     Mo, do = oracle.pm_basis(seqs[0], b, d, P)
