@@ -429,7 +429,7 @@ int rr_krylov_step_device(rr_krylov* kr, int64_t n_apps) {
 
 // The context's pinned buffer for small results, and behind it a word for a
 // handle's status, which kernels write; the caller holds ctx->pinned_mu.
-constexpr size_t kPinnedBytes = 64 << 10;
+constexpr size_t kPinnedBytes = 512 << 10;
 static int pinned_buffer(rr_ctx* ctx, uint32_t** buf, int** status) {
   if (!ctx->pinned) RR_CUDA(cudaHostAlloc((void**)&ctx->pinned, kPinnedBytes + sizeof(int), cudaHostAllocMapped));
   *buf = ctx->pinned;
@@ -570,7 +570,8 @@ int rr_krylov_get_curv(rr_krylov* kr, uint32_t* curv) {
   RR_CUDA(cudaSetDevice(ctx->device));
   // The gathering kernel also writes the handle's status: behind the block, both
   // in one copy to the pinned buffer, where they fit it, else into the pinned word
-  // (next() at 5003 x 4001, b = 3: 45.3 us with the pinned word, 41.0 so).
+  // (next() at 5003 x 4001, b = 3: 45.3 us with the pinned word, 41.0 so; a
+  // block of 250 KB 52 and 43).
   const size_t words = (size_t)kr->b * kr->mat->n;
   const bool small = 4 * (words + 1) <= kPinnedBytes;
   std::lock_guard<std::mutex> lk(ctx->pinned_mu);
