@@ -127,7 +127,9 @@ int rr_krylov_fill_status(rr_krylov* kr, char* buf, int64_t cap);
  * synchronisation.  Terms stay in the handle's device sequence buffer. */
 int rr_krylov_step_device(rr_krylov* kr, int64_t n_apps);
 /* Copy terms [from, to) of the device sequence buffer into the host array
- * seq[b(b+1)/2][seq_stride] (synchronises the context stream). */
+ * seq[b(b+1)/2][seq_stride] (synchronises the context stream).  RR_ETIMEOUT,
+ * with seq as it was, when a device-side wait of the handle's kernels had given
+ * up. */
 int rr_krylov_fetch(rr_krylov* kr, int64_t from, int64_t to, uint32_t* seq, int64_t seq_stride);
 /* Current sequence length (terms computed so far, including queued work). */
 int rr_krylov_length(const rr_krylov* kr, int64_t* len);
@@ -316,7 +318,9 @@ int rr_server_destroy(rr_server* server);
 
 /* Device bytes a matrix of this shape and its Krylov state hold while
  * resident (both CSR copies, blocks, preconditioner forms, sequence of the
- * length rule of src/main.rs:497-504), the figure admission and placement use. */
+ * length rule of src/main.rs:497-504, Gram sums of its passes and of runs of up
+ * to 512 applications), the figure admission and placement use; a service counts
+ * runs of its own length (chunk_apps). */
 int rr_footprint(int64_t m, int64_t n, int64_t nnz, int32_t b, uint64_t* bytes);
 /* The placement rule (host only): items in decreasing footprint order, each
  * on the device with the most room left (dev_free[d] minus what it already
