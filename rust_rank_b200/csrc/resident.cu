@@ -510,17 +510,23 @@ int prepare(rr_krylov* kr) {
   kr->res_top = 0;
   while (kr->res_top < kr->res_deepest && (mat->ctx->num_sms >> (kr->res_top + 1)) >= batches) ++kr->res_top;
   if (mat->ctx->coop_level <= kr->res_deepest) kr->res_top = std::max(kr->res_top, mat->ctx->coop_level);
+  kr->res_apps = std::min(mat->ctx->run_apps, kResMaxApps);
+  return RR_OK;
+}
+
+// At a handle's first run: its Gram slots, and behind them the barrier word.
+// Without room for them the handle takes the pass kernels.
+template <int B>
+int scratch(rr_krylov* kr) {
   // the limit is per kernel, shared by every thread of the process: always the largest
   RR_CUDA(cudaFuncSetAttribute(resident_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmem));
-  cudaStream_t s = mat->ctx->stream;
-  kr->res_apps = std::min(mat->ctx->run_apps, kResMaxApps);
-  if (kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps), s) != RR_OK) {  // no room: the pass kernels
+  cudaStream_t s = kr->mat->ctx->stream;
+  if (kr->res_gram.alloc_async(resident_gram_words(B, kr->res_apps) + 1, s) != RR_OK) {
     kr->res_deepest = -1;
     return RR_OK;
   }
   RR_CUDA(cudaMemsetAsync(kr->res_gram.ptr, 0, kr->res_gram.bytes(), s));
-  RR_TRY(kr->res_bar.alloc_async(1, s));
-  RR_CUDA(cudaMemsetAsync(kr->res_bar.ptr, 0, kr->res_bar.bytes(), s));
+  kr->res_bar = reinterpret_cast<unsigned int*>(kr->res_gram.ptr + resident_gram_words(B, kr->res_apps));
   return RR_OK;
 }
 
@@ -528,6 +534,9 @@ template <int B>
 int run(rr_krylov* kr, int apps, bool* taken) {
   const rr_matrix* mat = kr->mat;
   cudaStream_t s = mat->ctx->stream;
+  *taken = false;
+  if (!kr->res_bar) RR_TRY(scratch<B>(kr));
+  if (!kr->res_bar) return RR_OK;
   ResParams P;
   P.A = ResCsr{mat->A.rowptr.ptr, mat->A.cv.ptr, mat->A.rows};
   P.At = ResCsr{mat->At.rowptr.ptr, mat->At.cv.ptr, mat->At.rows};
@@ -542,7 +551,7 @@ int run(rr_krylov* kr, int apps, bool* taken) {
   P.drinv_r = kr->drinv_r.ptr;
   P.dcinv_r = kr->dcinv_r.ptr;
   P.gram = kr->res_gram.ptr;
-  P.bar = kr->res_bar.ptr;
+  P.bar = kr->res_bar;
   P.status = kr->d_status.ptr;
   P.limit_ns = mat->ctx->wait_limit_ns;
   P.missing = (unsigned int)mat->ctx->wait_missing;
@@ -573,7 +582,7 @@ int run(rr_krylov* kr, int apps, bool* taken) {
   const int np = kr->b * (kr->b + 1) / 2, NP = B * (B + 1) / 2;
   resident_finish_kernel<<<std::min((2 * apps * NP + 255) / 256, 296), 256, 0, s>>>(
       kr->res_gram.ptr, 2 * apps, kr->b, B, kr->S.ptr + (size_t)(kr->len - kr->base) * np, kr->d_term.ptr,
-      kr->res_bar.ptr, kr->M);
+      kr->res_bar, kr->M);
   RR_CUDA(cudaGetLastError());
   kr->launches += 2;
   kr->len += 2 * apps;

@@ -221,10 +221,11 @@ struct rr_krylov_s {
   int64_t graph_launches = 0;
   // runs with the CSR in shared memory (resident.cu): the shares of the device
   // they may take (2^-res_top down to 2^-res_deepest; -1 = the matrix does not
-  // fit), most applications of a run, Gram sums, barrier
+  // fit), most applications of a run; Gram sums and, behind them, the barrier
+  // word, allocated at the first run
   int res_top = 0, res_deepest = -1, res_apps = 0;
   rr::DevBuf<unsigned long long> res_gram;
-  rr::DevBuf<unsigned int> res_bar;
+  unsigned int* res_bar = nullptr;
   ~rr_krylov_s() {
     if (graph) cudaGraphExecDestroy(graph);
   }
