@@ -78,8 +78,8 @@ def test_contexts_run_side_by_side():
     the other, 7.6 times)."""
     steppers = [Stepper(700, 4, 10 * i) for i in range(8)]
     pieces = [128] * 8
-    one = min(_together(steppers[:1], pieces) for _ in range(4))
-    eight = min(_together(steppers, pieces) for _ in range(4))
+    one = min(_together(steppers[:1], pieces) for _ in range(8))
+    eight = min(_together(steppers, pieces) for _ in range(8))
     for s in steppers:
         s.close()
     assert eight < 5 * one, (one, eight)

@@ -24,7 +24,9 @@ dm = rr.CsrMatrix.from_arrays(rowptr, col, val, m, n).to_device(P)
 ks = rr.KrylovStream(dm, V, dr, dc, 0)
 ks.step_device(apps)                       # 65 MB of terms
 rr.default_context().synchronize()
-rest = torch.empty(torch.cuda.mem_get_info()[0] - (24 << 20), dtype=torch.uint8, device="cuda")
+rest = []
+while torch.cuda.mem_get_info()[0] > 48 << 20:   # not all of the free memory can be had in one piece
+    rest.append(torch.empty(max((torch.cuda.mem_get_info()[0] - (24 << 20)) * 7 // 8, 16 << 20), dtype=torch.uint8, device="cuda"))
 seq = np.zeros((b * (b + 1) // 2, 2 * apps + 1), np.uint32)
 ks.fetch(0, 2 * apps + 1, seq)
 del rest
