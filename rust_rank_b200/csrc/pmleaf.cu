@@ -75,6 +75,7 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 8;      // portable cluster size
 constexpr int kMaxLeaves = 64;
+constexpr uint64_t kShortNs = 200000ull;
 constexpr uint64_t kLandNs = 1000000ull;  // in which the messages in flight have long landed
 
 // Words of the shared-memory regions; RL = rows per lane (m <= 32 RL), CPW =
@@ -166,21 +167,24 @@ __device__ __forceinline__ bool bar_try(uint32_t a) {
       : "memory");
   return done != 0;
 }
-// Waits for the message of mbarrier q; gives up after wait_ns or once another
-// wait of this CTA did.
+// Waits for the message of mbarrier q; gives up after wait_ns, once another
+// wait of this CTA did, or soon if one of an earlier block did, whose basis is then
+// not there (looked up after kShortNs only: no wait of a running block takes so long).
 __device__ __forceinline__ bool bar_wait(uint32_t* sm, int q, volatile int* abort, const LeafBlock& P) {
   const uint32_t a = smem_addr(sm + 2 * q);
   if (bar_try(a)) return true;
   const uint64_t t0 = now_ns();
-  for (;;) {
+  do {
     if (bar_try(a)) return true;
     if (*abort) return false;
-    if (now_ns() - t0 > P.wait_ns) {
-      *abort = 1;
-      atomicExch(P.status, 3);
-      return false;
-    }
+  } while (now_ns() - t0 <= kShortNs);
+  while (now_ns() - t0 <= P.wait_ns && *(volatile int*)P.status != 3) {
+    if (bar_try(a)) return true;
+    if (*abort) return false;
   }
+  *abort = 1;
+  atomicExch(P.status, 3);
+  return false;
 }
 
 // *p = v where `on` holds, as one predicated store
@@ -997,7 +1001,7 @@ __global__ void __launch_bounds__(kThreads, 1) pm_leaf_block_kernel(LeafBlock P)
   P.Mout += (int64_t)z * P.out_bs;
   const int m = P.m, n = P.n, K = P.K;
   if (tid == 0) {
-    s_abort = *(volatile int*)P.status == 3;  // an earlier block gave up: its basis is not there
+    s_abort = 0;
     s_ok = 1;
   }
   if (tid < 8) sm[S::OFF_USED + tid] = 0;
