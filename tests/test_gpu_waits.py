@@ -150,7 +150,7 @@ def test_served_request_whose_run_gave_up(b):
 
 @pytest.mark.parametrize("b,d", [(1, 1), (2, 2), (4, 64), (8, 256), (16, 4), (16, 256), (32, 16), (32, 128)])
 def test_hand_offs_of_leaf_blocks(own_ctx, b, d):
-    """Every CTA of the cluster ends, the blocks after the first do not wait again, and the context's
+    """Every CTA of the cluster ends, the blocks after the first do not wait as long again, and the context's
     next generator is the oracle's."""
     rng = np.random.default_rng(b + d)
     seqs = [rng.integers(0, P, size=(b * (b + 1) // 2, d + 1)).astype(np.uint32) for _ in range(2)]
